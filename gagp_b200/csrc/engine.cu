@@ -233,9 +233,11 @@ void harvest(gagp_engine* e) {
 // lowered-program list sizes (fast, exact) and [4c+2] its next child; then
 // [4 kChunks + 1] the size of the shared exact-VM list of a round whose
 // ranges hand their exact-VM programs to one launch.
-constexpr int kCountWords = 4 * gagp_engine::kChunks + 4;
-// [4 kChunks + 2]: the size of the deferred bounded-region program list
+// [4 kChunks + 2]: the size of the deferred bounded-region program list;
+// [4 kChunks + 4, + 5]: its kernel's next item (64 bits).
 constexpr int kRegionCount = 4 * gagp_engine::kChunks + 2;
+constexpr int kRegionNext = 4 * gagp_engine::kChunks + 4;
+constexpr int kCountWords = 4 * gagp_engine::kChunks + 6;
 gagp_status ensure_region_workspace(gagp_engine* e, size_t words);
 
 gagp_status ensure_lists(gagp_engine* e, size_t items) {
@@ -1594,10 +1596,11 @@ gagp_status vm_general_launch(int sm_count, cudaStream_t stream, const gb::Searc
   return GAGP_OK;
 }
 
+constexpr int kRegionBlocks = 4, kRegionLanes = 16;  // of the bounded-region kernel: per SM, and per warp
 // The bounded-region workspace for plans of up to `words` int64 words per
 // lane (grown, never shrunk; the device is idle between API calls).
 gagp_status ensure_region_workspace(gagp_engine* e, size_t words) {
-  const int lanes = 2 * e->sm_count * gb::kRegionThreads;
+  const int lanes = kRegionBlocks * e->sm_count * (gb::kRegionThreads / 32) * kRegionLanes;
   if (e->region_ws && words <= e->region_ws_words && lanes <= e->region_lanes) return GAGP_OK;
   CUDA_TRY(cudaStreamSynchronize(e->stream));
   if (e->region_ws) cudaFree(e->region_ws);
@@ -1613,13 +1616,15 @@ gagp_status ensure_region_workspace(gagp_engine* e, size_t words) {
   return GAGP_OK;
 }
 
-// The deferred programs with bounded regions: a fixed grid of the region
-// workspace's lanes, after every exact-VM launch that deferred to it.
-gagp_status vm_region_launch(gagp_engine* e, cudaStream_t stream, const gb::SearchDesc* descs, int mode,
-                             const gb::ProgramRef* list, const int32_t* count) {
+// The deferred programs with bounded regions, after every exact-VM launch
+// that deferred to it: the workspace's lanes shared by kRegionBlocks blocks
+// per SM, 16 lanes per warp.
+gagp_status vm_region_launch(gagp_engine* e, cudaStream_t stream, const BatchView& v, int mode) {
   if (!e->region_ws) return fail(GAGP_DEVICE_ERROR, "bounded regions without a workspace");
-  gb::k_vm_region<<<e->region_lanes / gb::kRegionThreads, gb::kRegionThreads, 0, stream>>>(
-      descs, mode, list, count, e->region_ws, e->region_ws_words);
+  gb::k_vm_region<<<kRegionBlocks * e->sm_count, gb::kRegionThreads, 0, stream>>>(
+      v.d_desc, mode, e->d_region, e->d_counts + kRegionCount,
+      reinterpret_cast<unsigned long long*>(e->d_counts + kRegionNext), v.max_C, kRegionLanes, e->region_ws,
+      e->region_ws_words);
   return GAGP_OK;
 }
 
@@ -1692,8 +1697,7 @@ gagp_status launch_vm(gagp_engine* e, const BatchView& v, int mode, cudaStream_t
 
 gagp_status launch_start(gagp_engine* e, const BatchView& v) {
   { Timed t(e, KN_INIT); gb::k_init_population<<<blocks_for(v.total_members, 128), 128, 0, e->stream>>>(v.d_desc, v.d_member_off, v.n); }
-  CUDA_TRY(cudaMemsetAsync(e->d_counts, 0, 2 * sizeof(int32_t), e->stream));
-  CUDA_TRY(cudaMemsetAsync(e->d_counts + kRegionCount, 0, sizeof(int32_t), e->stream));
+  CUDA_TRY(cudaMemsetAsync(e->d_counts, 0, kCountWords * sizeof(int32_t), e->stream));
   {
     Timed t(e, KN_LOWER);
     gb::k_lower<<<blocks_for(v.total_members, gb::kLowerWarps), gb::kLowerWarps * 32, 0, e->stream>>>(
@@ -1705,7 +1709,7 @@ gagp_status launch_start(gagp_engine* e, const BatchView& v) {
       st != GAGP_OK)
     return st;
   if (v.regions)
-    if (const gagp_status st = vm_region_launch(e, e->stream, v.d_desc, 0, e->d_region, e->d_counts + kRegionCount);
+    if (const gagp_status st = vm_region_launch(e, e->stream, v, 0);
         st != GAGP_OK)
       return st;
   { Timed t(e, KN_KEYS); gb::k_member_keys<<<blocks_for(v.total_members, 128), 128, 0, e->stream>>>(v.d_desc, v.d_member_off, v.n); }
@@ -1834,7 +1838,7 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
       return st2;
   }
   if (v.regions)
-    if (const gagp_status st2 = vm_region_launch(e, e->stream, v.d_desc, 1, e->d_region, e->d_counts + kRegionCount);
+    if (const gagp_status st2 = vm_region_launch(e, e->stream, v, 1);
         st2 != GAGP_OK)
       return st2;
   if (v.generational) {
@@ -1999,8 +2003,8 @@ struct EvalPlan {
   int stride, code_stride, bc_stride;
   size_t region_words;  // bounded-region workspace per lane (0: the grammar has none)
 };
-// Lanes of a row evaluation's bounded-region kernel.
-constexpr int kRowRegionBlocks = 64;
+// A row evaluation's bounded-region kernel: blocks, and lanes per warp.
+constexpr int kRowRegionBlocks = 256, kRowRegionLanes = 8;
 
 EvalPlan plan_eval(const gagp_grammar* g, const gagp_cases* c, int rows) {
   EvalPlan p{};
@@ -2028,13 +2032,13 @@ EvalPlan plan_eval(const gagp_grammar* g, const gagp_cases* c, int rows) {
   p.fitness = L.take(8 * R); p.wrong = L.take(4 * R); p.errors = L.take(4 * R);
   p.counters = L.take(8 * GAGP_COUNTERS); p.round = L.take(16);
   p.fast = L.take(sizeof(gb::ProgramRef) * R); p.general = L.take(sizeof(gb::ProgramRef) * R);
-  p.counts = L.take(16); p.off = L.take(8);
+  p.counts = L.take(32); p.off = L.take(8);
   p.region_words = 0;
   for (int r = 0; r < g->region_count; ++r)
     if (g->regions[r].traversal == 0)
       p.region_words = std::max(p.region_words, gb::region_lane_words(gb::region_info_of(g->regions[r])));
   p.region_list = L.take(sizeof(gb::ProgramRef) * R);
-  p.region_ws = L.take(8 * std::max<size_t>(1, p.region_words * kRowRegionBlocks * gb::kRegionThreads));
+  p.region_ws = L.take(8 * std::max<size_t>(1, p.region_words * kRowRegionBlocks * (gb::kRegionThreads / 32) * kRowRegionLanes));
   return p;
 }
 
@@ -2185,7 +2189,7 @@ gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g,
   CUDA_TRY(up(p.off, off, sizeof off));
   CUDA_TRY(cudaMemsetAsync(b + p.counters, 0, 8 * GAGP_COUNTERS, stream));
   CUDA_TRY(cudaMemsetAsync(b + p.round, 0, 16, stream));
-  CUDA_TRY(cudaMemsetAsync(b + p.counts, 0, 16, stream));
+  CUDA_TRY(cudaMemsetAsync(b + p.counts, 0, 32, stream));
   const gb::SearchDesc* dd = at<gb::SearchDesc>(b, p.desc);
   const int32_t* doff = at<int32_t>(b, p.off);
   gb::ProgramRef* fast = at<gb::ProgramRef>(b, p.fast);
@@ -2209,8 +2213,9 @@ gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g,
       st != GAGP_OK)
     return st;
   if (p.region_words)
-    gb::k_vm_region<<<kRowRegionBlocks, gb::kRegionThreads, 0, stream>>>(dd, 0, region_list, counts + 2,
-                                                                          at<int64_t>(b, p.region_ws), p.region_words);
+    gb::k_vm_region<<<kRowRegionBlocks, gb::kRegionThreads, 0, stream>>>(
+        dd, 0, region_list, counts + 2, reinterpret_cast<unsigned long long*>(counts + 4), C, kRowRegionLanes,
+        at<int64_t>(b, p.region_ws), p.region_words);
   CUDA_TRY(cudaGetLastError());
   int32_t round[4];
   CUDA_TRY(cudaMemcpyAsync(round, b + p.round, sizeof round, cudaMemcpyDeviceToHost, stream));

@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(kLowerWarps * 32, 8) k_lower(const SearchDesc*
         s.code_temps[slot] = temps;
         s.vm_acc[2 * size_t(slot)] = 0;
         s.vm_acc[2 * size_t(slot) + 1] = 0;
+        if (mode == 0 && s.errors) s.errors[slot] = 0;
         fast_list[atomicAdd(&list_count[0], 1)] = ProgramRef{si, slot};
         atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[9]),
                   (unsigned long long)(row_bytes + 8ull * (len + t.nc) + 16));
@@ -143,6 +144,9 @@ __global__ void __launch_bounds__(kLowerWarps * 32, 8) k_lower(const SearchDesc*
         // temporaries
         s.bc_locals[slot] = r.locals | (r.stack_bound << 8) | (r.main << 16);
         s.code_temps[slot] = r.main_constants;
+        s.vm_acc[2 * size_t(slot)] = 0;
+        s.vm_acc[2 * size_t(slot) + 1] = 0;
+        if (mode == 0 && s.errors) s.errors[slot] = 0;
         general_list[atomicAdd(general_count, 1)] = ProgramRef{si, slot};
         atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[9]),
                   (unsigned long long)(row_bytes + 20ull * bl + 8ull * r.constants + 16));
@@ -152,17 +156,56 @@ __global__ void __launch_bounds__(kLowerWarps * 32, 8) k_lower(const SearchDesc*
   }
 }
 
-__device__ __forceinline__ void store_result(const SearchDesc& s, int mode, int slot, int64_t loss, uint32_t wrong,
-                                             uint32_t errors) {
+__device__ __forceinline__ void store_result(const SearchDesc& s, int mode, int slot, int64_t loss, uint32_t wrong) {
   const double f = -double(loss);
   if (mode == 0) {
     s.fitness[slot] = f;
     s.wrong[slot] = s.has_wrong ? wrong : 0;
-    if (s.errors) s.errors[slot] = errors;
   } else {
     s.c_fitness[slot] = f;
     s.c_wrong[slot] = s.has_wrong ? wrong : 0;
   }
+}
+
+// One tile's loss and wrong count (and, where they are kept, its runtime
+// errors) added to program `slot` of a search; returns whether this was the
+// last of the program's `tiles` tiles, which then stores the program's
+// result and counts its evaluation.  Loss (40 bits), wrong count (16) and
+// finished tiles (8) share one word where they fit -- one atomic per tile
+// and no fence -- and take two words with a fence between them otherwise.
+// One lane calls it.
+__device__ __forceinline__ bool add_tile_result(const SearchDesc& s, int mode, int slot, unsigned tiles, int64_t loss,
+                                                uint32_t wrong, uint32_t errors) {
+  unsigned long long* acc = s.vm_acc + 2 * size_t(slot);
+  const uint64_t worst = s.metric == GAGP_METRIC_EXACT ? 1 : uint64_t(s.penalty_int);
+  if (mode == 0 && s.errors && errors) atomicAdd(&s.errors[slot], errors);
+  bool last;
+  int64_t total;
+  uint32_t total_wrong;
+  if (tiles < 256 && s.C < 65536 && uint64_t(s.C) * worst < (1ULL << 40)) {
+    const unsigned long long mine = (unsigned long long)loss | ((unsigned long long)wrong << 40) | (1ULL << 56);
+    const unsigned long long sum = atomicAdd(&acc[0], mine) + mine;
+    last = unsigned(sum >> 56) == tiles;
+    total = int64_t(sum & ((1ULL << 40) - 1));
+    total_wrong = uint32_t((sum >> 40) & 0xffffu);
+  } else {
+    atomicAdd(&acc[0], (unsigned long long)loss);
+    __threadfence();
+    const unsigned long long before = atomicAdd(&acc[1], (unsigned long long)wrong | (1ULL << 32));
+    last = unsigned(before >> 32) == tiles - 1;
+    total_wrong = uint32_t(before) + wrong;
+    total = 0;
+    if (last) {
+      __threadfence();
+      total = int64_t(atomicAdd(&acc[0], 0ULL));
+    }
+  }
+  if (last) {
+    store_result(s, mode, slot, total, total_wrong);
+    atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[0]), 1ULL);
+    atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[2]), (unsigned long long)s.C);
+  }
+  return last;
 }
 
 // General VM: the programs the accumulator VM cannot run (list programs,
@@ -278,7 +321,8 @@ __global__ void __launch_bounds__(kGeneralWarps * 32) k_vm_general(const SearchD
         te += red_errors[w];
         ts += red_steps[w];
       }
-      store_result(s, mode, p.slot, tl, tw, te);
+      store_result(s, mode, p.slot, tl, tw);
+      if (mode == 0 && s.errors) s.errors[p.slot] = te;
       atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[24]), ts);
       atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[0]), 1ULL);
       atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[2]), (unsigned long long)s.C);
@@ -288,23 +332,39 @@ __global__ void __launch_bounds__(kGeneralWarps * 32) k_vm_general(const SearchD
 }
 
 // Programs with bounded regions (deferred by k_vm_general): a fixed grid of
-// blocks of kRegionThreads, one program per block at a time and one case
-// per thread at a time on the per-thread interpreter
-// (run_program_regions), each thread with its own `ws_words` words of
-// frames and memo cells in `ws` (gridDim x kRegionThreads lanes).
+// persistent warps, each taking the next (program, group of cases) from
+// `next_item` (zeroed before the launch), one case per lane on the
+// per-thread interpreter (run_program_regions), each lane with its own
+// `ws_words` words of frames and memo cells in `ws` (`lanes` per warp).
+//
+// What bounds it: the cases of one program walk their recurrences along
+// different paths, so lanes of a warp rarely share an instruction (2.7 of 32
+// when a warp took 32 cases) and a warp's time is the sum of its lanes',
+// while a round's few hundred programs left most of the GPU idle.  So a
+// group is as small as still gives about kRegionItems items per warp: a
+// round of 200 programs x 40 cases runs one case per warp.
 constexpr int kRegionThreads = 128;
+constexpr int kRegionItems = 4;
 __global__ void __launch_bounds__(kRegionThreads) k_vm_region(const SearchDesc* descs, int mode, const ProgramRef* list,
-                                                              const int32_t* list_count, int64_t* ws,
-                                                              size_t ws_words) {
-  __shared__ int64_t red_loss[kRegionThreads / 32];
-  __shared__ uint32_t red_wrong[kRegionThreads / 32], red_errors[kRegionThreads / 32];
-  __shared__ unsigned long long red_steps[kRegionThreads / 32];
+                                                              const int32_t* list_count, unsigned long long* next_item,
+                                                              int max_C, int lanes, int64_t* ws, size_t ws_words) {
   const int count = *list_count;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int64_t* mine = ws + (size_t(blockIdx.x) * kRegionThreads + threadIdx.x) * ws_words;
-  for (int i = blockIdx.x; i < count; i += gridDim.x) {
-    const ProgramRef p = list[i];
+  const long long warps = (long long)gridDim.x * (kRegionThreads / 32);
+  int group = 1;
+  while (group < lanes && (long long)count * max_C > kRegionItems * warps * group) group *= 2;
+  const int groups = (max_C + group - 1) / group;
+  const unsigned long long items = (unsigned long long)count * groups;
+  int64_t* mine = ws + ((size_t(blockIdx.x) * (kRegionThreads / 32) + warp) * lanes + min(lane, lanes - 1)) * ws_words;
+  for (;;) {
+    unsigned long long item = 0;
+    if (lane == 0) item = atomicAdd(next_item, 1ULL);
+    item = __shfl_sync(kFull, item, 0);
+    if (item >= items) break;
+    const ProgramRef p = list[item / groups];
     const SearchDesc& s = descs[p.search];
+    const int c = int(item % groups) * group + lane;
+    if (c - lane >= s.C) continue;
     const int n = s.bc_len[p.slot], shape = s.bc_locals[p.slot];
     const int n_locals = shape & 0xff, n_main = (shape >> 16) & 0xffff;
     const int32_t* code = s.bc + size_t(p.slot) * 5 * s.bc_stride;
@@ -314,7 +374,7 @@ __global__ void __launch_bounds__(kRegionThreads) k_vm_region(const SearchDesc* 
     int64_t loss = 0;
     uint32_t wrong = 0, errors = 0;
     uint64_t steps = 0;
-    for (int c = threadIdx.x; c < s.C; c += kRegionThreads) {
+    if (lane < group && c < s.C) {
       int64_t value = 0;
       int tag = 0;
       if (run_program_regions(view, s.regions, s.n_regions, code, n, n_main, consts, main_consts, n_locals, c, mine,
@@ -326,33 +386,15 @@ __global__ void __launch_bounds__(kRegionThreads) k_vm_region(const SearchDesc* 
         ++errors;
       }
     }
+    __syncwarp();
     loss = warp_sum(loss);
     wrong = warp_sum(wrong);
     errors = warp_sum(errors);
     steps = warp_sum(steps);
     if (lane == 0) {
-      red_loss[warp] = loss;
-      red_wrong[warp] = wrong;
-      red_errors[warp] = errors;
-      red_steps[warp] = steps;
+      add_tile_result(s, mode, p.slot, unsigned((s.C + group - 1) / group), loss, wrong, errors);
+      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[24]), (unsigned long long)steps);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int64_t tl = 0;
-      uint32_t tw = 0, te = 0;
-      unsigned long long ts = 0;
-      for (int w = 0; w < kRegionThreads / 32; ++w) {
-        tl += red_loss[w];
-        tw += red_wrong[w];
-        te += red_errors[w];
-        ts += red_steps[w];
-      }
-      store_result(s, mode, p.slot, tl, tw, te);
-      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[24]), ts);
-      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[0]), 1ULL);
-      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[2]), (unsigned long long)s.C);
-    }
-    __syncthreads();
   }
 }
 
@@ -397,40 +439,12 @@ __global__ void __launch_bounds__(256, K == 4 ? 2 : 4) k_vm_fast(const SearchDes
     loss = warp_sum(loss);
     wrong = warp_sum(wrong);
     if (lane == 0) {
-      unsigned long long* acc = s.vm_acc + 2 * size_t(p.slot);
       const unsigned tiles = unsigned((s.C + 32 * K - 1) / (32 * K));
-      const uint64_t worst = s.metric == GAGP_METRIC_EXACT ? 1 : uint64_t(s.penalty_int);
-      bool last;
-      int64_t total;
-      uint32_t total_wrong;
-      if (tiles < 256 && s.C < 65536 && uint64_t(s.C) * worst < (1ULL << 40)) {
-        // loss (40 bits), wrong count (16) and finished tiles (8) of the
-        // program in one word: one atomic per tile and no fence
-        const unsigned long long mine = (unsigned long long)loss | ((unsigned long long)wrong << 40) | (1ULL << 56);
-        const unsigned long long sum = atomicAdd(&acc[0], mine) + mine;
-        last = unsigned(sum >> 56) == tiles;
-        total = int64_t(sum & ((1ULL << 40) - 1));
-        total_wrong = uint32_t((sum >> 40) & 0xffffu);
-      } else {
-        atomicAdd(&acc[0], (unsigned long long)loss);
-        __threadfence();
-        const unsigned long long before = atomicAdd(&acc[1], (unsigned long long)wrong | (1ULL << 32));
-        last = unsigned(before >> 32) == tiles - 1;
-        total_wrong = uint32_t(before) + wrong;
-        total = 0;
-        if (last) {
-          __threadfence();
-          total = int64_t(atomicAdd(&acc[0], 0ULL));
-        }
-      }
-      if (last) {  // the last tile of the program
-        store_result(s, mode, p.slot, total, total_wrong, 0);  // accumulator programs never fail
-        // the program's instructions over all its cases, counted once
+      // accumulator programs never fail; the program's instructions over all
+      // its cases are counted once
+      if (add_tile_result(s, mode, p.slot, tiles, loss, wrong, 0))
         atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[3]),
                   (unsigned long long)s.code_len[p.slot] * (unsigned long long)s.C);
-        atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[0]), 1ULL);
-        atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[2]), (unsigned long long)s.C);
-      }
     }
   }
 }
