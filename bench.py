@@ -471,7 +471,7 @@ def vm_entry(stats: dict, delta: dict, clock_mhz, sm_count: int = 148) -> dict:
     (one warp instruction per cycle on each of the SMs' 4 sub-partitions)."""
     out = {}
     fast = stats.get("k_vm_fast", {"ms": 0, "launches": 0})
-    exact = stats.get("k_vm_general", {"ms": 0, "launches": 0})
+    exact = stats.get("k_vm_exact", {"ms": 0, "launches": 0})
     if fast["ms"] > 0:
         out["fast"] = {"kernel_ms": fast["ms"], "launches": fast["launches"],
                        "accumulator_ops_per_s": delta["accumulator_ops"] / (fast["ms"] / 1000.0)}
@@ -483,7 +483,7 @@ def vm_entry(stats: dict, delta: dict, clock_mhz, sm_count: int = 148) -> dict:
         out["program_cases_per_s"] = delta["program_cases"] / (ms / 1000.0)
     issue = vm_issue_summary(ARGS_WORKLOAD[0])
     clock = (clock_mhz or 1965.0) * 1e6
-    for name, st, key in (("k_vm_fast", fast, "fast"), ("k_vm_general", exact, "exact")):
+    for name, st, key in (("k_vm_fast", fast, "fast"), ("k_vm_exact", exact, "exact")):
         if name in issue and st["launches"] and key in out:
             per_launch_s = st["ms"] / st["launches"] / 1000.0
             slots = sm_count * 4 * clock * per_launch_s

@@ -64,6 +64,7 @@ struct Search {
   // can fail); otherwise only the rare program past the accumulator VM's
   // limits does
   bool exact_heavy = false;
+  bool exact_possible = false;  // a program of its may need the exact VM
   size_t region_words = 0;  // the largest bounded-region plan's workspace per lane (0: none)
   gb::SearchDesc* d_desc = nullptr;   // single-search batch descriptor
   int32_t* d_off = nullptr;           // {0, P, 0, B}: member and child offsets
@@ -91,8 +92,9 @@ struct gagp_engine {
   size_t max_smem = 0;
   // batch scratch
   gb::ProgramRef* d_fast = nullptr;
-  gb::ProgramRef* d_general = nullptr;
-  gb::ProgramRef* d_region = nullptr;  // programs with bounded regions, deferred by the exact VM
+  gb::ProgramRef* d_exact = nullptr;    // register code
+  gb::ProgramRef* d_general = nullptr;  // reference bytecode for the interpreter
+  gb::ProgramRef* d_region = nullptr;   // programs with bounded regions
   int32_t* d_counts = nullptr;
   // the bounded-region kernel's frame and memo workspace: region_ws_words
   // int64 words per lane, region_lanes lanes (sized by the largest plan admitted)
@@ -156,11 +158,11 @@ namespace {
 
 enum KernelId {
   KN_INIT, KN_LOWER, KN_VM_FAST, KN_KEYS, KN_START, KN_RECORD, KN_VARY, KN_CHILD, KN_PLACE,
-  KN_COMMIT, KN_STREAM, KN_LEVELS, KN_VM_GENERAL, KN_INDEX, KN_COUNT
+  KN_COMMIT, KN_STREAM, KN_LEVELS, KN_VM_EXACT, KN_INDEX, KN_COUNT
 };
 const char* const kKernelNames[KN_COUNT] = {"k_init_population", "k_lower", "k_vm_fast",
                                             "k_member_keys", "k_start", "k_record", "k_vary", "k_child_results",
-                                            "k_place", "k_commit", "k_stream", "k_place_levels", "k_vm_general",
+                                            "k_place", "k_commit", "k_stream", "k_place_levels", "k_vm_exact",
                                             "k_member_index"};
 
 cudaEvent_t take_event(gagp_engine* e) {
@@ -229,26 +231,31 @@ void harvest(gagp_engine* e) {
   e->event_next = 0;
 }
 
-// Device counters of a round: per variation range c, [4c] and [4c+1] its
-// lowered-program list sizes (fast, exact) and [4c+2] its next child; then
-// [4 kChunks + 1] the size of the shared exact-VM list of a round whose
-// ranges hand their exact-VM programs to one launch.
-// [4 kChunks + 2]: the size of the deferred bounded-region program list;
-// [4 kChunks + 4, + 5]: its kernel's next item (64 bits).
-constexpr int kRegionCount = 4 * gagp_engine::kChunks + 2;
-constexpr int kRegionNext = 4 * gagp_engine::kChunks + 4;
-constexpr int kCountWords = 4 * gagp_engine::kChunks + 6;
+// Device counters of a round: per variation range c, [4c] its accumulator
+// program list's size and [4c+2] its next child; then the sizes of the lists
+// the ranges share -- accumulator programs (of exact-heavy rounds), register
+// code, interpreter programs, programs with bounded regions -- and, 64 bits
+// each, the next items of the exact VM's two lists and the region kernel's.
+constexpr int kSharedFast = 4 * gagp_engine::kChunks;
+constexpr int kExactCount = kSharedFast + 1;
+constexpr int kGeneralCount = kSharedFast + 2;
+constexpr int kRegionCount = kSharedFast + 3;
+constexpr int kExactNext = kSharedFast + 4;
+constexpr int kRegionNext = kExactNext + 4;
+constexpr int kCountWords = kRegionNext + 2;
 gagp_status ensure_region_workspace(gagp_engine* e, size_t words);
 
 gagp_status ensure_lists(gagp_engine* e, size_t items) {
   if (items <= e->list_capacity) return GAGP_OK;
   if (e->d_fast) cudaFree(e->d_fast);
+  if (e->d_exact) cudaFree(e->d_exact);
   if (e->d_general) cudaFree(e->d_general);
   if (e->d_region) cudaFree(e->d_region);
-  e->d_fast = e->d_general = e->d_region = nullptr;
+  e->d_fast = e->d_exact = e->d_general = e->d_region = nullptr;
   e->list_capacity = 0;
   const size_t cap = std::max<size_t>({items, size_t(1024), 2 * e->list_capacity});
   CUDA_TRY(cudaMalloc(&e->d_fast, cap * sizeof(gb::ProgramRef)));
+  CUDA_TRY(cudaMalloc(&e->d_exact, cap * sizeof(gb::ProgramRef)));
   CUDA_TRY(cudaMalloc(&e->d_general, cap * sizeof(gb::ProgramRef)));
   CUDA_TRY(cudaMalloc(&e->d_region, cap * sizeof(gb::ProgramRef)));
   if (!e->d_counts) CUDA_TRY(cudaMalloc(&e->d_counts, kCountWords * sizeof(int32_t)));
@@ -773,6 +780,10 @@ int bytecode_bound(const gagp_grammar* g, int maxv) {
   return per_node * maxv + 2;
 }
 
+// Instructions of a program's bytecode row, rounded so that a row also holds
+// register code in 16-byte words.
+int bytecode_stride(const gagp_grammar* g, int maxv) { return int(align_up(size_t(bytecode_bound(g, maxv)), 4)); }
+
 // Whether a grammar's programs mostly need the exact VM: it holds
 // traversals or bound reads, or operations that can raise a runtime error
 // (modulo and division by zero, list builtins).
@@ -800,6 +811,18 @@ bool exact_heavy(const gagp_grammar* g) {
       return true;
   }
   return false;
+}
+
+// Whether any program of a grammar can need the exact VM.  A program of
+// accumulator operations goes there only when its bytecode may exceed the
+// fuel or when it needs more than kMaxTemps temporaries.  The fewest nodes of
+// a tree of need k are T(k) = 1 + min(2 T(k-1), 3 T(k-2)) (two children of
+// need k-1, or an if over three of need k-2), T(0) = 2, T(1) = 5: a seventh
+// temporary takes T(7) = 135 nodes.
+bool exact_possible(const gagp_grammar* g, int fuel) {
+  static_assert(gb::kMaxTemps == 6, "the node bound is the seventh temporary's");
+  const int maxv = g->max_nodes - g->fixed_nodes;
+  return exact_heavy(g) || maxv >= 135 || bytecode_bound(g, maxv) > fuel;
 }
 
 // Device copy of the traversal table.
@@ -839,7 +862,7 @@ Plan plan_search(const gagp_grammar* g, const gagp_cases* c, const gagp_search_c
   const int maxv = g->max_nodes - g->fixed_nodes;
   p.stride = int(align_up(size_t(maxv), 4));
   p.code_stride = 2 * maxv + 8;
-  p.bc_stride = bytecode_bound(g, maxv);
+  p.bc_stride = bytecode_stride(g, maxv);
   p.slots = std::max(P, B);
   const long long draws = (long long)B * cfg->replacement_size + 1;
   p.stream_capacity = int(((draws + 311) / 312 + 2) * 312);
@@ -1171,7 +1194,7 @@ gagp_status gagp_b200_engine_create(int32_t device, uint64_t arena_bytes, gagp_e
   CUDA_TRY(cudaFuncSetAttribute(gb::k_vm_fast<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(e->max_smem) - 1024));
   CUDA_TRY(cudaFuncSetAttribute(gb::k_vm_fast<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(e->max_smem) - 1024));
   CUDA_TRY(cudaFuncSetAttribute(gb::k_vary, cudaFuncAttributeMaxDynamicSharedMemorySize, int(e->max_smem) - 1024));
-  CUDA_TRY(cudaFuncSetAttribute(gb::k_vm_general, cudaFuncAttributeMaxDynamicSharedMemorySize, int(e->max_smem) - 1024));
+  CUDA_TRY(cudaFuncSetAttribute(gb::k_vm_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gb::kExactSmem)));
   *out = e.release();
   return GAGP_OK;
 }
@@ -1189,6 +1212,7 @@ void gagp_b200_engine_destroy(gagp_engine* e) {
   if (e->pool) cudaMemPoolDestroy(e->pool);
   if (e->pinned) cudaFreeHost(e->pinned);
   cudaFree(e->d_fast);
+  cudaFree(e->d_exact);
   cudaFree(e->d_general);
   cudaFree(e->d_region);
   cudaFree(e->region_ws);
@@ -1243,6 +1267,7 @@ gagp_status gagp_b200_search_create(gagp_engine* e, const gagp_grammar* g, const
   s->fixed_nodes = g->fixed_nodes;
   s->has_wrong = cfg->metric != GAGP_METRIC_LEGACY;
   s->exact_heavy = exact_heavy(g);
+  s->exact_possible = exact_possible(g, cfg->fuel);
   s->region_words = 0;
   for (int r = 0; r < g->region_count; ++r)
     if (g->regions[r].traversal == 0)
@@ -1464,10 +1489,11 @@ struct BatchView {
   int32_t* d_child_off = nullptr;    // n + 1
   int n = 0, total_members = 0, total_children = 0, max_P = 0, max_lanes = 1, max_rounds = 0, max_stride = 4;
   long long max_draws = 0;
-  int max_code_stride = 2, max_bc_stride = 2;
+  int max_code_stride = 2;
   int max_C = 1, max_inputs = 0;
   int min_B = 1 << 30;               // the smallest round of the batch
   bool exact_heavy = false;          // some search's programs mostly need the exact VM
+  bool exact_possible = false;       // some search's programs may need it
   bool regions = false;              // some search's grammar has bounded regions
   bool generational = false;         // the batch's schedule (one per batch)
   std::vector<int> child_off;        // host copy of the child offsets (n + 1)
@@ -1525,11 +1551,10 @@ gagp_status make_batch_view(gagp_engine* e, const std::vector<Search*>& list, Ba
   v->max_stride = 4;
   v->max_draws = 0;
   v->max_code_stride = 2;
-  v->max_bc_stride = 2;
   v->max_lanes = 1;
   v->max_C = 1;
   v->max_inputs = 0;
-  v->exact_heavy = false;
+  v->exact_heavy = v->exact_possible = false;
   v->regions = false;
   v->child_off.assign(1, 0);
   v->image_bytes.clear();
@@ -1537,6 +1562,7 @@ gagp_status make_batch_view(gagp_engine* e, const std::vector<Search*>& list, Ba
     v->child_off.push_back(v->child_off.back() + s->B);
     v->image_bytes.push_back(size_t(s->desc.gen_image_bytes));
     v->exact_heavy |= s->exact_heavy;
+    v->exact_possible |= s->exact_possible;
     v->regions |= s->region_words > 0;
     v->max_C = std::max(v->max_C, s->desc.C);
     v->max_inputs = std::max(v->max_inputs, s->desc.n_inputs);
@@ -1547,7 +1573,6 @@ gagp_status make_batch_view(gagp_engine* e, const std::vector<Search*>& list, Ba
     v->max_rounds = std::max(v->max_rounds, s->total_rounds);
     v->max_stride = std::max(v->max_stride, s->stride);
     v->max_code_stride = std::max(v->max_code_stride, s->desc.code_stride);
-    v->max_bc_stride = std::max(v->max_bc_stride, s->desc.bc_stride);
     v->max_draws = std::max(v->max_draws, (long long)s->B * s->desc.replacement_size + 1);
     v->min_B = std::min(v->min_B, s->B);
   }
@@ -1556,8 +1581,6 @@ gagp_status make_batch_view(gagp_engine* e, const std::vector<Search*>& list, Ba
 
 int blocks_for(int items, int threads) { return std::max(1, (items + threads - 1) / threads); }
 
-// Evaluates lowered programs listed by k_lower: counts[0] programs on the
-// fast (accumulator) VM, counts[1] on the exact VM.
 // Fast-VM launch of one instantiation.
 void vm_fast_launch(int lanes, int blocks, int threads, size_t smem, cudaStream_t stream, const gb::SearchDesc* descs,
                     int mode, const gb::ProgramRef* list, const int32_t* counts, int temp_stride, int code_stride,
@@ -1570,30 +1593,29 @@ void vm_fast_launch(int lanes, int blocks, int threads, size_t smem, cudaStream_
   }
 }
 
-// Exact-VM launch over counts[1] programs: persistent blocks of 8 warps,
-// each program's bytecode staged in dynamic shared memory with the warp-SIMD
-// VM's slots (gb::general_smem_bytes).
-constexpr int kGeneralThreads = gb::kGeneralWarps * 32;
-size_t vm_general_smem(int bc_stride_max) { return gb::general_smem_bytes(bc_stride_max); }
-// `heavy`: most programs may be on the list, so the grid fills every SM;
-// otherwise the list is rarely more than a handful of programs and a
-// quarter of the SMs take them (an empty launch of a full grid costs a few
-// microseconds on every range's critical path).
-gagp_status vm_general_launch(int sm_count, cudaStream_t stream, const gb::SearchDesc* descs, int mode,
-                              const gb::ProgramRef* list, const int32_t* counts, int bc_stride_max, bool heavy,
-                              gb::ProgramRef* deferred, int32_t* deferred_count) {
-  const size_t smem = vm_general_smem(bc_stride_max);
-  int blocks = std::max(1, sm_count / 4);
-  if (heavy) {
-    int per_sm = 0;
-    const cudaError_t occ = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gb::k_vm_general, kGeneralThreads,
-                                                                          smem);
-    if (occ != cudaSuccess) return fail(GAGP_DEVICE_ERROR, std::string("exact VM occupancy: ") + cudaGetErrorString(occ));
-    blocks = sm_count * std::max(1, per_sm);
-  }
-  gb::k_vm_general<<<blocks, kGeneralThreads, smem, stream>>>(descs, mode, list, counts + 1, bc_stride_max, deferred,
-                                                              deferred_count);
-  return GAGP_OK;
+// Exact-VM launch over the register-code and interpreter lists (next: their
+// next items, zeroed).  `heavy`: most programs may be on them, so the grid
+// fills every SM; otherwise they are rarely more than a handful of programs
+// and a quarter of the SMs take them.
+void vm_exact_launch(int sm_count, cudaStream_t stream, const gb::SearchDesc* descs, int mode,
+                     const gb::LowerLists& lists, int32_t* next, int max_C, bool heavy) {
+  const int blocks = heavy ? 3 * sm_count : std::max(1, sm_count / 4);
+  gb::k_vm_exact<<<blocks, gb::kExactWarps * 32, gb::kExactSmem, stream>>>(
+      descs, mode, lists, reinterpret_cast<unsigned long long*>(next), max_C);
+}
+// Lowering of batch items [lo, hi).
+void lower_launch(cudaStream_t stream, const gb::SearchDesc* descs, const int32_t* off, int n, int mode,
+                  const gb::LowerLists& lists, int lo, int hi, bool exact) {
+  const int blocks = blocks_for(hi - lo, gb::kLowerWarps);
+  if (exact) gb::k_lower<true><<<blocks, gb::kLowerWarps * 32, 0, stream>>>(descs, off, n, mode, lists, lo, hi);
+  else gb::k_lower<false><<<blocks, gb::kLowerWarps * 32, 0, stream>>>(descs, off, n, mode, lists, lo, hi);
+}
+// The engine's program lists; accumulator programs to `fast`, counted in
+// counter word `fast_word`.
+gb::LowerLists engine_lists(gagp_engine* e, gb::ProgramRef* fast, int fast_word) {
+  int32_t* c = e->d_counts;
+  return gb::LowerLists{fast, e->d_exact, e->d_general, e->d_region, c + fast_word, c + kExactCount, c + kGeneralCount,
+                        c + kRegionCount};
 }
 
 constexpr int kRegionBlocks = 4, kRegionLanes = 16;  // of the bounded-region kernel: per SM, and per warp
@@ -1616,9 +1638,8 @@ gagp_status ensure_region_workspace(gagp_engine* e, size_t words) {
   return GAGP_OK;
 }
 
-// The deferred programs with bounded regions, after every exact-VM launch
-// that deferred to it: the workspace's lanes shared by kRegionBlocks blocks
-// per SM, 16 lanes per warp.
+// The programs with bounded regions: the workspace's lanes shared by
+// kRegionBlocks blocks per SM, 16 lanes per warp.
 gagp_status vm_region_launch(gagp_engine* e, cudaStream_t stream, const BatchView& v, int mode) {
   if (!e->region_ws) return fail(GAGP_DEVICE_ERROR, "bounded regions without a workspace");
   gb::k_vm_region<<<kRegionBlocks * e->sm_count, gb::kRegionThreads, 0, stream>>>(
@@ -1686,13 +1707,15 @@ gagp_status launch_vm_fast(gagp_engine* e, const BatchView& v, int mode, cudaStr
   return GAGP_OK;
 }
 
-// Both VMs over one range's lists: counts[0] fast programs, counts[1] exact.
-gagp_status launch_vm(gagp_engine* e, const BatchView& v, int mode, cudaStream_t stream, const gb::ProgramRef* fast,
-                      const gb::ProgramRef* general, const int32_t* counts, const VmPlan& plan) {
-  if (const gagp_status st = launch_vm_fast(e, v, mode, stream, fast, counts, plan); st != GAGP_OK) return st;
-  Timed t(e, KN_VM_GENERAL, stream);
-  return vm_general_launch(e->sm_count, stream, v.d_desc, mode, general, counts, v.max_bc_stride, v.exact_heavy,
-                           e->d_region, e->d_counts + kRegionCount);
+// The exact VM and the bounded-region kernel over a round's shared lists
+// (nothing for a batch whose programs never need them).
+gagp_status launch_vm_exact(gagp_engine* e, const BatchView& v, int mode) {
+  if (v.exact_possible) {
+    Timed t(e, KN_VM_EXACT);
+    vm_exact_launch(e->sm_count, e->stream, v.d_desc, mode, engine_lists(e, e->d_fast, kSharedFast),
+                    e->d_counts + kExactNext, v.max_C, v.exact_heavy);
+  }
+  return v.regions ? vm_region_launch(e, e->stream, v, mode) : GAGP_OK;
 }
 
 gagp_status launch_start(gagp_engine* e, const BatchView& v) {
@@ -1700,18 +1723,15 @@ gagp_status launch_start(gagp_engine* e, const BatchView& v) {
   CUDA_TRY(cudaMemsetAsync(e->d_counts, 0, kCountWords * sizeof(int32_t), e->stream));
   {
     Timed t(e, KN_LOWER);
-    gb::k_lower<<<blocks_for(v.total_members, gb::kLowerWarps), gb::kLowerWarps * 32, 0, e->stream>>>(
-        v.d_desc, v.d_member_off, v.n, 0, e->d_fast, e->d_general, e->d_counts, e->d_counts + 1, 0, v.total_members);
+    lower_launch(e->stream, v.d_desc, v.d_member_off, v.n, 0, engine_lists(e, e->d_fast, kSharedFast), 0,
+                 v.total_members, v.exact_possible);
   }
   VmPlan start_plan;
   start_plan.lanes = v.max_lanes;
-  if (const gagp_status st = launch_vm(e, v, 0, e->stream, e->d_fast, e->d_general, e->d_counts, start_plan);
+  if (const gagp_status st = launch_vm_fast(e, v, 0, e->stream, e->d_fast, e->d_counts + kSharedFast, start_plan);
       st != GAGP_OK)
     return st;
-  if (v.regions)
-    if (const gagp_status st = vm_region_launch(e, e->stream, v, 0);
-        st != GAGP_OK)
-      return st;
+  if (const gagp_status st = launch_vm_exact(e, v, 0); st != GAGP_OK) return st;
   { Timed t(e, KN_KEYS); gb::k_member_keys<<<blocks_for(v.total_members, 128), 128, 0, e->stream>>>(v.d_desc, v.d_member_off, v.n); }
   { Timed t(e, KN_START); gb::k_start<<<v.n, 256, 0, e->stream>>>(v.d_desc, v.n); }
   return cudaPeekAtLastError() == cudaSuccess ? GAGP_OK : fail(GAGP_DEVICE_ERROR, cudaGetErrorString(cudaGetLastError()));
@@ -1749,8 +1769,8 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
     }
     CUDA_TRY(cudaEventRecord(e->drawn, e->draws));
   }
-  // per range c: counts[4c] / [4c+1] lowered-program list sizes, [4c+2] the
-  // next child of the variation warps; range c's lists start at item lo
+  // per range c: counts[4c] its accumulator programs, [4c+2] the next child
+  // of the variation warps; range c's accumulator list starts at item lo
   CUDA_TRY(cudaMemsetAsync(e->d_counts, 0, kCountWords * sizeof(int32_t), e->stream));
   CUDA_TRY(cudaEventRecord(e->chunk_fork, e->stream));
   const int chunks = v.total_children >= 4096 ? gagp_engine::kChunks : 1;
@@ -1774,17 +1794,12 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
     }
   }
   const size_t vary_smem = warps * gb::warp_rows_bytes(v.max_stride) + image_max;
-  // With ranges, the VM that a round rarely needs gets one launch for all
-  // ranges once they have joined: the exact VM in rounds of mostly
-  // accumulator programs, and in rounds of mostly exact-VM programs (list
-  // programs) both, so that the exact VM's persistent blocks see every
-  // program at once.  A per-range launch, mostly empty, still waits for SM
-  // room (shared memory) behind the other ranges' VM blocks, on its range's
-  // critical path.  The lowering then lists those programs in one shared
-  // list (counts at shared_count: [0] fast, [1] exact).
-  const bool shared_exact = chunks > 1;
+  // The ranges share the exact VM's lists and one launch of it, once they
+  // have joined, and in rounds of mostly exact-VM programs (list programs)
+  // one of the accumulator VM too.  A per-range launch, mostly empty, would
+  // still wait for SM room (shared memory) behind the other ranges' VM
+  // blocks, on its range's critical path.
   const bool shared_fast = chunks > 1 && v.exact_heavy;
-  int32_t* shared_count = e->d_counts + 4 * gagp_engine::kChunks;
   int per_sm = 0;
   CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gb::k_vary, warps * 32, vary_smem));
   for (int c = 0; c < chunks; ++c) {
@@ -1805,42 +1820,22 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
     CUDA_TRY(cudaStreamWaitEvent(st, e->indexed, 0));
     {
       Timed t(e, KN_LOWER, st);
-      gb::k_lower<<<blocks_for(hi - lo, gb::kLowerWarps), gb::kLowerWarps * 32, 0, st>>>(
-          v.d_desc, v.d_child_off, v.n, 1, shared_fast ? e->d_fast : e->d_fast + lo,
-          shared_exact ? e->d_general : e->d_general + lo, shared_fast ? shared_count : counts,
-          shared_exact ? shared_count + 1 : counts + 1, lo, hi);
+      lower_launch(st, v.d_desc, v.d_child_off, v.n, 1,
+                   engine_lists(e, shared_fast ? e->d_fast : e->d_fast + lo, shared_fast ? kSharedFast : 4 * c), lo, hi,
+                   v.exact_possible);
     }
-    if (shared_fast) {
-      // both VMs after the join
-    } else if (shared_exact) {
+    if (!shared_fast)
       if (const gagp_status st2 = launch_vm_fast(e, v, 1, st, e->d_fast + lo, counts, vm); st2 != GAGP_OK) return st2;
-    } else {
-      if (const gagp_status st2 = launch_vm(e, v, 1, st, e->d_fast + lo, e->d_general + lo, counts, vm);
-          st2 != GAGP_OK)
-        return st2;
-    }
     if (chunks > 1) {
       CUDA_TRY(cudaEventRecord(e->chunk_done[c], st));
       CUDA_TRY(cudaStreamWaitEvent(e->stream, e->chunk_done[c], 0));
     }
   }
-  if (shared_exact) {
-    // all ranges' exact-VM programs (and, in exact-heavy rounds, their
-    // accumulator programs) at once
-    if (shared_fast)
-      if (const gagp_status st2 = launch_vm_fast(e, v, 1, e->stream, e->d_fast, shared_count, vm); st2 != GAGP_OK)
-        return st2;
-    Timed t(e, KN_VM_GENERAL);
-    if (const gagp_status st2 = vm_general_launch(e->sm_count, e->stream, v.d_desc, 1, e->d_general, shared_count,
-                                                  v.max_bc_stride, v.exact_heavy, e->d_region,
-                                                  e->d_counts + kRegionCount);
+  if (shared_fast)
+    if (const gagp_status st2 = launch_vm_fast(e, v, 1, e->stream, e->d_fast, e->d_counts + kSharedFast, vm);
         st2 != GAGP_OK)
       return st2;
-  }
-  if (v.regions)
-    if (const gagp_status st2 = vm_region_launch(e, e->stream, v, 1);
-        st2 != GAGP_OK)
-      return st2;
+  if (const gagp_status st2 = launch_vm_exact(e, v, 1); st2 != GAGP_OK) return st2;
   if (v.generational) {
     // every child becomes the member of its index (reproduce's swap), after
     // the reused children have read their sources' results and the history
@@ -1998,11 +1993,14 @@ namespace {
 struct EvalPlan {
   Layout L;
   size_t desc, ex, info, minimum, local_types, regions, inputs, expected, lists, node, cval, len, code, code_len, kpool,
-      code_temps, vm_acc, bc, bc_len, bc_locals, bc_consts, fitness, wrong, errors, counters, round, fast, general,
-      counts, off, region_list, region_ws;
+      code_temps, vm_acc, bc, bc_len, bc_locals, bc_consts, fitness, wrong, errors, counters, round, fast, exact,
+      general, counts, off, region_list, region_ws;
   int stride, code_stride, bc_stride;
   size_t region_words;  // bounded-region workspace per lane (0: the grammar has none)
 };
+// Counter words of a row evaluation: the four lists' sizes, then the next
+// items (64 bits) of the exact VM's two lists and the region kernel's.
+constexpr int kRowCountWords = 10;
 // A row evaluation's bounded-region kernel: blocks, and lanes per warp.
 constexpr int kRowRegionBlocks = 256, kRowRegionLanes = 8;
 
@@ -2011,7 +2009,7 @@ EvalPlan plan_eval(const gagp_grammar* g, const gagp_cases* c, int rows) {
   const int maxv = g->max_nodes - g->fixed_nodes;
   p.stride = int(align_up(size_t(std::max(1, maxv)), 4));
   p.code_stride = 2 * maxv + 8;
-  p.bc_stride = bytecode_bound(g, maxv);
+  p.bc_stride = bytecode_stride(g, maxv);
   const int E = g->expression_count, C = c->case_count;
   const size_t R = size_t(std::max(1, rows)), S = size_t(p.stride);
   auto& L = p.L;
@@ -2031,8 +2029,9 @@ EvalPlan plan_eval(const gagp_grammar* g, const gagp_cases* c, int rows) {
   p.bc_consts = L.take(8 * R * p.bc_stride);
   p.fitness = L.take(8 * R); p.wrong = L.take(4 * R); p.errors = L.take(4 * R);
   p.counters = L.take(8 * GAGP_COUNTERS); p.round = L.take(16);
-  p.fast = L.take(sizeof(gb::ProgramRef) * R); p.general = L.take(sizeof(gb::ProgramRef) * R);
-  p.counts = L.take(32); p.off = L.take(8);
+  p.fast = L.take(sizeof(gb::ProgramRef) * R); p.exact = L.take(sizeof(gb::ProgramRef) * R);
+  p.general = L.take(sizeof(gb::ProgramRef) * R);
+  p.counts = L.take(4 * kRowCountWords); p.off = L.take(8);
   p.region_words = 0;
   for (int r = 0; r < g->region_count; ++r)
     if (g->regions[r].traversal == 0)
@@ -2189,14 +2188,15 @@ gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g,
   CUDA_TRY(up(p.off, off, sizeof off));
   CUDA_TRY(cudaMemsetAsync(b + p.counters, 0, 8 * GAGP_COUNTERS, stream));
   CUDA_TRY(cudaMemsetAsync(b + p.round, 0, 16, stream));
-  CUDA_TRY(cudaMemsetAsync(b + p.counts, 0, 32, stream));
+  CUDA_TRY(cudaMemsetAsync(b + p.counts, 0, 4 * kRowCountWords, stream));
   const gb::SearchDesc* dd = at<gb::SearchDesc>(b, p.desc);
   const int32_t* doff = at<int32_t>(b, p.off);
   gb::ProgramRef* fast = at<gb::ProgramRef>(b, p.fast);
-  gb::ProgramRef* general = at<gb::ProgramRef>(b, p.general);
   int32_t* counts = at<int32_t>(b, p.counts);
-  gb::k_lower<<<blocks_for(R, gb::kLowerWarps), gb::kLowerWarps * 32, 0, stream>>>(dd, doff, 1, 0, fast, general, counts,
-                                                                                  counts + 1, 0, R);
+  const gb::LowerLists lists{fast, at<gb::ProgramRef>(b, p.exact), at<gb::ProgramRef>(b, p.general),
+                             at<gb::ProgramRef>(b, p.region_list), counts, counts + 1, counts + 2, counts + 3};
+  const bool exact = exact_possible(g, cfg->fuel);
+  lower_launch(stream, dd, doff, 1, 0, lists, 0, R, exact);
   const int warps = 8;
   const int lanes = d.vm_cases_per_lane;
   const int temp_stride = gb::kMaxTemps * lanes * 32;
@@ -2206,15 +2206,10 @@ gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g,
   const int per_sm = std::max(1, std::min(4, int((max_smem - 1024) / smem)));
   vm_fast_launch(lanes, sm_count * per_sm, warps * 32, smem, stream, dd, 0, fast, counts, temp_stride, code_stride,
                  p.stride, C);
-  if (vm_general_smem(p.bc_stride) > max_smem - 1024) return fail(GAGP_DECLINED, "program too long for the exact VM");
-  gb::ProgramRef* region_list = at<gb::ProgramRef>(b, p.region_list);
-  if (const gagp_status st = vm_general_launch(sm_count, stream, dd, 0, general, counts, p.bc_stride, true,
-                                               region_list, counts + 2);
-      st != GAGP_OK)
-    return st;
+  if (exact) vm_exact_launch(sm_count, stream, dd, 0, lists, counts + 4, C, true);
   if (p.region_words)
     gb::k_vm_region<<<kRowRegionBlocks, gb::kRegionThreads, 0, stream>>>(
-        dd, 0, region_list, counts + 2, reinterpret_cast<unsigned long long*>(counts + 4), C, kRowRegionLanes,
+        dd, 0, lists.region, counts + 3, reinterpret_cast<unsigned long long*>(counts + 8), C, kRowRegionLanes,
         at<int64_t>(b, p.region_ws), p.region_words);
   CUDA_TRY(cudaGetLastError());
   int32_t round[4];
@@ -2263,7 +2258,7 @@ gagp_status static_scratch_on(int device, StaticDevice** out) {
     CUDA_TRY(cudaFuncSetAttribute(gb::k_vm_fast<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 1024));
     CUDA_TRY(cudaFuncSetAttribute(gb::k_vm_fast<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 1024));
     CUDA_TRY(cudaFuncSetAttribute(gb::k_vm_fast<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 1024));
-    CUDA_TRY(cudaFuncSetAttribute(gb::k_vm_general, cudaFuncAttributeMaxDynamicSharedMemorySize, smem - 1024));
+    CUDA_TRY(cudaFuncSetAttribute(gb::k_vm_exact, cudaFuncAttributeMaxDynamicSharedMemorySize, int(gb::kExactSmem)));
     d.scratch = static_cast<char*>(ptr);
     d.sm_count = sms;
     d.max_smem = size_t(smem);

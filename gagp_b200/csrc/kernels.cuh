@@ -12,6 +12,7 @@
 
 #include "operators.cuh"
 #include "vm.cuh"
+#include "exact.cuh"
 
 namespace gb {
 
@@ -71,18 +72,33 @@ __global__ void k_init_population(const SearchDesc* descs, const int32_t* off, i
 }
 
 // ----------------------------------------------------------- lowering
+// Where lowered programs are listed, with each list's size: accumulator
+// programs, register code, reference bytecode for the per-thread
+// interpreter, and programs with bounded regions.
+struct LowerLists {
+  ProgramRef *fast, *exact, *general, *region;
+  int32_t *fast_count, *exact_count, *general_count, *region_count;
+};
 // mode 0: the members (initial evaluation); mode 1: this round's children
 // that reuse no member's result; batch items [lo, hi).  One warp per row:
-// the accumulator program when the row is total and fits the fuel (listed in
-// fast_list, counted in list_count[0]), else the reference bytecode for the
-// general VM (lane 0; listed in general_list, counted in *general_count).
+// the accumulator program when the row is total and fits the fuel, else
+// register code for the exact VM, else the reference bytecode (lane 0).
+// Exact false: no program of the batch can need the exact VM
+// (exact_possible in the engine), so the other lowerings, with their shared
+// memory and local arrays, stay out of the kernel and a row the accumulator
+// lowering rejects is one the reference's compiler rejects too.
 constexpr int kLowerWarps = 4;
-__global__ void __launch_bounds__(kLowerWarps * 32, 8) k_lower(const SearchDesc* descs, const int32_t* off, int n,
-                                                            int mode, ProgramRef* fast_list, ProgramRef* general_list,
-                                                            int32_t* list_count, int32_t* general_count, int lo,
-                                                            int hi) {
-  __shared__ LowerScratch scratch[kLowerWarps];
+union LowerSmem {
+  LowerScratch fast;
+  ExactScratch exact;
+};
+template <bool Exact>
+__global__ void __launch_bounds__(kLowerWarps * 32, Exact ? 7 : 8)
+    k_lower(const SearchDesc* descs, const int32_t* off, int n, int mode, LowerLists lists, int lo, int hi) {
+  using Scratch = typename std::conditional<Exact, LowerSmem, LowerScratch>::type;
+  __shared__ Scratch scratch[kLowerWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  LowerScratch& fast_scratch = reinterpret_cast<LowerScratch&>(scratch[warp]);
   const int total_items = min(off[n], hi);
   for (int item = lo + blockIdx.x * kLowerWarps + warp; item < total_items; item += gridDim.x * kLowerWarps) {
     const int si = find_search(off, n, item);
@@ -114,45 +130,59 @@ __global__ void __launch_bounds__(kLowerWarps * 32, 8) k_lower(const SearchDesc*
     }
     int temps = 0;
     const int len = lower_accumulator_warp(s, t.node, t.n, t.cval, t.nc, s.code + size_t(slot) * s.code_stride,
-                                           s.code_stride, s.kpool + size_t(slot) * s.stride, scratch[warp], &temps);
+                                           s.code_stride, s.kpool + size_t(slot) * s.stride, fast_scratch, &temps);
     // row and its length read; code words, constants, length, temps and list entry written
     const uint64_t row_bytes = 8ull * (t.n + t.nc) + 4;
+    if (lane == 0) {
+      s.vm_acc[2 * size_t(slot)] = 0;
+      s.vm_acc[2 * size_t(slot) + 1] = 0;
+      if (mode == 0 && s.errors) s.errors[slot] = 0;
+    }
     if (len >= 0) {
       if (lane == 0) {
         s.code_len[slot] = len;
         s.code_temps[slot] = temps;
-        s.vm_acc[2 * size_t(slot)] = 0;
-        s.vm_acc[2 * size_t(slot) + 1] = 0;
-        if (mode == 0 && s.errors) s.errors[slot] = 0;
-        fast_list[atomicAdd(&list_count[0], 1)] = ProgramRef{si, slot};
+        lists.fast[atomicAdd(lists.fast_count, 1)] = ProgramRef{si, slot};
         atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[9]),
                   (unsigned long long)(row_bytes + 8ull * (len + t.nc) + 16));
       }
       continue;
     }
-    if (lane == 0) {
-      LowerResult r{};
-      const int bl = lower_program(lower_view(s), t.node, t.cval, t.n, t.nc, s.bc + size_t(slot) * 5 * s.bc_stride,
-                                   s.bc_stride, s.bc_consts + size_t(slot) * s.bc_stride, s.bc_stride, &r);
-      if (bl < 0) {
-        raise_error(s, 30);  // the phase compiler rejected a constructed program
-      } else {
-        s.bc_len[slot] = bl;
-        // the main code's length marks a program with bounded regions (its
-        // records and phase code follow); an exact-VM program keeps its
-        // main constant count where an accumulator program keeps its
-        // temporaries
-        s.bc_locals[slot] = r.locals | (r.stack_bound << 8) | (r.main << 16);
-        s.code_temps[slot] = r.main_constants;
-        s.vm_acc[2 * size_t(slot)] = 0;
-        s.vm_acc[2 * size_t(slot) + 1] = 0;
-        if (mode == 0 && s.errors) s.errors[slot] = 0;
-        general_list[atomicAdd(general_count, 1)] = ProgramRef{si, slot};
-        atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[9]),
-                  (unsigned long long)(row_bytes + 20ull * bl + 8ull * r.constants + 16));
+    if constexpr (!Exact) {
+      if (lane == 0) raise_error(s, 30);  // the phase compiler rejects the row
+    } else {
+      int32_t* bc = s.bc + size_t(slot) * 5 * s.bc_stride;
+      int64_t* bc_consts = s.bc_consts + size_t(slot) * s.bc_stride;
+      const int exact = lower_exact_warp(s, t.node, t.n, t.cval, t.nc, reinterpret_cast<uint4*>(bc),
+                                         s.bc_stride * 5 / 4, bc_consts, scratch[warp].exact);
+      if (lane == 0) {
+        if (exact >= 0) {
+          lists.exact[atomicAdd(lists.exact_count, 1)] = ProgramRef{si, slot};
+          atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[9]),
+                    (unsigned long long)(row_bytes + 16ull * (exact + 1) + 16));
+        } else {
+          LowerResult r{};
+          const int bl = lower_program(lower_view(s), t.node, t.cval, t.n, t.nc, bc, s.bc_stride, bc_consts,
+                                       s.bc_stride, &r);
+          if (bl < 0) {
+            raise_error(s, 30);  // the phase compiler rejected a constructed program
+          } else {
+            s.bc_len[slot] = bl;
+            // the main code's length (a program with bounded regions: its
+            // records and phase code follow); an exact-VM program keeps its
+            // main constant count where an accumulator program keeps its
+            // temporaries
+            s.bc_locals[slot] = r.locals | (r.stack_bound << 8) | (r.main << 16);
+            s.code_temps[slot] = r.main_constants;
+            if (r.main < bl) lists.region[atomicAdd(lists.region_count, 1)] = ProgramRef{si, slot};
+            else lists.general[atomicAdd(lists.general_count, 1)] = ProgramRef{si, slot};
+            atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[9]),
+                      (unsigned long long)(row_bytes + 20ull * bl + 8ull * r.constants + 16));
+          }
+        }
       }
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 
@@ -208,130 +238,80 @@ __device__ __forceinline__ bool add_tile_result(const SearchDesc& s, int mode, i
   return last;
 }
 
-// General VM: the programs the accumulator VM cannot run (list programs,
-// possible runtime errors or fuel exhaustion) on the exact interpreter.
-// Persistent blocks of 8 warps take one program of the list at a time and
-// stage its bytecode and constants in shared memory.  A program whose costs
-// are all 1..255 and whose locals and stack fit kSimdSlots runs on the
-// warp-SIMD VM (run_program_simd): the block's warps take its tiles of 32
-// cases; any other runs on run_program, a case per thread.  The block
-// reduces the losses in order-free integer sums.  A separate kernel from the
-// fast VM, so that the interpreters' registers and local arrays do not
-// lower the fast VM's occupancy.
+// The exact VMs: the programs the accumulator VM cannot run.  Persistent
+// warps, each taking the next (program, tile of 32 cases) from `next`
+// (next[0] register code, next[1] the interpreter's programs; zeroed before
+// the launch).  A tile adds its sums to the program's accumulators.
 //
-// Dynamic shared memory: constants (bc_stride_max int64), the staged SIMD
-// words (bc_stride_max uint4), the 5-int code (bc_stride_max instructions),
-// a jump-target bit per instruction and per warp kSimdSlots x 32 int64 slots.
-constexpr int kGeneralWarps = 8;
-__host__ __device__ __forceinline__ size_t general_smem_bytes(int bc_stride_max) {
-  return size_t(bc_stride_max) * (8 + 16 + 20) + 8 * ((size_t(bc_stride_max) + 63) / 64) + 16 +
-         size_t(kGeneralWarps) * kSimdSlots * 32 * 8;
+// Tiles are taken one warp at a time, not a block per program, because the
+// tiles of a list program take unequal time (cases are ordered by list
+// length): blocks spent half their warps' time at the barrier that ended a
+// program.  All programs' last tiles, the longest lists, come first, so that
+// the short ones fill the end of the launch.
+//
+// Dynamic shared memory: kExactSlots x 32 int64 per warp; 24 warps per SM.
+constexpr int kExactWarps = 8;
+constexpr size_t kExactSmem = size_t(kExactWarps) * kExactSlots * 32 * sizeof(int64_t);
+__device__ __noinline__ bool run_program_apart(const VmView& v, const int32_t* code, int n, const int64_t* consts,
+                                               int n_locals, int c, int64_t* value, int* tag, uint64_t* steps) {
+  return run_program(v, code, n, consts, n_locals, c, *value, *tag, *steps);
 }
-__global__ void __launch_bounds__(kGeneralWarps * 32) k_vm_general(const SearchDesc* descs, int mode,
-                                                                   const ProgramRef* list, const int32_t* list_count,
-                                                                   int bc_stride_max, ProgramRef* deferred,
-                                                                   int32_t* deferred_count) {
-  extern __shared__ __align__(16) int64_t smem_general[];
-  __shared__ int64_t red_loss[kGeneralWarps];
-  __shared__ uint32_t red_wrong[kGeneralWarps], red_errors[kGeneralWarps];
-  __shared__ unsigned long long red_steps[kGeneralWarps];
-  int64_t* consts = smem_general;
-  uint4* words = reinterpret_cast<uint4*>(smem_general + bc_stride_max);
-  int32_t* code = reinterpret_cast<int32_t*>(smem_general + 3 * size_t(bc_stride_max));
-  unsigned long long* targets =
-      reinterpret_cast<unsigned long long*>(smem_general + 3 * size_t(bc_stride_max) + (5 * size_t(bc_stride_max) + 1) / 2);
-  int64_t* slots_all = reinterpret_cast<int64_t*>(targets + (size_t(bc_stride_max) + 63) / 64);
-  const int count = *list_count;
+__global__ void __launch_bounds__(kExactWarps * 32, 3) k_vm_exact(const SearchDesc* descs, int mode, LowerLists lists,
+                                                                  unsigned long long* next, int max_C) {
+  extern __shared__ __align__(16) int64_t smem_exact[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int64_t* slots = slots_all + size_t(warp) * kSimdSlots * 32;
-  for (int i = blockIdx.x; i < count; i += gridDim.x) {
-    const ProgramRef p = list[i];
-    const SearchDesc& s = descs[p.search];
-    const int n = s.bc_len[p.slot], shape = s.bc_locals[p.slot];
-    const int n_locals = shape & 0xff, stack_bound = (shape >> 8) & 0xff;
-    if (((shape >> 16) & 0xffff) < n) {
-      // a program with bounded regions: k_vm_region runs it with a frame
-      // and memo workspace per lane
-      if (threadIdx.x == 0) deferred[atomicAdd(deferred_count, 1)] = p;
-      continue;
-    }
-    bool simd_ok = n_locals + stack_bound <= kSimdSlots;
-    {
-      const int32_t* gcode = s.bc + size_t(p.slot) * 5 * s.bc_stride;
-      const int64_t* gconsts = s.bc_consts + size_t(p.slot) * s.bc_stride;
-      for (int k = threadIdx.x; k < 5 * n; k += blockDim.x) code[k] = gcode[k];
-      for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        consts[k] = gconsts[k];  // at most one constant per instruction
-        const int32_t* x = gcode + 5 * k;
-        const int cost = x[4];
-        simd_ok &= cost >= 1 && cost <= 255 && x[0] >= 0 && x[0] < 64;
-        words[k] = simd_stage(gcode, k);
+  int64_t* slots = smem_exact + size_t(warp) * kExactSlots * 32;
+  const int tiles_max = (max_C + 31) / 32;
+  for (int which = 0; which < 2; ++which) {
+    const ProgramRef* list = which == 0 ? lists.exact : lists.general;
+    const unsigned long long count = which == 0 ? *lists.exact_count : *lists.general_count;
+    const unsigned long long items = count * tiles_max;
+    for (;;) {
+      if (!items) break;
+      unsigned long long item = 0;
+      if (lane == 0) item = atomicAdd(&next[which], 1ULL);
+      item = __shfl_sync(kFull, item, 0);
+      if (item >= items) break;
+      const ProgramRef p = list[item % count];
+      const SearchDesc& s = descs[p.search];
+      const int c = (tiles_max - 1 - int(item / count)) * 32 + lane;
+      if (c - lane >= s.C) continue;
+      const bool live = c < s.C;
+      const VmView view = vm_view(s);
+      const int32_t* code = s.bc + size_t(p.slot) * 5 * s.bc_stride;
+      const int64_t* consts = s.bc_consts + size_t(p.slot) * s.bc_stride;
+      int64_t loss = 0;
+      uint32_t wrong = 0, errors = 0;
+      uint64_t steps = 0;
+      bool ok = false;
+      int64_t value = 0;
+      int tag = s.result_type;
+      if (which == 0) {
+        const ExactCase r = run_exact(view, reinterpret_cast<const uint4*>(code), consts, c, live, slots);
+        ok = r.ok;
+        value = r.value;
+        steps = r.steps;
+      } else if (live) {
+        ok = run_program_apart(view, code, s.bc_len[p.slot], consts, s.bc_locals[p.slot] & 0xff, c, &value, &tag, &steps);
       }
-      for (int k = threadIdx.x; k < (n + 63) / 64; k += blockDim.x) targets[k] = 0;
-    }
-    simd_ok = __syncthreads_and(simd_ok);
-    if (simd_ok && threadIdx.x == 0) simd_fuse(code, n, words, targets);
-    __syncthreads();
-    const VmView view = vm_view(s);
-    int64_t loss = 0;
-    uint32_t wrong = 0, errors = 0;
-    uint64_t steps = 0;
-    if (simd_ok) {
-      for (int c0 = warp * 32; c0 < s.C; c0 += kGeneralWarps * 32) {
-        const int c = c0 + lane;
-        const bool live = c < s.C;
-        const SimdCase r = run_program_simd(view, words, n, consts, n_locals, c, live, slots);
-        if (live) {
-          if (r.ok) loss += case_loss(s, s.result_type, r.value, s.expected[c], wrong);
-          else { loss += error_loss(s); ++wrong; ++errors; }
-        }
-        steps += r.steps;
+      if (live) {
+        if (ok) loss = case_loss(s, tag, value, s.expected[c], wrong);
+        else { loss = error_loss(s); wrong = 1; errors = 1; }
       }
-    } else {
-      for (int c = threadIdx.x; c < s.C; c += blockDim.x) {
-        int64_t value = 0;
-        int tag = 0;
-        if (run_program(view, code, n, consts, n_locals, c, value, tag, steps)) {
-          loss += case_loss(s, tag, value, s.expected[c], wrong);
-        } else {
-          loss += error_loss(s);
-          ++wrong;
-          ++errors;
-        }
+      __syncwarp();
+      loss = warp_sum(loss);
+      wrong = warp_sum(wrong);
+      errors = warp_sum(errors);
+      steps = warp_sum(steps);
+      if (lane == 0) {
+        add_tile_result(s, mode, p.slot, unsigned((s.C + 31) / 32), loss, wrong, errors);
+        atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[24]), (unsigned long long)steps);
       }
     }
-    loss = warp_sum(loss);
-    wrong = warp_sum(wrong);
-    errors = warp_sum(errors);
-    steps = warp_sum(steps);
-    if (lane == 0) {
-      red_loss[warp] = loss;
-      red_wrong[warp] = wrong;
-      red_errors[warp] = errors;
-      red_steps[warp] = steps;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int64_t tl = 0;
-      uint32_t tw = 0, te = 0;
-      unsigned long long ts = 0;
-      for (int w = 0; w < kGeneralWarps; ++w) {
-        tl += red_loss[w];
-        tw += red_wrong[w];
-        te += red_errors[w];
-        ts += red_steps[w];
-      }
-      store_result(s, mode, p.slot, tl, tw);
-      if (mode == 0 && s.errors) s.errors[p.slot] = te;
-      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[24]), ts);
-      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[0]), 1ULL);
-      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[2]), (unsigned long long)s.C);
-    }
-    __syncthreads();
   }
 }
 
-// Programs with bounded regions (deferred by k_vm_general): a fixed grid of
+// Programs with bounded regions: a fixed grid of
 // persistent warps, each taking the next (program, group of cases) from
 // `next_item` (zeroed before the launch), one case per lane on the
 // per-thread interpreter (run_program_regions), each lane with its own

@@ -1,10 +1,11 @@
 // On-device lowering of a phase row.
 //
-// Two outputs per program:
+// Two outputs per program (a third, register code, is in exact.cuh):
 //  * the reference bytecode -- compile_phase_tree for value phases
 //    (cpp/src/evolution/repro/gpu/device/phase_compile.cuh:207-895) plus the
 //    RETURN that patch_whole_program appends (phase_layout.hpp:476-500) --
-//    executed by the exact general VM (fuel, errors, per-lane control flow);
+//    executed by the per-thread interpreter (run_program) and, with bounded
+//    regions, by run_program_regions;
 //  * an accumulator program for the fast VM, when the program is provably
 //    free of runtime errors and of fuel exhaustion: every operation is total
 //    (no unprotected division or modulo) and the bytecode length, an upper
@@ -1004,7 +1005,7 @@ __host__ __device__ __forceinline__ uint32_t accumulator_op_of(int node_kind, in
 }
 
 // Accumulator program of a row, by one warp; returns the instruction count
-// (the same on every lane), or -1 when the row needs the general VM.
+// (the same on every lane), or -1 when the row needs the exact VM.
 // *temps_out: temporaries used.  The lanes classify the nodes, number the
 // constants, copy the constant pool and bound the bytecode length in
 // parallel, then emit the code together (lower_accumulator_emit).
@@ -1028,7 +1029,7 @@ __device__ inline int lower_accumulator_warp(const SearchDesc& s, const uint64_t
       if (arity == 0) {
         m.aop[i] = kLeafOp;
         // the accumulator VM reads constants and Int/Bool inputs; a bound
-        // read (a traversal binder) needs the general VM
+        // read (a traversal binder) needs the exact VM
         total &= nk == TK_CONSTANT || nk == TK_LOCAL;
       } else {
         const uint32_t op = accumulator_op_of(nk, __ldg(&info[o].opcode), __ldg(&info[o].operand));

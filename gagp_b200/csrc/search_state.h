@@ -239,7 +239,7 @@ struct SearchDesc {
   // ---- lowered programs (children, or members during the initial evaluation)
   uint2* code; int32_t* code_len; int64_t* kpool;
   int32_t code_stride;                 // accumulator instructions per program slot
-  int32_t* code_temps;                 // temporaries; <0: needs the general VM
+  int32_t* code_temps;                 // temporaries; an interpreter program: its main constants
   // per program slot, the fast VM's tile accumulators: [2 slot] loss (bits
   // 0-39) | wrong cases (40-55) | tiles done (56-63) when the search's case
   // count and penalty fit those fields; otherwise [2 slot] the loss sum and

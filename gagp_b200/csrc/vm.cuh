@@ -335,7 +335,7 @@ __device__ inline void run_accumulator(const SearchDesc& s, int slot, const VmWa
   ops_out = uint64_t(len) * uint64_t(case_end - case_begin);
 }
 
-// ------------------------------------------------------------ general VM
+// ------------------------------------------------------------ interpreter
 // What the exact VM reads of a search: the case inputs (input-major), their
 // tags, the IntList arena and the fuel.
 struct VmView {
@@ -793,256 +793,6 @@ __host__ __device__ inline bool run_program_regions(const VmView& v, const Regio
   const RegionRun rr{regions, n_regions, code + 5 * n_main, n - n_main, consts + main_consts, ws, ws_words};
   int fuel = v.fuel;
   return run_code<false>(v, code, n_main, consts, n_locals, lv, lt, set, fuel, &rr, value, tag, steps);
-}
-
-// ------------------------------------------------------------ warp-SIMD exact VM
-// The exact VM for the 32 cases of one tile, executed by one warp with one
-// decoded instruction at a time: every lane keeps its own instruction
-// pointer, fuel and result, and at each step the lanes whose pointer is the
-// smallest among the running lanes execute the instruction there together
-// (a warp-uniform opcode, so no divergence inside the step).  Lanes that
-// are ahead -- past a branch the others did not take, or out of a loop the
-// others are still in -- wait until the others reach them, so branch joins
-// and loop exits re-merge the warp.  The thread-per-case VM instead lets the
-// lanes drift apart, after which every distinct opcode of a step runs
-// serially.
-//
-// The stack and the locals live in shared memory as [slot][lane] columns of
-// int64 payloads: locals first (inputs preset), then the stack.  Tags are
-// not kept: the lowering's output is well typed (each operation's operands
-// have the grammar's types, the stack depth and the definedness of every
-// local are fixed per instruction), so none of the reference VM's type,
-// underflow or uninitialised-local checks can fail on it and the result's
-// tag is the phase's type; the checks that can fail on some case -- fuel,
-// modulo by zero, index range -- are kept.  Results equal run_program's.
-//
-// Staged instruction (uint4): x = op (bits 0-6) | jump when true (bit 7) |
-// instructions it stands for (bits 8-11) | binary operation (bits 12-15) |
-// their summed fuel (bits 16-31); y, z, w: operands.  The kernel stages a
-// program this way only when every cost is in 1..255 and its locals and
-// stack fit kSimdSlots; otherwise it runs it on run_program.
-//
-// Superinstructions.  One thread of the block fuses, left to right, short
-// straight-line runs that start anywhere but hold no jump target past their
-// first instruction: LOAD a; LOAD b; op; STORE c (S_BIN_LL_ST), the same
-// with PUSH_CONST k for the second load (S_BIN_LC_ST), LOAD a; LOAD b / PUSH
-// k; comparison; JMP_IF_FALSE/TRUE t (S_JCMP_LL / S_JCMP_LC), LOAD a; LOAD b;
-// CALL index; STORE c (S_INDEX_LL_ST), the three-instruction prefixes of the
-// binary forms (S_BIN_LL, S_BIN_LC), op; STORE c (S_BIN_ST) and LOAD a;
-// STORE c (S_MOVE).  A fused instruction charges the summed fuel before it
-// runs (a timeout anywhere inside the run, or an error of one of its
-// instructions, ends the case with an error in both forms, and otherwise
-// every instruction runs) and counts as the instructions it stands for.  The
-// skipped slots are never reached: jumps land only on run starts.
-enum : int {
-  S_MOVE = 64, S_BIN_LL, S_BIN_LC, S_BIN_LL_ST, S_BIN_LC_ST, S_JCMP_LL, S_JCMP_LC, S_INDEX_LL_ST, S_BIN_ST, S_FAIL
-};
-constexpr int kSimdSlots = 24;
-constexpr int kSimdDone = 0x7fffffff;
-
-__device__ __forceinline__ uint4 simd_plain(int op, int a, int cost) {
-  return make_uint4(uint32_t(op & 0x7f) | (1u << 8) | (uint32_t(cost) << 16), uint32_t(a), 0u, 0u);
-}
-// The staged word of instruction k of `code` (5 ints per instruction).  The
-// one type error the lowering emits on purpose -- NEG of the Bool constant
-// that a for_range pushes for a bound that is not a non-negative Int --
-// stages as S_FAIL, which charges the NEG's fuel and fails the case as the
-// reference's NEG does; every other NEG has an Int operand.
-__device__ __forceinline__ uint4 simd_stage(const int32_t* code, int k) {
-  const int32_t* x = code + 5 * k;
-  const bool bool_neg = x[0] == OP_NEG && k > 0 && code[5 * (k - 1)] == OP_PUSH_CONST &&
-                        (code[5 * (k - 1) + 1] & kBoolConst);
-  return simd_plain(bool_neg ? S_FAIL : x[0], x[2], x[4]);
-}
-__device__ __forceinline__ bool simd_binary_op(int op) {
-  return op == OP_ADD || op == OP_SUB || op == OP_MUL || op == OP_MOD || (op >= OP_LT && op <= OP_NE);
-}
-__device__ __forceinline__ bool simd_compare_op(int op) { return op >= OP_LT && op <= OP_NE; }
-// One binary operation of the reference VM on Int payloads (comparisons give
-// 0/1); false on a modulo by zero (ZeroDiv).
-__device__ __forceinline__ bool simd_binary(int op, int64_t x, int64_t y, int64_t& r) {
-  switch (op) {
-    case OP_ADD: r = wrap_add(x, y); return true;
-    case OP_SUB: r = wrap_sub(x, y); return true;
-    case OP_MUL: r = wrap_mul(x, y); return true;
-    case OP_MOD:
-      if (y == 0) return false;
-      r = py_mod(x, y);
-      return true;
-    case OP_LT: r = x < y; return true;
-    case OP_LE: r = x <= y; return true;
-    case OP_GT: r = x > y; return true;
-    case OP_GE: r = x >= y; return true;
-    case OP_EQ: r = x == y; return true;
-    default: r = x != y; return true;
-  }
-}
-
-// The fusion pass over a staged program (code: 5 ints per instruction; words
-// hold the plain staging; targets: n bits, zeroed).  One thread.
-__device__ inline void simd_fuse(const int32_t* code, int n, uint4* words, unsigned long long* targets) {
-  auto op_at = [&](int k) { return code[5 * k]; };
-  auto a_at = [&](int k) { return code[5 * k + 2]; };
-  auto cost_at = [&](int k) { return uint32_t(code[5 * k + 4]); };
-  for (int k = 0; k < n; ++k) {
-    const int op = op_at(k), t = a_at(k);
-    if ((op == OP_JMP || op == OP_JMP_IF_FALSE || op == OP_JMP_IF_TRUE) && t >= 0 && t < n)
-      targets[t >> 6] |= 1ull << (t & 63);
-  }
-  // instructions k+1 .. k+len-1 exist and none is a jump target
-  auto free_run = [&](int k, int len) {
-    if (k + len > n) return false;
-    for (int j = 1; j < len; ++j)
-      if (targets[(k + j) >> 6] >> ((k + j) & 63) & 1) return false;
-    return true;
-  };
-  auto fused = [&](int k, int len, int op, int bop, bool jt, uint32_t y, uint32_t z, uint32_t w) {
-    uint32_t cost = 0;
-    for (int j = 0; j < len; ++j) cost += cost_at(k + j);
-    words[k] = make_uint4(uint32_t(op) | (uint32_t(jt) << 7) | (uint32_t(len) << 8) | (uint32_t(bop - OP_ADD) << 12) |
-                              (cost << 16),
-                          y, z, w);
-  };
-  for (int k = 0; k < n;) {
-    const int o0 = op_at(k), o1 = k + 1 < n ? op_at(k + 1) : -1, o2 = k + 2 < n ? op_at(k + 2) : -1,
-              o3 = k + 3 < n ? op_at(k + 3) : -1;
-    const bool second = o1 == OP_LOAD || o1 == OP_PUSH_CONST;
-    int len = 1;
-    if (o0 == OP_LOAD && second && simd_binary_op(o2) && o3 == OP_STORE && free_run(k, 4)) {
-      fused(k, 4, o1 == OP_LOAD ? S_BIN_LL_ST : S_BIN_LC_ST, o2, false, a_at(k), a_at(k + 1), a_at(k + 3));
-      len = 4;
-    } else if (o0 == OP_LOAD && second && simd_compare_op(o2) && (o3 == OP_JMP_IF_FALSE || o3 == OP_JMP_IF_TRUE) &&
-               free_run(k, 4)) {
-      fused(k, 4, o1 == OP_LOAD ? S_JCMP_LL : S_JCMP_LC, o2, o3 == OP_JMP_IF_TRUE, a_at(k), a_at(k + 1), a_at(k + 3));
-      len = 4;
-    } else if (o0 == OP_LOAD && o1 == OP_LOAD && o2 == OP_CALL_BUILTIN && a_at(k + 2) == B_INDEX && o3 == OP_STORE &&
-               free_run(k, 4)) {
-      fused(k, 4, S_INDEX_LL_ST, OP_ADD, false, a_at(k), a_at(k + 1), a_at(k + 3));
-      len = 4;
-    } else if (o0 == OP_LOAD && second && simd_binary_op(o2) && free_run(k, 3)) {
-      fused(k, 3, o1 == OP_LOAD ? S_BIN_LL : S_BIN_LC, o2, false, a_at(k), a_at(k + 1), 0);
-      len = 3;
-    } else if (simd_binary_op(o0) && o1 == OP_STORE && free_run(k, 2)) {
-      fused(k, 2, S_BIN_ST, o0, false, a_at(k + 1), 0, 0);
-      len = 2;
-    } else if (o0 == OP_LOAD && o1 == OP_STORE && free_run(k, 2)) {
-      fused(k, 2, S_MOVE, OP_ADD, false, a_at(k), a_at(k + 1), 0);
-      len = 2;
-    }
-    k += len;
-  }
-}
-
-struct SimdCase {
-  int64_t value;
-  bool ok;
-  uint32_t steps;
-};
-
-__device__ inline SimdCase run_program_simd(const VmView& v, const uint4* code, int n, const int64_t* consts,
-                                            int n_locals, int c, bool live, int64_t* slots) {
-  const int lane = threadIdx.x & 31;
-  SimdCase out{0, false, 0};
-  // locals [0, n_locals): inputs preset; the stack follows
-  for (int j = 0; j < v.n_inputs; ++j)
-    if (live) slots[j * 32 + lane] = __ldg(&v.inputs[size_t(j) * v.C + c]);
-  int ip = live ? 0 : kSimdDone, sp = n_locals, fuel = v.fuel;
-  auto at = [&](int k) -> int64_t& { return slots[k * 32 + lane]; };
-  for (;;) {
-    const int ipm = __reduce_min_sync(kFull, ip);
-    if (ipm == kSimdDone) break;
-    if (ip != ipm) continue;
-    const uint4 w = code[ipm];
-    const int op = int(w.x & 0x7fu), len = int((w.x >> 8) & 0xfu), bop = OP_ADD + int((w.x >> 12) & 0xfu);
-    const int cost = int(w.x >> 16), a = int(w.y);
-    if (fuel < cost) { ip = kSimdDone; continue; }  // Timeout
-    fuel -= cost;
-    out.steps += len;
-    ip += len;
-    switch (op) {
-      case OP_PUSH_CONST: at(sp++) = consts[a]; break;
-      case OP_LOAD: { const int64_t x = at(a); at(sp++) = x; break; }
-      case OP_STORE: at(a) = at(--sp); break;
-      case OP_CHECK_INT: break;
-      case OP_NEG: at(sp - 1) = wrap_neg(at(sp - 1)); break;
-      case OP_NOT: at(sp - 1) ^= 1; break;
-      case OP_ADD: case OP_SUB: case OP_MUL: case OP_MOD:
-      case OP_LT: case OP_LE: case OP_GT: case OP_GE: case OP_EQ: case OP_NE: {
-        const int64_t y = at(--sp), x = at(sp - 1);
-        int64_t r;
-        if (!simd_binary(op, x, y, r)) { ip = kSimdDone; break; }  // ZeroDiv
-        at(sp - 1) = r;
-        break;
-      }
-      case OP_JMP: ip = a; break;
-      case OP_JMP_IF_FALSE: case OP_JMP_IF_TRUE: {
-        const int64_t y = at(--sp);
-        if ((op == OP_JMP_IF_FALSE) == (y == 0)) ip = a;
-        break;
-      }
-      case OP_CALL_BUILTIN: {
-        int64_t r = 0;
-        if (a == B_IS_INT) {
-          r = 1;  // a for_range bound: an Int in a well-typed program
-        } else if (a == B_LEN) {
-          r = __ldg(&v.lists[at(sp - 1)]);
-        } else if (a == B_INDEX) {
-          const int64_t j0 = at(--sp), h = at(sp - 1), len_h = __ldg(&v.lists[h]);
-          const int64_t j = j0 < 0 ? j0 + len_h : j0;
-          if (j < 0 || j >= len_h) { ip = kSimdDone; break; }  // index out of range
-          r = __ldg(&v.lists[h + 1 + j]);
-        } else if (a == B_ABS) {
-          const int64_t x = at(sp - 1);
-          r = x < 0 ? wrap_neg(x) : x;
-        } else {
-          const int64_t q = at(--sp), p = at(sp - 1);
-          r = a == B_MIN ? (p < q ? p : q) : a == B_MAX ? (p > q ? p : q) : a == B_IDIV0 ? idiv0(p, q)
-            : a == B_IMOD0 ? imod0(p, q) : a == B_TRUNC_DIV0 ? tdiv0(p, q) : tmod0(p, q);
-        }
-        at(sp - 1) = r;
-        break;
-      }
-      case OP_RETURN:
-        out.value = at(sp - 1);
-        out.ok = true;
-        ip = kSimdDone;
-        break;
-      case S_MOVE: at(int(w.z)) = at(a); break;
-      case S_BIN_LL: case S_BIN_LC: case S_BIN_LL_ST: case S_BIN_LC_ST: {
-        const int64_t x = at(a), y = (op == S_BIN_LL || op == S_BIN_LL_ST) ? at(int(w.z)) : consts[w.z];
-        int64_t r;
-        if (!simd_binary(bop, x, y, r)) { ip = kSimdDone; break; }  // ZeroDiv
-        if (op == S_BIN_LL || op == S_BIN_LC) at(sp++) = r;
-        else at(int(w.w)) = r;
-        break;
-      }
-      case S_JCMP_LL: case S_JCMP_LC: {
-        const int64_t x = at(a), y = op == S_JCMP_LL ? at(int(w.z)) : consts[w.z];
-        int64_t r;
-        simd_binary(bop, x, y, r);  // a comparison: never fails
-        if ((r != 0) == bool(w.x & 0x80u)) ip = int(w.w);
-        break;
-      }
-      case S_INDEX_LL_ST: {
-        const int64_t h = at(a), j0 = at(int(w.z)), len_h = __ldg(&v.lists[h]);
-        const int64_t j = j0 < 0 ? j0 + len_h : j0;
-        if (j < 0 || j >= len_h) { ip = kSimdDone; break; }  // index out of range
-        at(int(w.w)) = __ldg(&v.lists[h + 1 + j]);
-        break;
-      }
-      case S_BIN_ST: {
-        const int64_t y = at(--sp), x = at(--sp);
-        int64_t r;
-        if (!simd_binary(bop, x, y, r)) { ip = kSimdDone; break; }  // ZeroDiv
-        at(a) = r;
-        break;
-      }
-      case S_FAIL: ip = kSimdDone; break;  // NEG of a Bool: a type error
-      default:
-        ip = kSimdDone;  // not emitted by the lowering
-    }
-  }
-  return out;
 }
 
 }  // namespace gb

@@ -1,0 +1,106 @@
+"""Register code on the exact VM against the interpreter of the reference
+bytecode (GPU).
+
+The device lowers list, let, statement and charged programs straight to
+register code and sums their fuel per straight-line stretch; the host
+harness lowers the same rows to the reference's bytecode and runs it
+instruction by instruction (both pinned to the reference by
+test_lower_host.py).  Every program must score the same at case counts around
+the VM's tiles and at fuels that run out before, inside and after its loops,
+and programs with more constants than the VM keeps in slots must too.  All
+scores are integers, so the comparison is exact."""
+import copy
+import glob
+import gzip
+import json
+import os
+
+import numpy as np
+import pytest
+
+from gagp_b200 import abi, grammar as G, task as T, workloads as W
+from oracle import oracle
+
+import golden_util as GU
+import host_harness as H
+
+pytestmark = pytest.mark.gpu
+LOWER_DIR = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "lower")
+NAMES = sorted(os.path.basename(p)[:-len(".json.gz")] for p in glob.glob(os.path.join(LOWER_DIR, "*.json.gz"))
+               if "grid" not in p)
+
+
+@pytest.fixture(scope="module")
+def engine():
+    from gagp_b200 import build
+    from gagp_b200.engine import Engine
+    build.build()
+    with Engine(0) as e:
+        yield e
+
+
+def _cycled(cases, n):
+    at = np.arange(n) % len(cases.expected)
+    return abi.CasesBlob(cases.inputs[at], cases.input_tags, cases.expected[at], cases.expected_tag, cases.list_values)
+
+
+def _expected(lt, rows, programs, fuel):
+    """Fitness and wrong count of each lowered program by the interpreter."""
+    cases, penalty = lt.cases, int(abs(lt.settings.penalty))
+    fitness, wrong = [], []
+    for code, consts, n_locals, _ in programs:
+        loss = bad = 0
+        for c in range(len(cases.expected)):
+            ok, value, tag, _ = H.run(cases, lt.tables.local_types, fuel, code, consts, n_locals, c)
+            want = int(cases.expected[c])
+            same = ok and tag == cases.expected_tag and value == want
+            bad += not same
+            if lt.settings.metric == "exact":
+                loss += not same
+            elif not ok or tag != G.TAG_INT or cases.expected_tag != G.TAG_INT:
+                loss += penalty
+            else:
+                loss += min(abs(value - want), penalty)
+        fitness.append(float(-loss))
+        wrong.append(bad)
+    return fitness, wrong
+
+
+@pytest.mark.parametrize("name", NAMES)
+@pytest.mark.parametrize("count,fuel", [(1, None), (31, 40), (33, 173), (65, 9)])
+def test_register_code_matches_interpreter(engine, name, count, fuel):
+    with gzip.open(os.path.join(LOWER_DIR, name + ".json.gz"), "rt") as f:
+        fx = json.load(f)
+    lt = GU.load_task(fx)
+    blob = abi.GrammarBlob(lt.tables)
+    picked = [r for r in fx["lower"]["rows"] if r["status"] == 0][:48]
+    rows = abi.RowsBuffer.from_rows([(r["origins"], r["constants"]) for r in picked],
+                                    lt.tables.max_nodes - lt.tables.fixed_nodes)
+    lt.cases = _cycled(lt.cases, count)
+    lt.settings.fuel = fuel or lt.settings.fuel
+    programs = [H.lower(blob, r["origins"], r["constants"]) for r in picked]
+    got_f, got_w = engine.evaluate_rows(lt, rows)
+    want_f, want_w = _expected(lt, rows, programs, lt.settings.fuel)
+    assert list(got_f) == want_f
+    assert list(got_w) == want_w
+
+
+def test_programs_of_many_constants(engine):
+    files = W.list_threshold(population=96, generations=2, seed=11, cases=40)
+    grammar = copy.deepcopy(files.grammar)
+    for alt in grammar["nonterminals"][2]["alternatives"]:
+        if alt["id"] == "one":
+            alt["weight"] = 6
+            alt["expression"] = {"constant": {"type": "Int", "range": ["-40000000000", "40000000000"]}}
+        if alt["id"] in ("add", "sub"):
+            alt["weight"] = 8
+    files.grammar = grammar
+    lt = T.from_files(files)
+    blob = abi.GrammarBlob(lt.tables)
+    rows = oracle.initial_population(blob, lt.settings)
+    assert max(len(set(rows.row(i)[1])) for i in range(rows.count)) > 8
+    programs = [H.lower(blob, *rows.row(i)) for i in range(rows.count)]
+    got_f, got_w = engine.evaluate_rows(lt, rows)
+    want_f, want_w = _expected(lt, rows, programs, lt.settings.fuel)
+    assert list(got_f) == want_f
+    assert list(got_w) == want_w
