@@ -234,14 +234,16 @@ void harvest(gagp_engine* e) {
 // Device counters of a round: per variation range c, [4c] its accumulator
 // program list's size and [4c+2] its next child; then the sizes of the lists
 // the ranges share -- accumulator programs (of exact-heavy rounds), register
-// code, interpreter programs, programs with bounded regions -- and, 64 bits
-// each, the next items of the exact VM's two lists and the region kernel's.
+// code of few and of many slots, interpreter programs, programs with bounded
+// regions -- and, 64 bits each, the next items of the exact VM's three lists
+// and the region kernel's.
 constexpr int kSharedFast = 4 * gagp_engine::kChunks;
 constexpr int kExactCount = kSharedFast + 1;
-constexpr int kGeneralCount = kSharedFast + 2;
-constexpr int kRegionCount = kSharedFast + 3;
-constexpr int kExactNext = kSharedFast + 4;
-constexpr int kRegionNext = kExactNext + 4;
+constexpr int kWideCount = kSharedFast + 2;
+constexpr int kGeneralCount = kSharedFast + 3;
+constexpr int kRegionCount = kSharedFast + 4;
+constexpr int kExactNext = kSharedFast + 6;
+constexpr int kRegionNext = kExactNext + 6;
 constexpr int kCountWords = kRegionNext + 2;
 gagp_status ensure_region_workspace(gagp_engine* e, size_t words);
 
@@ -1599,7 +1601,7 @@ void vm_fast_launch(int lanes, int blocks, int threads, size_t smem, cudaStream_
 // and a quarter of the SMs take them.
 void vm_exact_launch(int sm_count, cudaStream_t stream, const gb::SearchDesc* descs, int mode,
                      const gb::LowerLists& lists, int32_t* next, int max_C, bool heavy) {
-  const int blocks = heavy ? 3 * sm_count : std::max(1, sm_count / 4);
+  const int blocks = heavy ? gb::kExactBlocks * sm_count : std::max(1, sm_count / 4);
   gb::k_vm_exact<<<blocks, gb::kExactWarps * 32, gb::kExactSmem, stream>>>(
       descs, mode, lists, reinterpret_cast<unsigned long long*>(next), max_C);
 }
@@ -1614,8 +1616,8 @@ void lower_launch(cudaStream_t stream, const gb::SearchDesc* descs, const int32_
 // counter word `fast_word`.
 gb::LowerLists engine_lists(gagp_engine* e, gb::ProgramRef* fast, int fast_word) {
   int32_t* c = e->d_counts;
-  return gb::LowerLists{fast, e->d_exact, e->d_general, e->d_region, c + fast_word, c + kExactCount, c + kGeneralCount,
-                        c + kRegionCount};
+  return gb::LowerLists{fast, e->d_exact, e->d_general, e->d_region, int(e->list_capacity), c + fast_word,
+                        c + kExactCount, c + kWideCount, c + kGeneralCount, c + kRegionCount};
 }
 
 constexpr int kRegionBlocks = 4, kRegionLanes = 16;  // of the bounded-region kernel: per SM, and per warp
@@ -1998,9 +2000,9 @@ struct EvalPlan {
   int stride, code_stride, bc_stride;
   size_t region_words;  // bounded-region workspace per lane (0: the grammar has none)
 };
-// Counter words of a row evaluation: the four lists' sizes, then the next
-// items (64 bits) of the exact VM's two lists and the region kernel's.
-constexpr int kRowCountWords = 10;
+// Counter words of a row evaluation: the lists' sizes, then (64 bits, from
+// word 6) the next items of the exact VM's three lists and the region kernel's.
+constexpr int kRowCountWords = 14;
 // A row evaluation's bounded-region kernel: blocks, and lanes per warp.
 constexpr int kRowRegionBlocks = 256, kRowRegionLanes = 8;
 
@@ -2194,7 +2196,8 @@ gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g,
   gb::ProgramRef* fast = at<gb::ProgramRef>(b, p.fast);
   int32_t* counts = at<int32_t>(b, p.counts);
   const gb::LowerLists lists{fast, at<gb::ProgramRef>(b, p.exact), at<gb::ProgramRef>(b, p.general),
-                             at<gb::ProgramRef>(b, p.region_list), counts, counts + 1, counts + 2, counts + 3};
+                             at<gb::ProgramRef>(b, p.region_list), R, counts, counts + 1, counts + 2, counts + 3,
+                             counts + 4};
   const bool exact = exact_possible(g, cfg->fuel);
   lower_launch(stream, dd, doff, 1, 0, lists, 0, R, exact);
   const int warps = 8;
@@ -2206,10 +2209,10 @@ gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g,
   const int per_sm = std::max(1, std::min(4, int((max_smem - 1024) / smem)));
   vm_fast_launch(lanes, sm_count * per_sm, warps * 32, smem, stream, dd, 0, fast, counts, temp_stride, code_stride,
                  p.stride, C);
-  if (exact) vm_exact_launch(sm_count, stream, dd, 0, lists, counts + 4, C, true);
+  if (exact) vm_exact_launch(sm_count, stream, dd, 0, lists, counts + 6, C, true);
   if (p.region_words)
     gb::k_vm_region<<<kRowRegionBlocks, gb::kRegionThreads, 0, stream>>>(
-        dd, 0, lists.region, counts + 3, reinterpret_cast<unsigned long long*>(counts + 8), C, kRowRegionLanes,
+        dd, 0, lists.region, counts + 4, reinterpret_cast<unsigned long long*>(counts + 12), C, kRowRegionLanes,
         at<int64_t>(b, p.region_ws), p.region_words);
   CUDA_TRY(cudaGetLastError());
   int32_t round[4];

@@ -75,9 +75,12 @@ __global__ void k_init_population(const SearchDesc* descs, const int32_t* off, i
 // Where lowered programs are listed, with each list's size: accumulator
 // programs, register code, reference bytecode for the per-thread
 // interpreter, and programs with bounded regions.
+// Register code shares one list of `exact_capacity`: programs of at most
+// kExactNarrow slots from its front, the others from its back.
 struct LowerLists {
   ProgramRef *fast, *exact, *general, *region;
-  int32_t *fast_count, *exact_count, *general_count, *region_count;
+  int exact_capacity;
+  int32_t *fast_count, *exact_count, *wide_count, *general_count, *region_count;
 };
 // mode 0: the members (initial evaluation); mode 1: this round's children
 // that reuse no member's result; batch items [lo, hi).  One warp per row:
@@ -153,11 +156,14 @@ __global__ void __launch_bounds__(kLowerWarps * 32, Exact ? 7 : 8)
     } else {
       int32_t* bc = s.bc + size_t(slot) * 5 * s.bc_stride;
       int64_t* bc_consts = s.bc_consts + size_t(slot) * s.bc_stride;
+      int slots = 0;
       const int exact = lower_exact_warp(s, t.node, t.n, t.cval, t.nc, reinterpret_cast<uint4*>(bc),
-                                         s.bc_stride * 5 / 4, bc_consts, scratch[warp].exact);
+                                         s.bc_stride * 5 / 4, bc_consts, scratch[warp].exact, &slots);
       if (lane == 0) {
         if (exact >= 0) {
-          lists.exact[atomicAdd(lists.exact_count, 1)] = ProgramRef{si, slot};
+          const int at = slots <= kExactNarrow ? atomicAdd(lists.exact_count, 1)
+                                               : lists.exact_capacity - 1 - atomicAdd(lists.wide_count, 1);
+          lists.exact[at] = ProgramRef{si, slot};
           atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[9]),
                     (unsigned long long)(row_bytes + 16ull * (exact + 1) + 16));
         } else {
@@ -240,8 +246,9 @@ __device__ __forceinline__ bool add_tile_result(const SearchDesc& s, int mode, i
 
 // The exact VMs: the programs the accumulator VM cannot run.  Persistent
 // warps, each taking the next (program, tile of 32 cases) from `next`
-// (next[0] register code, next[1] the interpreter's programs; zeroed before
-// the launch).  A tile adds its sums to the program's accumulators.
+// (zeroed before the launch): next[0] register code of few slots, next[1] of
+// many, next[2] the interpreter's programs.  A tile adds its sums to the
+// program's accumulators.
 //
 // Tiles are taken one warp at a time, not a block per program, because the
 // tiles of a list program take unequal time (cases are ordered by list
@@ -249,32 +256,46 @@ __device__ __forceinline__ bool add_tile_result(const SearchDesc& s, int mode, i
 // program.  All programs' last tiles, the longest lists, come first, so that
 // the short ones fill the end of the launch.
 //
-// Dynamic shared memory: kExactSlots x 32 int64 per warp; 24 warps per SM.
-constexpr int kExactWarps = 8;
-constexpr size_t kExactSmem = size_t(kExactWarps) * kExactSlots * 32 * sizeof(int64_t);
+// Dynamic shared memory per warp: kExactNarrow x 32 int64, and the code of a
+// program of up to kExactStaged - 1 instructions (a longer one is read in
+// place).  Programs of more slots run afterwards on every second warp, with
+// the next warp's slots too.
+constexpr int kExactWarps = 8, kExactBlocks = 4, kExactStaged = 64;
+static_assert(kExactSlots == 2 * kExactNarrow, "a wide program takes two warps' slots");
+constexpr size_t kExactSmem = size_t(kExactWarps) * (kExactNarrow * 32 * sizeof(int64_t) + kExactStaged * sizeof(uint4));
 __device__ __noinline__ bool run_program_apart(const VmView& v, const int32_t* code, int n, const int64_t* consts,
                                                int n_locals, int c, int64_t* value, int* tag, uint64_t* steps) {
   return run_program(v, code, n, consts, n_locals, c, *value, *tag, *steps);
 }
-__global__ void __launch_bounds__(kExactWarps * 32, 3) k_vm_exact(const SearchDesc* descs, int mode, LowerLists lists,
-                                                                  unsigned long long* next, int max_C) {
+__global__ void __launch_bounds__(kExactWarps * 32, kExactBlocks) k_vm_exact(const SearchDesc* descs, int mode,
+                                                                             LowerLists lists,
+                                                                             unsigned long long* next, int max_C) {
   extern __shared__ __align__(16) int64_t smem_exact[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int64_t* slots = smem_exact + size_t(warp) * kExactSlots * 32;
-  const int tiles_max = (max_C + 31) / 32;
-  for (int which = 0; which < 2; ++which) {
-    const ProgramRef* list = which == 0 ? lists.exact : lists.general;
-    const unsigned long long count = which == 0 ? *lists.exact_count : *lists.general_count;
-    const unsigned long long items = count * tiles_max;
+  int64_t* slots = smem_exact + size_t(warp) * kExactNarrow * 32;
+  uint4* staged = reinterpret_cast<uint4*>(smem_exact + size_t(kExactWarps) * kExactNarrow * 32) + warp * kExactStaged;
+  const unsigned tiles_max = unsigned(max_C + 31) / 32;
+  for (int which = 0; which < 3; ++which) {
+    const unsigned count = unsigned(which == 0 ? *lists.exact_count : which == 1 ? *lists.wide_count : *lists.general_count);
+    const unsigned long long items = (unsigned long long)count * tiles_max;
+    if (which == 1) {
+      if (!items) continue;
+      __syncthreads();  // the narrow programs' slots are free
+      if (warp & 1) continue;
+    }
     for (;;) {
       if (!items) break;
       unsigned long long item = 0;
       if (lane == 0) item = atomicAdd(&next[which], 1ULL);
       item = __shfl_sync(kFull, item, 0);
       if (item >= items) break;
-      const ProgramRef p = list[item % count];
+      const unsigned turn = items >> 32 ? unsigned(item / count) : unsigned(item) / count;
+      const unsigned index = unsigned(item - (unsigned long long)turn * count);
+      const ProgramRef p = which == 0   ? lists.exact[index]
+                           : which == 1 ? lists.exact[lists.exact_capacity - 1 - int(index)]
+                                        : lists.general[index];
       const SearchDesc& s = descs[p.search];
-      const int c = (tiles_max - 1 - int(item / count)) * 32 + lane;
+      const int c = int(tiles_max - 1 - turn) * 32 + lane;
       if (c - lane >= s.C) continue;
       const bool live = c < s.C;
       const VmView view = vm_view(s);
@@ -286,8 +307,16 @@ __global__ void __launch_bounds__(kExactWarps * 32, 3) k_vm_exact(const SearchDe
       bool ok = false;
       int64_t value = 0;
       int tag = s.result_type;
-      if (which == 0) {
-        const ExactCase r = run_exact(view, reinterpret_cast<const uint4*>(code), consts, c, live, slots);
+      if (which < 2) {
+        const uint4* words = reinterpret_cast<const uint4*>(code);
+        const uint4 head = __ldg(words);
+        const int n = int(head.x & 0xffffu);
+        const bool fits = n < kExactStaged;
+        if (fits)
+          for (int k = lane; k <= n; k += 32) staged[k] = __ldg(&words[1 + k]);
+        __syncwarp();
+        const ExactCase r = run_exact(view, fits ? staged : words + 1, head, consts, c, live, slots);
+        __syncwarp();
         ok = r.ok;
         value = r.value;
         steps = r.steps;

@@ -104,3 +104,24 @@ def test_programs_of_many_constants(engine):
     want_f, want_w = _expected(lt, rows, programs, lt.settings.fuel)
     assert list(got_f) == want_f
     assert list(got_w) == want_w
+
+
+@pytest.mark.parametrize("cases", [33, 96])
+def test_long_programs(engine, cases):
+    """Programs of up to 200 nodes over a modulo that can fail: register code
+    past what a warp stages in shared memory, ifs too large for a select."""
+    files = W.poly4(population=256, generations=2, seed=3, cases=cases, max_nodes=200)
+    grammar = copy.deepcopy(files.grammar)
+    for alt in grammar["nonterminals"][0]["alternatives"]:
+        alt["weight"] = {"x": 2, "c": 1, "iflt": 3}.get(alt["id"], 2)
+        if alt["id"] == "imod0":
+            alt["expression"]["signature"] = "mod(Int,Int)->Int"
+    files.grammar = grammar
+    lt = T.from_files(files)
+    blob = abi.GrammarBlob(lt.tables)
+    rows = oracle.initial_population(blob, lt.settings)
+    assert max(rows.node_counts) > 150
+    got_f, got_w = engine.evaluate_rows(lt, rows)
+    want_f, want_w, _ = oracle.evaluate(blob, lt.cases, lt.settings, rows)
+    assert np.array_equal(got_f, want_f)
+    assert np.array_equal(got_w, want_w)
