@@ -1493,7 +1493,7 @@ struct BatchView {
   long long max_draws = 0;
   int max_code_stride = 2;
   int max_C = 1, max_inputs = 0;
-  int min_B = 1 << 30;               // the smallest round of the batch
+  int max_B = 0;                     // the largest round of the batch
   bool exact_heavy = false;          // some search's programs mostly need the exact VM
   bool exact_possible = false;       // some search's programs may need it
   bool regions = false;              // some search's grammar has bounded regions
@@ -1554,6 +1554,7 @@ gagp_status make_batch_view(gagp_engine* e, const std::vector<Search*>& list, Ba
   v->max_draws = 0;
   v->max_code_stride = 2;
   v->max_lanes = 1;
+  v->max_B = 0;
   v->max_C = 1;
   v->max_inputs = 0;
   v->exact_heavy = v->exact_possible = false;
@@ -1576,7 +1577,7 @@ gagp_status make_batch_view(gagp_engine* e, const std::vector<Search*>& list, Ba
     v->max_stride = std::max(v->max_stride, s->stride);
     v->max_code_stride = std::max(v->max_code_stride, s->desc.code_stride);
     v->max_draws = std::max(v->max_draws, (long long)s->B * s->desc.replacement_size + 1);
-    v->min_B = std::min(v->min_B, s->B);
+    v->max_B = std::max(v->max_B, s->B);
   }
   return ensure_lists(e, size_t(std::max(v->total_members, v->total_children)));
 }
@@ -1761,7 +1762,7 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
   if (!v.generational) {
     CUDA_TRY(cudaStreamWaitEvent(e->draws, e->fork, 0));
     { Timed t(e, KN_STREAM, e->draws); gb::k_stream<<<v.n, 256, 0, e->draws>>>(v.d_desc, v.n); }
-    if (v.total_children >= gb::kClusterMinChildren) {
+    if (v.max_B >= gb::kClusterMinChildren) {
       // the placement levels follow from the draws alone: found here, beside
       // the variation, so the placement itself only compares and writes keys
       Timed t(e, KN_LEVELS, e->draws);
@@ -1859,12 +1860,6 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
     { Timed t(e, KN_STREAM); gb::k_gen_finish<<<v.n, 256, 0, e->stream>>>(v.d_desc, v.n); }
     return cudaPeekAtLastError() == cudaSuccess ? GAGP_OK : fail(GAGP_DEVICE_ERROR, cudaGetErrorString(cudaGetLastError()));
   }
-  // rounds of kClusterMinChildren or more children get their results from
-  // the cluster placement itself
-  if (v.min_B < gb::kClusterMinChildren) {
-    Timed t(e, KN_CHILD);
-    gb::k_child_results<<<blocks_for(v.total_children, 128), 128, 0, e->stream>>>(v.d_desc, v.d_child_off, v.n);
-  }
   {
     Timed t(e, KN_PLACE);
     // member keys plus as many 16-bit staged draws as fit (B * replacement + slack)
@@ -1875,11 +1870,15 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
     bytes = std::min(bytes, limit);
     CUDA_TRY(cudaStreamWaitEvent(e->stream, e->join, 0));
     CUDA_TRY(cudaStreamWaitEvent(e->stream, e->drawn, 0));
-    // the cluster placement first; the single-block kernel replays what it could not place
-    const int local_P = (v.max_P + gb::kPlaceCtas - 1) / gb::kPlaceCtas;
-    const size_t cluster_bytes = size_t(local_P + 2) * (sizeof(uint64_t) + sizeof(int32_t)) + 16;
-    gb::k_place_cluster<<<v.n * gb::kPlaceCtas, gb::kClusterThreads, cluster_bytes, e->stream>>>(v.d_desc, v.n);
-    gb::k_place<<<v.n, gb::kPlaceThreads, bytes, e->stream>>>(v.d_desc, v.n, int(bytes), 1);
+    // the cluster placement first, where a round is large enough for it; the
+    // single-block kernel places the others and replays what it could not place
+    const bool cluster = v.max_B >= gb::kClusterMinChildren;
+    if (cluster) {
+      const int local_P = (v.max_P + gb::kPlaceCtas - 1) / gb::kPlaceCtas;
+      const size_t cluster_bytes = size_t(local_P + 2) * (sizeof(uint64_t) + sizeof(int32_t)) + 16;
+      gb::k_place_cluster<<<v.n * gb::kPlaceCtas, gb::kClusterThreads, cluster_bytes, e->stream>>>(v.d_desc, v.n);
+    }
+    gb::k_place<<<v.n, gb::kPlaceThreads, bytes, e->stream>>>(v.d_desc, v.n, int(bytes), cluster);
   }
   { Timed t(e, KN_COMMIT); gb::k_commit<<<blocks_for(size_t(v.total_members) * gb::kCommitLanes, 256), 256, 0, e->stream>>>(v.d_desc, v.d_member_off, v.n); }
   return cudaPeekAtLastError() == cudaSuccess ? GAGP_OK : fail(GAGP_DEVICE_ERROR, cudaGetErrorString(cudaGetLastError()));

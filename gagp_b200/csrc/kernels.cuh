@@ -5,8 +5,8 @@
 // offsets array (items of search i are [off[i], off[i+1])).  A single search
 // is a batch of one.  Per round (run_phase_population_steady,
 // cpp/src/evolution/evolve.cpp:388-427):
-//   k_record (epoch start) -> k_vary -> k_lower -> k_vm_fast (exact-VM programs included)
-//   -> k_child_results -> k_place -> k_commit
+//   k_record (epoch start) -> k_vary -> k_lower -> k_vm_fast / k_vm_exact / k_vm_region
+//   -> k_place (k_place_cluster for large rounds) -> k_commit
 #pragma once
 #include <cooperative_groups.h>
 
@@ -836,19 +836,17 @@ __device__ inline void child_result(const SearchDesc& s, int b) {
     // the generational evaluate copies a reused member's case counts too
     // (HostPhasePopulation::evaluate, phase_population_cpu.cpp:252-253), so
     // its program-case total covers every member
-    if (s.generational) atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[2]), (unsigned long long)s.C);
+    atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[2]), (unsigned long long)s.C);
   }
 }
 
-// Results of all children before any placement, thread per child, for
-// rounds that the single-block placement takes.
+// Results of all children of a generational round, thread per child.
 __global__ void k_child_results(const SearchDesc* descs, const int32_t* off, int n) {
   const int item = blockIdx.x * blockDim.x + threadIdx.x;
   if (item >= off[n]) return;
   const int si = find_search(off, n, item);
   const SearchDesc& s = descs[si];
   if (!search_live(s)) return;
-  if (s.B >= kClusterMinChildren && !s.generational) return;  // the cluster placement forms these
   const int b = item - off[si];
   child_result(s, b);
 }
@@ -932,22 +930,29 @@ constexpr int kPlaceThreads = 1024;
 __device__ __forceinline__ bool key_before(uint64_t ka, int va, uint64_t kb, int vb) {
   return ka < kb || (ka == kb && va < vb);
 }
-// after_cluster: the cluster placement ran first; return if it placed the
-// round (place_state 1), replay it on the exact windowed path if it found a
-// redraw (2), or place it here if it did not take it (0).
-__global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* descs, int n, int dyn_bytes,
-                                                            int after_cluster) {
-  extern __shared__ __align__(16) uint64_t keys[];
-  __shared__ uint64_t mt[312], nw[312];
-  __shared__ uint64_t ck_stage[1024];
-  __shared__ uint64_t scan_key[32];
-  __shared__ int scan_idx[32];
-  __shared__ long long shared_pos, shared_wp;
-  __shared__ int shared_best, shared_fail, ready_count[2], redraw_at;
-  const SearchDesc& s = descs[blockIdx.x];
-  if (!search_live(s)) return;
-  const int cluster_state = after_cluster ? *s.place_state : 0;
-  if (cluster_state == 1) return;
+// Per: children per thread of the level-parallel path, the fewest that hold
+// the search's round (1 up to 1024 children, 4 up to 4096, 16 beyond).  What
+// bounds it is latency: two barriers a level, and the children's keys.  With
+// 16 children per thread whatever the round, 64 of the 1024 threads placed a
+// round of 1024 children and loaded each level's keys from global memory:
+// 64 us, and 9 us more for a kernel that formed their results.  With up to 4,
+// rounds below kClusterMinChildren form their children's results here and the
+// keys stay in registers: 21 us.
+struct PlaceShared {
+  uint64_t mt[312], nw[312];
+  uint64_t ck_stage[1024];
+  uint64_t scan_key[32];
+  int scan_idx[32];
+  long long pos, wp;
+  int best, fail, ready_count[2], redraw_at;
+};
+template <int Per>
+__device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, uint64_t* keys, int dyn_bytes,
+                                         int cluster_state) {
+  uint64_t (&mt)[312] = sh.mt, (&nw)[312] = sh.nw, (&ck_stage)[1024] = sh.ck_stage, (&scan_key)[32] = sh.scan_key;
+  int (&scan_idx)[32] = sh.scan_idx, (&ready_count)[2] = sh.ready_count;
+  long long &shared_pos = sh.pos, &shared_wp = sh.wp;
+  int &shared_best = sh.best, &shared_fail = sh.fail, &redraw_at = sh.redraw_at;
   const long long t0 = clock64();
   const int P = s.P, B = s.B, rs = s.replacement_size, cap = s.stream_capacity;
   const int tid = threadIdx.x;
@@ -958,6 +963,28 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* de
   }
   for (int i = tid; i < 312; i += blockDim.x) mt[i] = s.mt[i];
   __syncthreads();
+  // the children's results and keys: formed here for a round the cluster
+  // kernel leaves out
+  constexpr int kPerThread = Per;
+  constexpr bool kKeep = Per <= 4;  // the children's keys stay in registers
+  uint64_t kept[kKeep ? Per : 1];
+  if constexpr (kKeep) {
+    int reused_here = 0;
+#pragma unroll
+    for (int t = 0; t < Per; ++t) {
+      const int b = tid * Per + t;
+      kept[t] = ~0ULL;
+      if (b < B) {
+        bool reused = false;
+        kept[t] = B < kClusterMinChildren ? child_result_of(s, b, &reused) : s.c_key[b];
+        reused_here += reused;
+      }
+    }
+    for (int o = 16; o; o >>= 1) reused_here += __shfl_xor_sync(kFull, reused_here, o);
+    if ((tid & 31) == 0 && reused_here)
+      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[1]), (unsigned long long)reused_here);
+    __syncthreads();  // the windowed path reads every child's key
+  }
   const long long rp = stream_ptrs(s)[0];
   long long wp = stream_ptrs(s)[1];
   const long long need = (long long)B * rs + 1;
@@ -967,7 +994,6 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* de
   }
   const long long t1 = clock64();
   // ---------------------------------------------------- level-parallel path
-  constexpr int kPerThread = 16;
   // owner area after the keys, 16-byte aligned, with 64 bytes of slack for
   // the per-thread 16-byte reads of the staged draws
   int32_t* owner = reinterpret_cast<int32_t*>(keys + P + (P & 1));
@@ -981,8 +1007,12 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* de
     // begin + t's two draws, and once it is placed, its victim
     const int base = int(rp % cap);
     const int begin = tid * kPerThread;
-    constexpr int kBatch = 4;  // child keys loaded together
+    constexpr int kBatch = kPerThread < 4 ? kPerThread : 4;  // child keys loaded together
     const uint64_t* __restrict__ ckey = s.c_key;
+    auto key_of = [&](int t) -> uint64_t {
+      if constexpr (kKeep) return kept[t];
+      else return ckey[begin + t];
+    };
     // the 2B draws (residues < P <= 65536), staged as 16-bit values in the
     // owner area with coalesced loads, then read back per thread: child j's
     // pair is the 32-bit word j
@@ -999,15 +1029,20 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* de
     uint32_t cand[kPerThread];
     uint32_t pending = 0;
     {
-      static_assert(kPerThread % 4 == 0, "draw pairs are read four at a time");
-      const uint4* pairs = reinterpret_cast<const uint4*>(owner) + size_t(begin) / 4;
+      if constexpr (kPerThread % 4 == 0) {
+        const uint4* pairs = reinterpret_cast<const uint4*>(owner) + size_t(begin) / 4;
 #pragma unroll
-      for (int q = 0; q < kPerThread / 4; ++q) {
-        const uint4 v = begin < B ? pairs[q] : make_uint4(0, 0, 0, 0);
-        cand[4 * q] = v.x;
-        cand[4 * q + 1] = v.y;
-        cand[4 * q + 2] = v.z;
-        cand[4 * q + 3] = v.w;
+        for (int q = 0; q < kPerThread / 4; ++q) {
+          const uint4 v = begin < B ? pairs[q] : make_uint4(0, 0, 0, 0);
+          cand[4 * q] = v.x;
+          cand[4 * q + 1] = v.y;
+          cand[4 * q + 2] = v.z;
+          cand[4 * q + 3] = v.w;
+        }
+      } else {
+#pragma unroll
+        for (int t = 0; t < kPerThread; ++t)
+          cand[t] = begin + t < B ? reinterpret_cast<const uint32_t*>(owner)[begin + t] : 0;
       }
 #pragma unroll
       for (int t = 0; t < kPerThread; ++t) {
@@ -1050,7 +1085,7 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* de
         for (int h = 0; h < kPerThread; h += kBatch) {
           uint64_t kv[kBatch];
 #pragma unroll
-          for (int u = 0; u < kBatch; ++u) kv[u] = (ready >> (h + u) & 1) ? ckey[begin + h + u] : 0;
+          for (int u = 0; u < kBatch; ++u) kv[u] = (ready >> (h + u) & 1) ? key_of(h + u) : 0;
 #pragma unroll
           for (int u = 0; u < kBatch; ++u)
             if (ready >> (h + u) & 1) {
@@ -1089,7 +1124,7 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* de
     for (int h = 0; h < kPerThread; h += kBatch) {
       uint64_t kv[kBatch];
 #pragma unroll
-      for (int u = 0; u < kBatch; ++u) kv[u] = begin + h + u < B ? ckey[begin + h + u] : ~0ULL;
+      for (int u = 0; u < kBatch; ++u) kv[u] = begin + h + u < B ? key_of(h + u) : ~0ULL;
 #pragma unroll
       for (int u = 0; u < kBatch; ++u)
         if (begin + h + u < B && key_before(kv[u], int(cand[h + u]), mk, mv)) {
@@ -1136,7 +1171,7 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* de
     for (int h = 0; h < kPerThread; h += kBatch) {
       uint64_t kv[kBatch];
 #pragma unroll
-      for (int u = 0; u < kBatch; ++u) kv[u] = begin + h + u < B ? ckey[begin + h + u] : 0;
+      for (int u = 0; u < kBatch; ++u) kv[u] = begin + h + u < B ? key_of(h + u) : 0;
 #pragma unroll
       for (int u = 0; u < kBatch; ++u)
         if (!hit && begin + h + u < B) {
@@ -1337,6 +1372,22 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* de
   }
 }
 
+// after_cluster: the cluster placement ran first; return if it placed the
+// round (place_state 1), replay it on the exact windowed path if it found a
+// redraw (2), or place it here if it did not take it (0).
+__global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* descs, int n, int dyn_bytes,
+                                                            int after_cluster) {
+  extern __shared__ __align__(16) uint64_t place_keys[];
+  __shared__ PlaceShared sh;
+  const SearchDesc& s = descs[blockIdx.x];
+  if (!search_live(s)) return;
+  const int cluster_state = after_cluster ? *s.place_state : 0;
+  if (cluster_state == 1) return;
+  if (s.B <= kPlaceThreads) place_round<1>(s, sh, place_keys, dyn_bytes, cluster_state);
+  else if (s.B <= 4 * kPlaceThreads) place_round<4>(s, sh, place_keys, dyn_bytes, cluster_state);
+  else place_round<16>(s, sh, place_keys, dyn_bytes, cluster_state);
+}
+
 // Cluster placement: the level-parallel placement above, spread over a
 // cluster of kPlaceCtas blocks that share their shared memory.  Member m
 // lives in block m % kPlaceCtas (its key and level owner); thread g of the
@@ -1471,9 +1522,8 @@ __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThr
   const int P = s.P, B = s.B, cap = s.stream_capacity;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long rp = stream_ptrs(s)[0], wp = stream_ptrs(s)[1];
-  // the children's results and keys (k_child_results leaves rounds of this
-  // size to this kernel), formed before any decision so that the single-block
-  // placement finds them too
+  // the children's results and keys, formed before any decision so that the
+  // single-block placement finds them too
   const int begin = (rank * kClusterThreads + tid) * kClusterPer;
   uint64_t kv[kClusterPer];  // the children's keys
   if (B >= kClusterMinChildren) {
