@@ -210,250 +210,256 @@ struct GenResult {
 struct GenTables {
   const GenExpr* gx;
   const GenNt* gnt;
-  const uint32_t* head;
   const GenLevel* level;
   const GenEntry* entry;
-  const gagp_domain* doms;
+  const GenDomain* doms;
   const gagp_value* vals;
-  const uint16_t* minimum;
-  const int4* extra;  // children 4..7 and their scopes, two int4 per expression (arity above 4 only)
+  const uint32_t* cell;
+  const uint16_t* row_of;
+  const int4* extra;  // children 4..7 and their rows, two int4 per expression (arity above 4 only)
 };
 __device__ __forceinline__ GenTables gen_tables(const SearchDesc& s, const char* image) {
   return GenTables{reinterpret_cast<const GenExpr*>(image), reinterpret_cast<const GenNt*>(image + s.gi.nt),
-                   reinterpret_cast<const uint32_t*>(image + s.gi.head),
                    reinterpret_cast<const GenLevel*>(image + s.gi.level),
                    reinterpret_cast<const GenEntry*>(image + s.gi.entry),
-                   reinterpret_cast<const gagp_domain*>(image + s.gi.doms),
+                   reinterpret_cast<const GenDomain*>(image + s.gi.doms),
                    reinterpret_cast<const gagp_value*>(image + s.gi.vals),
-                   reinterpret_cast<const uint16_t*>(image + s.gi.minimum),
+                   reinterpret_cast<const uint32_t*>(image + s.gi.cell),
+                   reinterpret_cast<const uint16_t*>(image + s.gi.row_of),
                    reinterpret_cast<const int4*>(image + s.gi.extra)};
 }
 
-// A precomputed draw level (GenLevel) in registers.
-struct LevelView {
-  double total;
-  unsigned bound, entry;
-  int last, below;
+// The draws of one generator stream in order.  Warp: every lane takes the
+// same draws, mixed 32 at a time (the stream is a counter mixed per draw); a
+// draw is then one shuffle, started when the one before it is taken.
+template <bool Warp>
+struct DrawStream {
+  Rng random;
+  uint64_t ahead, batch = 0;
+  int at = 0;
+  __device__ __forceinline__ explicit DrawStream(uint64_t seed) : random(seed) { refill(); }
+  __device__ __forceinline__ void refill() {
+    if (Warp) {
+      Rng mine(random.state + (threadIdx.x & 31) * 0x9e3779b97f4a7c15ULL);
+      batch = mine.next();
+      random.state += 32 * 0x9e3779b97f4a7c15ULL;
+      at = 0;
+      ahead = __shfl_sync(kFull, batch, 0);
+    } else {
+      ahead = random.next();
+    }
+  }
+  __device__ __forceinline__ uint64_t next() {
+    const uint64_t v = ahead;
+    if (Warp && ++at < 32) ahead = __shfl_sync(kFull, batch, at);
+    else refill();
+    return v;
+  }
 };
-__device__ __forceinline__ LevelView load_level(const GenLevel* p) {
-  const int4 a = *reinterpret_cast<const int4*>(p);
-  const int2 b = *(reinterpret_cast<const int2*>(p) + 2);
-  return LevelView{__hiloint2double(a.y, a.x), unsigned(a.z), unsigned(a.w), b.x, b.y};
-}
 
 // generate_phase<CompactTasks=true, EmitSites=true, Warp=false>
 // (cpp/src/evolution/repro/gpu/device/phase_generate.cuh:125-270): a typed
 // random subtree with min-cost feasibility and the FP64 weighted production
-// draw.  The draw uses round-to-nearest intrinsics so nothing is contracted
-// into an FMA; the reference's host build rounds every operation alike.
-// Tasks pack (expression:17, depth:7, scope_count:4, logical:4) in `pending`
-// (192 entries).  Emitted words carry depth relative to the generated root
-// (root = 1) and site depth relative to the budget `logical_depth`.
+// draw.  The sequential draw uses round-to-nearest intrinsics so nothing is
+// contracted into an FMA; the reference's host build rounds every operation
+// alike.  Tasks pack (expression:17, depth:7, scope_count:4, logical:4) in
+// `pending` (192 entries).  Emitted words carry depth relative to the generated
+// root (root = 1) and site depth relative to the budget `logical_depth`.
+//
+// Warp: the warp generates one subtree, every lane with the same state (the
+// lanes store the same words to the same addresses), and the lanes compare a
+// draw with a production each; otherwise each thread generates its own.
+//
+// What bounds it: the chain of one subtree's steps, which sets the variation
+// kernel's slowest child (an instruction every 5 cycles, most of them waiting
+// for the one before).  A task carries what its cell holds (minimum cost, a
+// reference's draw level), so a nonterminal and the production drawn for it
+// are one step of four lookups: the level, the limits (a lane each, the choice
+// value's FP64 multiplications and thresholds folded into 53-bit limits), the
+// production and its children's cells.  Draws are mixed ahead and a constant's
+// residue takes no division.  On the staged tables of the large scalar
+// grammar, a warp alone takes 393 cycles per task (514 with every SM full); a
+// lookup chain per task with the same draws took 637 (840).  The slowest
+// child of a resumed search of P = 777 generated for 112k cycles with the
+// draws in FP64 on one lane, 61k now.
+template <bool Warp>
 __device__ inline GenResult generate(const SearchDesc& s, const char* image, int root_expression, int scope_count,
                                      int depth, int capacity, uint64_t seed, uint64_t* out_node, int64_t* out_cval,
                                      int logical_depth, uint64_t* pending) {
   GenResult result{ST_INVALID, 0, 0, 0};
   const GenTables tables = gen_tables(s, image);
-  // the tables (staged in shared memory by the variation kernel), read once
-  // into registers; the sequential draw's production tables stay global
   const GenExpr* __restrict__ gx = tables.gx;
-  const GenNt* __restrict__ gnt = tables.gnt;
-  const uint32_t* __restrict__ head = tables.head;
   const GenLevel* __restrict__ gen_level = tables.level;
   const GenEntry* __restrict__ gen_entry = tables.entry;
-  const gagp_domain* __restrict__ doms = tables.doms;
-  const gagp_value* __restrict__ vals = tables.vals;
-  const uint16_t* __restrict__ minimum = tables.minimum;
-  const gagp_production* __restrict__ prods = s.prods;
-  const uint32_t* __restrict__ prod_minimum = s.prod_minimum;
-  const int n_ex = s.n_ex, n_nts = s.n_nts, n_prods = s.n_prods;
-  const int depth_count = s.depth_count, logical_count = s.logical_count;
-  const bool site_limited = s.site_depth > 0;
-  // minimum cost of (expression, depth, site budget); admission has checked
-  // every expression id a table holds, and the generator keeps depth and site
-  // budget inside the table, so only the root's lookup is range-checked
-  auto min_at = [&](int e, int d, int l) -> unsigned {
-    const unsigned v = minimum[(e * depth_count + d) * logical_count + l];
-    return v == kNoMinimum16 ? kNoId : v;
-  };
-  int next_site = -1;  // entry expression of a pending site
-  uint32_t next_class = kNoClass;
+  const uint32_t* __restrict__ cell_words = tables.cell;
+  const int n_ex = s.n_ex;
+  const int depth_count = s.depth_count, logical_count = s.logical_count, cells = depth_count * logical_count;
+  const int site_step = s.site_depth > 0 ? 1 : 0;
   if (root_expression < 0 || root_expression >= n_ex || scope_count < 0 || scope_count > 15 || depth <= 0 ||
       depth >= depth_count || depth > 64 || logical_depth < 0 || logical_depth >= logical_count ||
       capacity <= 0 || capacity > kCapacity || n_ex > 131071)
     return result;
   if (capacity > s.stride) capacity = s.stride;  // callers pass at most the node budget
-  // a task: expression, depth, scope, site budget and its minimum cost (the
-  // reservation made when it was pushed).  The task to run next is kept in a
-  // register (`next`, when have_next) rather than pushed and popped at once;
-  // `count` is what the reference's stack holds below it.
-  auto pack = [](unsigned e, unsigned d, unsigned n, unsigned l, unsigned required) -> uint64_t {
-    return uint64_t(e | (d << 17) | (n << 24) | (l << 28)) | (uint64_t(required) << 32);
-  };
-  unsigned reserved = min_at(root_expression, depth, logical_depth);
-  uint64_t next = pack(unsigned(root_expression), unsigned(depth), unsigned(scope_count), unsigned(logical_depth),
-                       reserved);
-  bool have_next = true;
+  // A task: its cell word (its minimum cost, reserved when it was pushed, and
+  // its level), and its expression with its depth (root 1) << 16 and the site
+  // budget used << 24, as its node word holds them.  Scopes are not kept:
+  // references are unscoped and nothing else asks.  The task to run next is
+  // kept in registers rather than pushed and popped at once; `count` is what
+  // the reference's stack holds below it.  What cannot happen with the tables
+  // admission checks (a task that was not reserved, a full stack at a
+  // nonterminal) is not tested, and a step's tests are one branch: every step
+  // emits a node or ends, so the loop is bounded by the capacity.
+  uint2* const stack = reinterpret_cast<uint2*>(pending);
+  uint2* const words_out = reinterpret_cast<uint2*>(out_node);
+  const int origin = (depth + 1) * logical_count + logical_depth;  // a node's cell is `origin` less its depth's and budget's
+  uint2 task = make_uint2(cell_words[int(tables.row_of[root_expression]) * cells + depth * logical_count + logical_depth],
+                          unsigned(root_expression) | 1u << 16);
   int count = 0;
-  if (reserved > unsigned(capacity)) { result.status = ST_CAPACITY; return result; }
-  Rng random(seed);
-  while (have_next || count) {
-    if (++result.steps > 8192) { result.status = ST_CAPACITY; return result; }
-    const uint64_t task = have_next ? next : pending[--count];
-    have_next = false;
-    const int t_expr = int(task & 0x1ffffu), t_depth = int((task >> 17) & 0x7fu);
-    const int t_scope = int((task >> 24) & 0xfu), t_logical = int((task >> 28) & 0xfu);
-    const unsigned required = unsigned(task >> 32);
-    if (required > reserved) return result;
-    reserved -= required;
-    const int4 ra = *reinterpret_cast<const int4*>(gx + t_expr);      // children
-    const int4 rb = *(reinterpret_cast<const int4*>(gx + t_expr) + 1);  // target, class, kinds, scopes
-    const int kind = int(int8_t(rb.z & 0xff)), arity = int(int8_t((rb.z >> 8) & 0xff));
-    const int target = rb.x;
-    if (kind == EK_REFERENCE) {
-      // admission: the target nonterminal exists, is unscoped (as is every
-      // reference) and its productions are in range
-      if (next_site >= 0) return result;
-      next_site = t_expr;
-      next_class = uint32_t(rb.y);
-      const int4 nt = *reinterpret_cast<const int4*>(gnt + target);
-      const int nt_offset = nt.x, nt_count = nt.y;
-      const bool normalized = nt.w != 0;
-      if (site_limited && t_logical == 0) { result.status = ST_CAPACITY; return result; }
-      const int n_logical = t_logical - (site_limited ? 1 : 0);
-      if (reserved > unsigned(capacity - result.nodes)) { result.status = ST_CAPACITY; return result; }
-      const unsigned available = unsigned(capacity - result.nodes) - reserved;
-      unsigned next_expr, need;
-      // the widest precomputed level whose productions all fit
-      LevelView lv = load_level(gen_level + head[(t_depth * logical_count + n_logical) * n_nts + target]);
-      while (lv.bound > available && lv.below >= 0) lv = load_level(gen_level + lv.below);
-      if (lv.bound <= available && lv.total == lv.total) {
-        const double choice = __dmul_rn(__dmul_rn(double(random.next() >> 11), 0x1.0p-53), lv.total);
-        const GenEntry* __restrict__ en = gen_entry + lv.entry;
-        int pick = lv.last;
-        if (nt_count <= 8) {
-          double th[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) th[k] = k < nt_count ? en[k].threshold : 0.0;
-#pragma unroll
-          for (int k = 7; k >= 0; --k)
-            if (k < nt_count && choice < th[k]) pick = k;
+  unsigned reserved = task.x & 0xffffu, room = unsigned(capacity);
+  if (reserved > room) { result.status = ST_CAPACITY; return result; }
+  DrawStream<Warp> random(seed);
+  for (;;) {
+    unsigned e = task.y & 0xffffu, place = task.y >> 16;
+    unsigned site = 0, site_class = kNoClass << 21;
+    const unsigned level = task.x >> 16;
+    reserved -= task.x & 0xffffu;
+    ++result.steps;
+    if (level != kNoReference) {
+      // a nonterminal and the production drawn for it, which runs at once.
+      // Admission: the target nonterminal exists, is unscoped (as is every
+      // reference) and its productions are in range.
+      site = (e + 1) << 16;
+      site_class = gx[e].shape << 21;
+      place += unsigned(site_step) << 8;
+      const unsigned available = room - reserved;
+      // the widest precomputed level whose productions all fit: bound, first
+      // entry, count, next narrower level
+      int4 lv = *reinterpret_cast<const int4*>(gen_level + level);
+      bool drawn = true;
+      if (unsigned(lv.x) > available) {
+        while (unsigned(lv.x) > available && lv.w >= 0) lv = *reinterpret_cast<const int4*>(gen_level + lv.w);
+        drawn = unsigned(lv.x) <= available;
+      }
+      if (drawn) {
+        const uint64_t bits = random.next() >> 11;
+        const GenEntry* __restrict__ en = gen_entry + unsigned(lv.y);
+        int pick = 0;
+        if (Warp) {
+          // lanes past the productions repeat the last one's limit
+          const int last = lv.z - 1;
+          int k = min(int(threadIdx.x & 31), last);
+          unsigned hits = __ballot_sync(kFull, bits < en[k].limit);
+          while (!hits) {  // the last feasible production's limit is past every draw
+            pick += 32;
+            k = min(pick + int(threadIdx.x & 31), last);
+            hits = __ballot_sync(kFull, bits < en[k].limit || pick > last);
+          }
+          pick = min(pick + __ffs(hits) - 1, last);
         } else {
-          for (int i = 0; i < nt_count; ++i)
-            if (choice < en[i].threshold) { pick = i; break; }
+          while (pick < lv.z - 1 && bits >= en[pick].limit) ++pick;
         }
-        const int2 picked = *(reinterpret_cast<const int2*>(en + pick) + 1);  // expression, need
-        next_expr = unsigned(picked.x);
-        need = unsigned(picked.y);
+        e = unsigned(en[pick].expression);
       } else {
         // the reference's draw step by step (no precomputed level applies)
-        const uint32_t* __restrict__ prow = prod_minimum + (t_depth * logical_count + n_logical) * n_prods + nt_offset;
+        const int budget = logical_depth - int(place >> 8), t_depth = depth + 1 - int(place & 0xffu);
+        if (room == 0 || t_depth < 1 || budget < 0) { result.status = ST_CAPACITY; return result; }
+        const int4 nt = *reinterpret_cast<const int4*>(tables.gnt + gx[e].target);
+        const int nt_offset = nt.x;
+        const bool normalized = nt.w != 0;
+        const gagp_production* __restrict__ prods = s.prods;
+        const uint32_t* __restrict__ prow = s.prod_minimum + (t_depth * logical_count + budget) * s.n_prods + nt_offset;
         uint64_t feasible_mask = 0;  // a bit per production for the first 64
-        for (int i = 0; i < nt_count && i < 64; ++i)
+        for (int i = 0; i < nt.y && i < 64; ++i)
           if (__ldg(&prow[i]) <= available) feasible_mask |= 1ULL << i;
         auto feasible = [&](int i) -> bool {
           return i < 64 ? (feasible_mask >> i & 1) : __ldg(&prow[i]) <= available;
         };
         double maximum = normalized ? 1.0 : 0.0, total = 0.0;
         if (!normalized)
-          for (int i = 0; i < nt_count; ++i) {
+          for (int i = 0; i < nt.y; ++i) {
             const double w = __ldg(&prods[nt_offset + i].weight);
             if (feasible(i) && w > maximum) maximum = w;
           }
         if (!(maximum > 0)) { result.status = ST_CAPACITY; return result; }
-        for (int i = 0; i < nt_count; ++i)
+        for (int i = 0; i < nt.y; ++i)
           if (feasible(i)) {
             const double w = __ldg(&prods[nt_offset + i].weight);
             total = __dadd_rn(total, normalized ? w : __ddiv_rn(w, maximum));
           }
         double choice = __dmul_rn(__dmul_rn(double(random.next() >> 11), 0x1.0p-53), total);
-        next_expr = 131071u;  // unselected
-        for (int i = 0; i < nt_count; ++i) {
+        int production = -1;
+        for (int i = 0; i < nt.y; ++i) {
           if (!feasible(i)) continue;
-          next_expr = unsigned(__ldg(&prods[nt_offset + i].expression));
+          production = __ldg(&prods[nt_offset + i].expression);
           const double w = __ldg(&prods[nt_offset + i].weight);
           choice = __dsub_rn(choice, normalized ? w : __ddiv_rn(w, maximum));
           if (choice < 0) break;
         }
-        if (next_expr == 131071u) return result;
-        need = min_at(int(next_expr), t_depth, n_logical);
+        if (production < 0) return result;
+        e = unsigned(production);
       }
-      if (count >= 192) return result;
-      reserved += need;
-      next = pack(next_expr, unsigned(t_depth), 0u, unsigned(n_logical), need);
-      have_next = true;
+      ++result.steps;
+    }
+    const int4 ra = *reinterpret_cast<const int4*>(gx + e);  // children, target, shape
+    const unsigned shape = unsigned(ra.w), kind = shape >> 24, arity = shape >> 16 & 0xfu;
+    const bool over = room == 0 || (place & 0xffu) > unsigned(depth) || place >> 8 > unsigned(logical_depth);
+    if (over || kind == EK_REFERENCE || kind == EK_ALIAS) {
+      // no room; a production that is a reference (a site within a site); an
+      // alias (declined at admission)
+      result.status = over && kind != EK_REFERENCE ? ST_CAPACITY : ST_INVALID;
+      return result;
+    }
+    words_out[result.nodes++] = make_uint2(e | site, place | (shape & kShapeNode) | site_class);
+    --room;
+    if (arity == 0) {
+      if (kind == EK_CONSTANT) {
+        // admission: the domain exists and is an Int range or a list of Ints
+        const GenDomain* dom = tables.doms + ra.z;
+        uint64_t v = random.next();
+        const uint64_t width = dom->width;
+        if (width) {
+          const uint64_t reject = dom->reject;
+          while (v < reject) v = random.next();
+          v -= __umul64hi(v, dom->magic) * width;  // at most two below the quotient
+          v = v >= width ? v - width : v;
+          v = v >= width ? v - width : v;
+        }
+        const int offset = dom->offset;
+        out_cval[result.constants++] = offset < 0 ? int64_t(uint64_t(dom->minimum) + v) : tables.vals[offset + int(v)].i;
+      }
+      if (!count) break;
+      task = stack[--count];
       continue;
     }
-    if (t_depth <= 0 || result.nodes >= capacity) { result.status = ST_CAPACITY; return result; }
-    if (kind == EK_CONSTANT) {
-      // admission: the domain exists and is an Int range or a list of Ints
-      const gagp_domain* domain = doms + target;
-      int64_t value;
-      if (domain->integer_range) {
-        value = random.integer(domain->minimum, domain->maximum);
-      } else {
-        const int v_offset = domain->value_offset, v_count = domain->value_count;
-        value = vals[v_offset + random.bounded(uint64_t(v_count))].i;
-      }
-      out_cval[result.constants++] = value;
-    } else if (kind != EK_OPERATION && kind != EK_INPUT && kind != EK_BOUND) {
-      return result;  // aliases are declined at admission
+    // an operation: the children's minimum costs are reserved and the children
+    // pushed last to first (the first straight into `task`); a step that
+    // cannot reserve them all, or push past the stack, ends the generation
+    const int4 rows = *(reinterpret_cast<const int4*>(gx + e) + 1);
+    ++place;
+    const uint32_t* __restrict__ words = cell_words + (origin - int(place & 0xffu) * logical_count - int(place >> 8));
+    if (count + int(arity) - 1 >= 192 || (place & 0xffu) > unsigned(depth) + 1) {
+      result.status = ST_CAPACITY;
+      return result;
     }
-    out_node[result.nodes++] = w_make(t_expr, next_site, depth - t_depth + 1, logical_depth - t_logical, arity,
-                                      kind == EK_CONSTANT, next_class);
-    next_site = -1;
-    next_class = kNoClass;
-    // the children's minimum costs, loaded together, then pushed last to
-    // first (the first child straight into `next`); a traversal has four
+    // kNoMinimum16 is past any room
+    const uint32_t w0 = words[rows.x], w1 = arity > 1 ? words[rows.y] : 0u, w2 = arity > 2 ? words[rows.z] : 0u,
+                   w3 = arity > 3 ? words[rows.w] : 0u;
+    reserved += (w0 & 0xffffu) + (w1 & 0xffffu) + (w2 & 0xffffu) + (w3 & 0xffffu);
+    const unsigned where = place << 16;
     if (arity > 4) {
-      // a bounded region: children 4..7 from the image's extra section,
-      // pushed last to first as below
-      const int4 xa = tables.extra[2 * t_expr], xb = tables.extra[2 * t_expr + 1];
-      for (int i = arity - 1; i >= 0; --i) {
-        if (count >= 192) { result.status = ST_CAPACITY; return result; }
-        const int child = i == 0 ? ra.x : i == 1 ? ra.y : i == 2 ? ra.z : i == 3 ? ra.w : i == 4 ? xa.x
-                          : i == 5 ? xa.y : i == 6 ? xa.z : xa.w;
-        const unsigned need = min_at(child, t_depth - 1, t_logical);
-        if (need > unsigned(capacity - result.nodes) || reserved > unsigned(capacity - result.nodes) - need) {
-          result.status = ST_CAPACITY;
-          return result;
-        }
-        const int child_scope = i < 4 ? int(int8_t((rb.w >> (8 * i)) & 0xff)) : int(int8_t((xb.x >> (8 * (i - 4))) & 0xff));
-        const int scope = child_scope >= 0 ? child_scope : t_scope;
-        const uint64_t t = pack(unsigned(child), unsigned(t_depth - 1), unsigned(scope), unsigned(t_logical), need);
-        if (i == 0) {
-          next = t;
-          have_next = true;
-        } else {
-          pending[count++] = t;
-        }
-        reserved += need;
+      // a bounded region: children 4..7 from the image's extra section
+      const int4 xa = tables.extra[2 * e], xb = tables.extra[2 * e + 1];
+      for (int i = int(arity) - 1; i >= 4; --i) {
+        const uint32_t word = words[i == 4 ? xb.x : i == 5 ? xb.y : i == 6 ? xb.z : xb.w];
+        reserved += word & 0xffffu;
+        stack[count++] = make_uint2(word, unsigned(i == 4 ? xa.x : i == 5 ? xa.y : i == 6 ? xa.z : xa.w) | where);
       }
-      continue;
     }
-    const unsigned need0 = arity > 0 ? min_at(ra.x, t_depth - 1, t_logical) : 0;
-    const unsigned need1 = arity > 1 ? min_at(ra.y, t_depth - 1, t_logical) : 0;
-    const unsigned need2 = arity > 2 ? min_at(ra.z, t_depth - 1, t_logical) : 0;
-    const unsigned need3 = arity > 3 ? min_at(ra.w, t_depth - 1, t_logical) : 0;
-    for (int i = arity - 1; i >= 0; --i) {
-      if (count >= 192) { result.status = ST_CAPACITY; return result; }
-      const int child = i == 0 ? ra.x : i == 1 ? ra.y : i == 2 ? ra.z : ra.w;
-      const unsigned need = i == 0 ? need0 : i == 1 ? need1 : i == 2 ? need2 : need3;
-      if (need > unsigned(capacity - result.nodes) || reserved > unsigned(capacity - result.nodes) - need) {
-        result.status = ST_CAPACITY;
-        return result;
-      }
-      const int child_scope = int(int8_t((rb.w >> (8 * i)) & 0xff));
-      const int scope = child_scope >= 0 ? child_scope : t_scope;
-      const uint64_t t = pack(unsigned(child), unsigned(t_depth - 1), unsigned(scope), unsigned(t_logical), need);
-      if (i == 0) {
-        next = t;
-        have_next = true;
-      } else {
-        pending[count++] = t;
-      }
-      reserved += need;
-    }
+    if (reserved > room) { result.status = ST_CAPACITY; return result; }
+    if (arity > 3) stack[count++] = make_uint2(w3, unsigned(ra.y) >> 16 | where);
+    if (arity > 2) stack[count++] = make_uint2(w2, (unsigned(ra.y) & 0xffffu) | where);
+    if (arity > 1) stack[count++] = make_uint2(w1, unsigned(ra.x) >> 16 | where);
+    task = make_uint2(w0, (unsigned(ra.x) & 0xffffu) | where);
   }
   if (reserved || !result.nodes) return result;
   result.status = ST_OK;

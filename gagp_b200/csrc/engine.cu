@@ -544,7 +544,10 @@ gagp_status admit(const gagp_grammar* g, const gagp_cases* c, const gagp_search_
 // below the smallest double T_i with f_i(T_i) >= 0, found by bisection over
 // the bit patterns of non-negative doubles.  The first production whose
 // threshold exceeds c is the one the sequential loop stops at (the last
-// feasible one when none does).  Levels with the same feasible set share
+// feasible one when none does).  c is monotone in the draw's 53 bits too, so
+// the tables hold, for each T_i, the smallest 53-bit draw whose c reaches it
+// (bisection with the same two multiplications), and a draw is compared with
+// integers.  Levels with the same feasible set share
 // their draw; past kMaxDrawEntries the remaining nonterminals keep the
 // sequential draw.
 constexpr size_t kMaxDrawEntries = size_t(1) << 16;
@@ -553,6 +556,9 @@ struct DrawTables {
   std::vector<uint32_t> head;  // per (depth, site budget, nonterminal): its widest level (0: none)
   std::vector<gb::GenLevel> level;
   std::vector<gb::GenEntry> entry;
+  std::vector<uint32_t> cell;    // [row][depth][site budget] (gb::GenImage::cell)
+  std::vector<uint16_t> row_of;  // each expression's row
+  int rows = 0;
 };
 
 // `with_draws` false: only the table sizes (for the memory plan).
@@ -562,14 +568,11 @@ DrawTables draw_tables(const gagp_grammar* g, bool with_draws) {
   DrawTables t;
   const size_t heads = size_t(std::max(1, NT)) * DC * LC;
   gb::GenLevel none{};
-  none.total = std::nan("");
   none.bound = gb::kNoId;
-  none.entry = 0;
-  none.last = -1;
   none.below = -1;
   t.level.assign(1, none);  // level 0: no precomputed draw
   t.head.assign(heads, 0);
-  struct Draw { double total; int last; std::vector<double> threshold; };
+  struct Draw { int last; std::vector<uint64_t> limit; };
   std::map<std::pair<int, std::vector<uint8_t>>, Draw> memo;
   auto from_bits = [](uint64_t b) { double d; std::memcpy(&d, &b, sizeof d); return d; };
   auto draw_of = [&](int nt, const std::vector<uint8_t>& feasible) -> const Draw& {
@@ -577,7 +580,7 @@ DrawTables draw_tables(const gagp_grammar* g, bool with_draws) {
     if (it != memo.end()) return it->second;
     const gagp_nonterminal& n = g->nonterminals[nt];
     const int off = n.production_offset, cnt = n.production_count;
-    Draw dr{std::nan(""), -1, std::vector<double>(cnt, 0.0)};
+    Draw dr{-1, std::vector<uint64_t>(cnt, 0)};
     double maximum = n.normalized_weights ? 1.0 : 0.0;
     for (int i = 0; i < cnt; ++i)
       if (feasible[i] && !n.normalized_weights && g->productions[off + i].weight > maximum)
@@ -605,13 +608,21 @@ DrawTables draw_tables(const gagp_grammar* g, bool with_draws) {
           const uint64_t mid = lo + (hi - lo) / 2;
           if (f(from_bits(mid), i) >= 0) hi = mid; else lo = mid;
         }
-        dr.threshold[i] = from_bits(hi);
+        // the smallest draw whose choice value reaches the threshold: the
+        // choice value u * total is monotone in the draw's 53 bits
+        const double threshold = from_bits(hi);
+        uint64_t first = 0, past = uint64_t(1) << 53;
+        while (first < past) {
+          const uint64_t mid = first + (past - first) / 2;
+          if (double(mid) * 0x1.0p-53 * total >= threshold) past = mid; else first = mid + 1;
+        }
+        dr.limit[i] = first;
       }
-      dr.total = total;
+      dr.limit[dr.last] = uint64_t(1) << 53;  // the pick when no earlier one is
     }
     return memo.emplace(std::make_pair(nt, feasible), std::move(dr)).first->second;
   };
-  std::map<std::tuple<int, uint32_t, std::vector<uint32_t>>, std::pair<uint32_t, std::pair<double, int>>> entry_memo;
+  std::map<std::tuple<int, uint32_t, std::vector<uint32_t>>, std::pair<uint32_t, int>> entry_memo;  // first entry, last pick
   std::map<std::tuple<uint32_t, uint32_t, int32_t>, int32_t> level_memo;
   for (int nt = 0; nt < NT; ++nt) {
     const gagp_nonterminal& n = g->nonterminals[nt];
@@ -650,21 +661,17 @@ DrawTables draw_tables(const gagp_grammar* g, bool with_draws) {
             const uint32_t at = uint32_t(t.entry.size());
             for (int i = 0; i < cnt; ++i) {
               gb::GenEntry en{};
-              en.threshold = dr ? dr->threshold[i] : 0.0;
+              en.limit = dr ? dr->limit[i] : 0;
               en.expression = g->productions[off + i].expression;
-              en.need = cost[i];
               t.entry.push_back(en);
             }
-            eit = entry_memo.emplace(ekey, std::make_pair(at, dr ? std::make_pair(dr->total, dr->last)
-                                                                  : std::make_pair(0.0, -1))).first;
+            eit = entry_memo.emplace(ekey, std::make_pair(at, dr ? dr->last : -1)).first;
           }
           gb::GenLevel lv = none;
-          lv.bound = bounds[k];
+          // a set without weight has no draw (nor has any narrower one)
+          lv.bound = !with_draws || eit->second.second >= 0 ? bounds[k] : gb::kNoId;
           lv.entry = eit->second.first;
-          if (with_draws) {
-            lv.total = eit->second.second.first;
-            lv.last = eit->second.second.second;
-          }
+          lv.count = uint32_t(cnt);
           lv.below = below;
           const auto lkey = std::make_tuple(lv.entry, lv.bound, lv.below);
           auto lit = level_memo.find(lkey);
@@ -678,6 +685,29 @@ DrawTables draw_tables(const gagp_grammar* g, bool with_draws) {
       }
   }
   if (t.entry.empty()) t.entry.push_back(gb::GenEntry{});
+  // the cell rows: a task's minimum cost and, for a reference, the level its
+  // draw starts from (one site budget further on under a site-depth limit)
+  std::map<std::vector<uint32_t>, int> rows;
+  t.row_of.assign(E, 0);
+  std::vector<uint32_t> row(size_t(DC) * LC);
+  for (int e = 0; e < E; ++e) {
+    const gagp_expression& x = g->expressions[e];
+    for (int d = 0; d < DC; ++d)
+      for (int l = 0; l < LC; ++l) {
+        const uint32_t cost = g->minimum[(size_t(e) * DC + d) * LC + l];
+        uint32_t level = gb::kNoReference;
+        if (x.kind == gb::EK_REFERENCE) {
+          const int budget = g->site_depth > 0 ? l - 1 : l;
+          level = budget >= 0 && x.target >= 0 && x.target < NT ? t.head[(size_t(d) * LC + budget) * NT + x.target] : 0;
+          if (level >= gb::kNoReference) level = 0;  // past 16 bits: the sequential draw
+        }
+        row[size_t(d) * LC + l] = (cost >= gb::kNoMinimum16 ? gb::kNoMinimum16 : cost) | level << 16;
+      }
+    const auto [it, fresh] = rows.emplace(row, int(rows.size()));
+    if (fresh) t.cell.insert(t.cell.end(), row.begin(), row.end());
+    t.row_of[e] = uint16_t(it->second);
+  }
+  t.rows = int(rows.size());
   return t;
 }
 
@@ -699,12 +729,12 @@ GenImageLayout gen_image_layout(const gagp_grammar* g, const DrawTables& t) {
   const int E = g->expression_count, NT = std::max(1, g->nonterminal_count);
   take(sizeof(gb::GenExpr) * size_t(E));  // expressions first: offset 0
   out.at.nt = take(sizeof(gb::GenNt) * size_t(NT));
-  out.at.head = take(sizeof(uint32_t) * t.head.size());
   out.at.level = take(sizeof(gb::GenLevel) * t.level.size());
   out.at.entry = take(sizeof(gb::GenEntry) * t.entry.size());
-  out.at.doms = take(sizeof(gagp_domain) * size_t(std::max(1, g->domain_count)));
+  out.at.doms = take(sizeof(gb::GenDomain) * size_t(std::max(1, g->domain_count)));
   out.at.vals = take(sizeof(gagp_value) * size_t(std::max(1, g->value_count)));
-  out.at.minimum = take(sizeof(uint16_t) * size_t(E) * g->depth_count * g->logical_depth_count);
+  out.at.cell = take(sizeof(uint32_t) * size_t(t.rows) * g->depth_count * g->logical_depth_count);
+  out.at.row_of = take(sizeof(uint16_t) * size_t(E));
   // children 4..7 (a bounded region's phases) only when an arity needs them
   int widest = 0;
   for (int i = 0; i < E; ++i)
@@ -721,41 +751,44 @@ std::vector<char> gen_image(const gagp_grammar* g, const std::vector<gb::ExprInf
   for (int i = 0; i < E; ++i) {
     const gagp_expression& x = g->expressions[i];
     gb::GenExpr& r = gx[i];
+    const int arity = info[i].arity;
+    const uint32_t cells = uint32_t(g->depth_count) * uint32_t(g->logical_depth_count);
+    auto child_of = [&](int k) { return k < arity && x.children[k] >= 0 && x.children[k] < E ? x.children[k] : 0; };
     for (int k = 0; k < 4; ++k) {
-      r.child[k] = k < GAGP_MAX_ARITY ? x.children[k] : -1;
-      r.child_scope[k] = k < GAGP_MAX_ARITY ? x.child_scope[k] : -1;
+      r.child[k] = uint16_t(child_of(k));
+      r.row[k] = t.row_of[child_of(k)] * cells;
     }
     r.target = x.target;
-    r.site_class = info[i].site_class;
-    r.kind = int8_t(x.kind);
-    r.arity = info[i].arity;
-    if (lay.at.extra && r.arity > 4) {
-      auto* extra = reinterpret_cast<int32_t*>(img.data() + lay.at.extra) + 8 * size_t(i);
+    r.shape = (uint32_t(info[i].site_class) & 0xffffu) | (uint32_t(arity) & 0xfu) << 16 |
+              uint32_t(x.kind == gb::EK_CONSTANT) << 20 | uint32_t(x.kind) << 24;
+    if (lay.at.extra && arity > 4) {
+      auto* extra = reinterpret_cast<uint32_t*>(img.data() + lay.at.extra) + 8 * size_t(i);
       for (int k = 4; k < 8; ++k) {
-        extra[k - 4] = x.children[k];
-        extra[4] |= int32_t(uint32_t(uint8_t(x.child_scope[k])) << (8 * (k - 4)));
+        extra[k - 4] = uint32_t(child_of(k));
+        extra[k] = t.row_of[child_of(k)] * cells;
       }
     }
-    // out-of-range counts keep their validity (admission bounds them anyway)
-    r.scope_count = int8_t(std::min(std::max(x.scope_count, -1), 100));
-    r.reserved = 0;
   }
   auto* nt = reinterpret_cast<gb::GenNt*>(img.data() + lay.at.nt);
   for (int i = 0; i < g->nonterminal_count; ++i) {
     const gagp_nonterminal& n = g->nonterminals[i];
     nt[i] = gb::GenNt{n.production_offset, n.production_count, n.scope_count, n.normalized_weights};
   }
-  std::memcpy(img.data() + lay.at.head, t.head.data(), sizeof(uint32_t) * t.head.size());
   std::memcpy(img.data() + lay.at.level, t.level.data(), sizeof(gb::GenLevel) * t.level.size());
   std::memcpy(img.data() + lay.at.entry, t.entry.data(), sizeof(gb::GenEntry) * t.entry.size());
-  if (g->domain_count) std::memcpy(img.data() + lay.at.doms, g->domains, sizeof(gagp_domain) * g->domain_count);
-  if (g->value_count) std::memcpy(img.data() + lay.at.vals, g->values, sizeof(gagp_value) * g->value_count);
-  auto* minimum = reinterpret_cast<uint16_t*>(img.data() + lay.at.minimum);
-  const size_t cells = size_t(E) * g->depth_count * g->logical_depth_count;
-  for (size_t i = 0; i < cells; ++i) {
-    const uint32_t v = g->minimum[i];
-    minimum[i] = v >= gb::kNoMinimum16 ? gb::kNoMinimum16 : uint16_t(v);
+  auto* doms = reinterpret_cast<gb::GenDomain*>(img.data() + lay.at.doms);
+  for (int i = 0; i < g->domain_count; ++i) {
+    const gagp_domain& x = g->domains[i];
+    gb::GenDomain& r = doms[i];
+    r.minimum = x.minimum;
+    r.width = x.integer_range ? uint64_t(x.maximum) - uint64_t(x.minimum) + 1 : uint64_t(x.value_count);
+    r.reject = r.width ? (0 - r.width) % r.width : 0;
+    r.magic = r.width ? ~uint64_t(0) / r.width : 0;
+    r.offset = x.integer_range ? -1 : x.value_offset;
   }
+  if (g->value_count) std::memcpy(img.data() + lay.at.vals, g->values, sizeof(gagp_value) * g->value_count);
+  std::memcpy(img.data() + lay.at.cell, t.cell.data(), sizeof(uint32_t) * t.cell.size());
+  std::memcpy(img.data() + lay.at.row_of, t.row_of.data(), sizeof(uint16_t) * t.row_of.size());
   return img;
 }
 

@@ -53,7 +53,7 @@ __global__ void k_init_population(const SearchDesc* descs, const int32_t* off, i
   GenResult g{ST_INVALID, 0, 0, 0};
   for (int logical = ramp, attempt = 0; g.status != ST_OK; ++attempt) {
     const int room = s.maxv < kCapacity ? s.maxv : kCapacity;
-    g = generate(s, s.gen_image, s.root_expression, 0, s.slot_max_depth, room,
+    g = generate<false>(s, s.gen_image, s.root_expression, 0, s.slot_max_depth, room,
                  mix64(s.seed ^ mix64((uint64_t(i) * 8 + 0) * 64 + uint64_t(attempt))), node, cval, logical, pending);
     // a statement program that reads a grammar local before assigning it
     // is retried with the next seed (phase_population_cpu.cpp:95-96)
@@ -751,8 +751,7 @@ __global__ void __launch_bounds__(128, 6) k_vary(const SearchDesc* descs, const 
     int reuse = -1, parent = -1;
     long long stamp[5] = {0, 0, 0, 0, 0};
     const long long started = clock64();
-    const int error = warp_vary_child(s, si == staged ? image : s.gen_image, child, s.round_seed[0], rows, &reuse,
-                                      &parent, stamp);
+    const int error = warp_vary_child(s, image, si == staged, child, s.round_seed[0], rows, &reuse, &parent, stamp);
     if (lane == 0 && collect_stats) {
       // per-phase SM cycles: selection, crossover, subtree generation, rest
       stamp[3] = clock64();

@@ -235,8 +235,8 @@ __device__ inline bool warp_locals_defined(const SearchDesc& s, const uint64_t* 
 // after selection, after crossover, after the mutation's subtree generation
 // (left 0 for phases not reached); stamp[4]: the generation's steps + 1 on
 // lane 0 (left 0 without a generation).
-__device__ inline int warp_vary_child(const SearchDesc& s, const char* image, int child, uint64_t seed, WarpRows& w,
-                                      int* reuse_out, int* parent_out, long long* stamp) {
+__device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bool staged, int child, uint64_t seed,
+                                      WarpRows& w, int* reuse_out, int* parent_out, long long* stamp) {
   const int lane = lane_id();
   *reuse_out = -1;
   // ---- crossover_child
@@ -295,15 +295,13 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, in
         const bool capped = s.mutation_max_nodes > 0 && s.mutation_max_nodes < uncapped;
         const int bounded = capped ? s.mutation_max_nodes : uncapped;
         const uint64_t gseed = m.next();
-        GenResult g{ST_INVALID, 0, 0, 0};
-        if (lane == 0) {
-          g = generate(s, image, entry, 0, s.slot_max_depth - depth + 1, bounded, gseed, w.gen.node, w.gen.cval,
-                       logical, w.pending);
-          stamp[4] = (long long)g.steps + 1;
-        }
-        g.status = __shfl_sync(kFull, g.status, 0);
-        g.nodes = __shfl_sync(kFull, g.nodes, 0);
-        g.constants = __shfl_sync(kFull, g.constants, 0);
+        // two copies of the generator, so that the staged one reads its
+        // tables with shared-memory loads and not generic ones
+        const GenResult g = staged ? generate<true>(s, image, entry, 0, s.slot_max_depth - depth + 1, bounded, gseed,
+                                                    w.gen.node, w.gen.cval, logical, w.pending)
+                                   : generate<true>(s, s.gen_image, entry, 0, s.slot_max_depth - depth + 1, bounded,
+                                                    gseed, w.gen.node, w.gen.cval, logical, w.pending);
+        stamp[4] = (long long)g.steps + 1;
         __syncwarp();
         stamp[2] = clock64();
         if (capped && g.status == ST_CAPACITY) {

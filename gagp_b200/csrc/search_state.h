@@ -41,14 +41,15 @@ struct ExprInfo {
 };
 
 // Subtree-generation view of one expression, two 16-byte loads: the first
-// four children, then target (nonterminal or domain), the crossover class of
-// the sites it opens, kind / arity / scope count and the children's scopes.
+// four children, the target (nonterminal or domain), the crossover class of
+// the sites it opens, and its kind << 24 with the arity and constant bits as a
+// node word's upper half holds them; then the children's rows in the cell
+// table (GenImage::cell), as offsets of their first words.
 struct alignas(16) GenExpr {
-  int32_t child[4];
+  uint16_t child[4];
   int32_t target;
-  int32_t site_class;
-  int8_t kind, arity, scope_count, reserved;
-  int8_t child_scope[4];
+  uint32_t shape;   // crossover class (16 bits) | arity << 16 | constant << 20 | kind << 24
+  uint32_t row[4];
 };
 // A nonterminal in one 16-byte load.
 struct alignas(16) GenNt {
@@ -57,38 +58,50 @@ struct alignas(16) GenNt {
 // Precomputed production draw of one nonterminal at one (depth, site
 // budget) for one feasibility level: the productions whose minimum cost is at
 // most `bound` are the feasible ones, and the draw over them is decided by
-// comparing the choice value with per-production thresholds (GenEntry).  A
+// comparing the draw's 53 bits with per-production limits (GenEntry).  A
 // nonterminal's levels at one (depth, site budget) form a chain from the
 // widest (every production of finite cost) down through `below`.
 struct alignas(16) GenLevel {
-  double total;     // the draw's weight sum; NaN: no precomputed draw
-  uint32_t bound;   // largest minimum cost of a feasible production (kNoId: none)
-  uint32_t entry;   // first of the nonterminal's production_count GenEntry
-  int32_t last;     // the last feasible production: the pick when no threshold exceeds the choice
+  uint32_t bound;   // largest minimum cost of a feasible production (kNoId: no precomputed draw)
+  uint32_t entry;   // first of the nonterminal's `count` GenEntry
+  uint32_t count;
   int32_t below;    // the next narrower level, -1: none
-  int32_t reserved[2];
 };
-// One production of a level's draw: the smallest choice value whose running
-// difference after this production is not negative (0: never picked), the
-// production's expression and its minimum cost at the level's (depth, site
-// budget).
+// One production of a level's draw: it is picked for draws (53 bits) below
+// `limit` and not below an earlier production's (0: never; the last feasible
+// one's is past every draw).
 struct alignas(16) GenEntry {
-  double threshold;
+  uint64_t limit;
   int32_t expression;
-  uint32_t need;
+  uint32_t reserved;
+};
+// A constant domain: an Int range of `width` values from `minimum` (0: every
+// Int), or `width` listed values from vals[offset].  A draw below `reject` is
+// drawn again (2^64 mod width), and floor((2^64 - 1) / width) gives residues
+// without a division (Rng::bounded_fixed).
+struct alignas(16) GenDomain {
+  int64_t minimum;
+  uint64_t width, reject, magic;
+  int32_t offset;  // -1: a range
+  int32_t reserved[3];
 };
 
 // Byte offsets of the subtree generator's image sections (GenExpr[n_ex] at
-// offset 0, each section 16-byte aligned): GenNt[n_nts]; head[depth_count *
-// logical_count * n_nts], the widest GenLevel of each nonterminal at each
-// (depth, site budget) (0: no precomputed draw); the GenLevel table (level 0
-// is the empty one) and GenEntry table, each record held once however many
-// heads share it; gagp_domain[n_doms]; gagp_value[n_vals]; the minimum cost
-// table as uint16 (kNoMinimum16: infeasible).
+// offset 0, each section 16-byte aligned): GenNt[n_nts]; the GenLevel table
+// (level 0 is the empty one) and GenEntry table, each record held once however
+// many cells share it; GenDomain[n_doms]; gagp_value[n_vals]; and `cell`, what
+// a task of an expression needs at each (depth, site budget): a word per cell
+// [depth_count * logical_count] and row, the minimum cost as 16 bits
+// (kNoMinimum16: infeasible) and, << 16, a reference's widest GenLevel there
+// (0: no precomputed draw; kNoReference: not a reference).  Expressions with
+// equal words share a row; `row_of` is each expression's row (uint16).
 struct GenImage {
-  int32_t nt, head, level, entry, doms, vals, minimum;
-  int32_t extra;  // children 4..7 of each expression and their scopes (two int4), when an arity exceeds 4
+  int32_t nt, level, entry, doms, vals, cell, row_of;
+  int32_t extra;  // children 4..7 of each expression and their rows (two int4), when an arity exceeds 4
 };
+constexpr uint32_t kNoReference = 0xffff;
+// GenExpr::shape's parts.
+constexpr uint32_t kShapeNode = 0x1f0000;  // arity and constant bits of a node word's upper half
 constexpr uint16_t kNoMinimum16 = 0xffff;
 
 // A traversal table entry (the reference's PhaseRegionInfo for a traversal,
