@@ -57,16 +57,22 @@ struct Rng {
   __device__ __forceinline__ uint64_t bounded(uint64_t upper) {
     if (upper - 1 < uint64_t(kSmallBound)) {
       // the same rejection bound and residue from 32-bit arithmetic, with no
-      // table load on the generator's dependent chain: m = 2^32 mod u, so
-      // the bound (2^64 - u) mod u = 2^64 mod u = m^2 mod u, and a draw
-      // v = hi * 2^32 + lo has v mod u = ((hi mod u) * m + lo mod u) mod u
-      // (every intermediate below 2^32 for u <= 2^16)
-      const uint32_t u = uint32_t(upper);
-      const uint32_t m = (0u - u) % u;
-      const uint32_t threshold = (m * m) % u;
+      // table load on the generator's dependent chain: with m = 2^32 mod u, a
+      // draw v = hi * 2^32 + lo has v mod u = ((hi mod u) * m + lo mod u) mod u
+      // and the bound (2^64 - u) mod u is m^2 mod u (every intermediate below
+      // 2^32 for u <= 2^16).  One division gives q = floor((2^32 - 1) / u);
+      // floor(x q / 2^32) is then at most one below floor(x / u), because
+      // q >= 2^32 / u - 1.  Only a draw below 2^16 can be below the bound.
+      const uint32_t u = uint32_t(upper), q = 0xffffffffu / u, t = 0xffffffffu - q * u;
+      const uint32_t m = t + 1 == u ? 0 : t + 1;
+      auto mod = [u, q](uint32_t x) -> uint32_t {
+        const uint32_t r = x - __umulhi(x, q) * u;
+        return r >= u ? r - u : r;
+      };
       for (;;) {
         const uint64_t v = next();
-        if (v >= threshold) return ((uint32_t(v >> 32) % u) * m + uint32_t(v) % u) % u;
+        if (v < kSmallBound && v < mod(m * m)) continue;
+        return mod(mod(uint32_t(v >> 32)) * m + mod(uint32_t(v)));
       }
     }
     const uint64_t threshold = (0 - upper) % upper;
@@ -476,18 +482,18 @@ struct SRow {
 
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
-__device__ inline void warp_copy(const uint64_t* from_node, const int64_t* from_cval, int n, int nc, uint64_t* to_node,
-                                 int64_t* to_cval) {
-  for (int i = lane_id(); i < n; i += 32) to_node[i] = from_node[i];
-  for (int i = lane_id(); i < nc; i += 32) to_cval[i] = from_cval[i];
-  __syncwarp();
-}
-
 // site_matches (phase_operators.cuh:51-54): a variation site of class `cls`
 // (any class when cls == kNoClass).
 __device__ __forceinline__ bool site_matches(uint64_t w, uint32_t cls) {
   const uint32_t c = w_class(w);
   return c != kNoClass && (cls == kNoClass || c == cls);
+}
+
+// The position of set bit `rank` (from 0) of `mask`: the lane that many set
+// bits lie below.  Every lane passes the same arguments.
+__device__ __forceinline__ int warp_nth_bit(unsigned mask, unsigned rank) {
+  const unsigned lane = lane_id();
+  return __ffs(__ballot_sync(kFull, (mask >> lane & 1u) && unsigned(__popc(mask & ((1u << lane) - 1u))) == rank)) - 1;
 }
 
 // choose_site (phase_operators.cuh:55-83 and the counted warp variant
@@ -505,12 +511,9 @@ __device__ inline int warp_choose_site(const SRow& t, Rng& random, bool counted,
     unsigned rank = unsigned(random.bounded(count));
     for (int chunk = 0; chunk < t.n; chunk += 32) {
       const int i = chunk + lane;
-      unsigned mask = __ballot_sync(kFull, i < t.n && site_matches(t.node[i], cls));
+      const unsigned mask = __ballot_sync(kFull, i < t.n && site_matches(t.node[i], cls));
       const unsigned c = __popc(mask);
-      if (rank < c) {
-        for (unsigned j = 0; j < rank; ++j) mask &= mask - 1;
-        return chunk + __ffs(mask) - 1;
-      }
+      if (rank < c) return chunk + warp_nth_bit(mask, rank);
       rank -= c;
     }
     return -1;
@@ -531,23 +534,16 @@ __device__ inline int warp_choose_site(const SRow& t, Rng& random, bool counted,
 
 // phase_subtree_end (device/phase_variation.cuh:81-91, warp form :213-229).
 __device__ inline int warp_subtree_end(const SRow& t, int start) {
+  // node words hold their depth: the subtree ends at the next node no deeper
+  // than its root
   if (start < 0 || start >= t.n) return -1;
-  const int lane = lane_id();
-  int pending = 1;
-  for (int chunk = start; chunk < t.n; chunk += 32) {
+  const int lane = lane_id(), depth = w_depth(t.node[start]);
+  for (int chunk = start + 1; chunk < t.n; chunk += 32) {
     const int i = chunk + lane;
-    const bool live = i < t.n;
-    int scan = live ? w_arity(t.node[i]) - 1 : 0;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int up = __shfl_up_sync(kFull, scan, o);
-      if (lane >= o) scan += up;
-    }
-    const unsigned hit = __ballot_sync(kFull, live && pending + scan == 0);
-    if (hit) return chunk + __ffs(hit);
-    pending += __shfl_sync(kFull, scan, 31);
+    const unsigned hit = __ballot_sync(kFull, i < t.n && w_depth(t.node[i]) <= depth);
+    if (hit) return chunk + __ffs(hit) - 1;
   }
-  return -1;
+  return t.n;
 }
 
 // Constant nodes among row positions [0, first) and [0, second), first <= second.
@@ -563,24 +559,17 @@ __device__ __forceinline__ void warp_count_constants2(const SRow& t, int first, 
   *b = cb;
 }
 
-template <typename T>
-__device__ __forceinline__ T warp_max(T v) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const T u = __shfl_xor_sync(kFull, v, o);
-    v = u > v ? u : v;
-  }
-  return v;
-}
-
 // splice_phase_tree (device/phase_variation.cuh:147-207): base with the
 // subtree [dest, end) replaced by donor's subtree [src, donor_end), into
 // `out`; the callers have found both subtree ends already.
 // Depth and site-depth limits are maxima of the output words; constants are
 // base[..dest) ++ donor subtree ++ base[end..), the prefix renumbering the
 // reference performs node by node.  Every lane returns the same result.
-__device__ inline GenResult warp_splice(const SRow& base, int dest, int end, const SRow& donor, int src, int donor_end,
-                                        SRow out, int stride, int max_depth, int site_limit) {
+// `base_within`: base's own nodes are known to keep both limits, so only the
+// donor's subtree is checked, before anything is written: most rejected
+// splices are.
+__device__ inline GenResult warp_splice(const SRow& base, bool base_within, int dest, int end, const SRow& donor, int src,
+                                        int donor_end, SRow out, int stride, int max_depth, int site_limit) {
   GenResult r{ST_INVALID, 0, 0};
   if (max_depth <= 0 || max_depth > 64 || base.n <= 0 || donor.n <= 0 || dest < 0 || dest >= base.n || src < 0 ||
       src >= donor.n)
@@ -594,6 +583,18 @@ __device__ inline GenResult warp_splice(const SRow& base, int dest, int end, con
   if (length > stride) { r.status = ST_CAPACITY; return r; }  // never reached: callers bound by the node budget
   const int ddepth = w_depth(a) - w_depth(b), dsval = w_sval(a) - w_sval(b);
   int maxd = 0, maxs = 0;
+  for (int i = src + lane_id(); i < donor_end; i += 32) {
+    const uint64_t w = w_shift(donor.node[i], ddepth, dsval);
+    maxd = max(maxd, w_depth(w));
+    maxs = max(maxs, w_sval(w));
+  }
+  if (!base_within)
+    for (int i = lane_id(); i < base.n; i += 32)
+      if (i < dest || i >= end) {
+        maxd = max(maxd, w_depth(base.node[i]));
+        maxs = max(maxs, w_sval(base.node[i]));
+      }
+  if (__any_sync(kFull, maxd > max_depth || (site_limit && maxs > site_limit))) { r.status = ST_CAPACITY; return r; }
   for (int i = lane_id(); i < length; i += 32) {
     uint64_t w;
     if (i >= dest && i < dest + inserted) {
@@ -603,8 +604,6 @@ __device__ inline GenResult warp_splice(const SRow& base, int dest, int end, con
       w = base.node[i < dest ? i : i + (end - dest) - inserted];
     }
     out.node[i] = w;
-    maxd = max(maxd, w_depth(w));
-    maxs = max(maxs, w_sval(w));
   }
   int bb, be, db, de;
   warp_count_constants2(base, dest, end, &bb, &be);
@@ -613,11 +612,7 @@ __device__ inline GenResult warp_splice(const SRow& base, int dest, int end, con
   for (int k = lane_id(); k < bb; k += 32) out.cval[k] = base.cval[k];
   for (int k = lane_id(); k < dc; k += 32) out.cval[bb + k] = donor.cval[db + k];
   for (int k = lane_id(); k < base.nc - be; k += 32) out.cval[bb + dc + k] = base.cval[be + k];
-  maxd = warp_max(maxd);
-  maxs = warp_max(maxs);
   __syncwarp();
-  if (maxd > max_depth) { r.status = ST_CAPACITY; return r; }
-  if (site_limit && maxs > site_limit) { r.status = ST_CAPACITY; return r; }
   r.status = ST_OK;
   r.nodes = length;
   r.constants = bb + dc + (base.nc - be);

@@ -235,21 +235,29 @@ __device__ inline bool warp_locals_defined(const SearchDesc& s, const uint64_t* 
 // after selection, after crossover, after the mutation's subtree generation
 // (left 0 for phases not reached); stamp[4]: the generation's steps + 1 on
 // lane 0 (left 0 without a generation).
-__device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bool staged, int child, uint64_t seed,
+__device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bool staged, int index, uint64_t seed,
                                       WarpRows& w, int* reuse_out, int* parent_out, long long* stamp) {
   const int lane = lane_id();
   *reuse_out = -1;
   // ---- crossover_child
-  Rng random(seed ^ (0x617089e168ULL + uint64_t(child)));
+  Rng random(seed ^ (0x617089e168ULL + uint64_t(index)));
   int parent, donor;
   warp_tournaments(s, random, &parent, &donor);
   *parent_out = parent;
   load_members(s, parent, w.parent, donor, w.donor);
   stamp[0] = clock64();
   if (w.parent.n <= 0 || w.parent.n > s.maxv || w.parent.nc > w.parent.n) return 1;
-  warp_copy(w.parent.node, w.parent.cval, w.parent.n, w.parent.nc, w.child.node, w.child.cval);
-  w.child.n = w.parent.n;
-  w.child.nc = w.parent.nc;
+  // the child is the parent's row until a splice replaces it; a splice goes
+  // to the one of the two row buffers the child does not occupy
+  SRow child = w.parent;
+  bool crossed = false, mutated = false;
+  // whether the parent's nodes keep the splices' limits (an imported row may
+  // be deeper than the depth limit, and then every splice that keeps the deep
+  // part is rejected)
+  bool within = true;
+  for (int i = lane; i < w.parent.n; i += 32)
+    within &= w_depth(w.parent.node[i]) <= s.slot_max_depth && (!s.site_depth || w_sval(w.parent.node[i]) <= s.site_depth);
+  within = __all_sync(kFull, within);
   const int total = w.parent.n;
   const bool gated = s.crossover_probability < 1 && random.unit() >= s.crossover_probability;
   if (!gated) {
@@ -262,14 +270,15 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bo
       const int ae = warp_subtree_end(w.parent, dest), be = warp_subtree_end(w.donor, src);
       if (ae < 0 || be < 0) return 3;
       if (total - (ae - dest) + (be - src) > s.maxv) continue;
-      const GenResult r = warp_splice(w.parent, dest, ae, w.donor, src, be, w.out, s.stride, s.slot_max_depth,
+      const GenResult r = warp_splice(w.parent, within, dest, ae, w.donor, src, be, w.out, s.stride, s.slot_max_depth,
                                       s.site_depth);
       // a splice that reads a grammar local before assigning it is a
       // rejected attempt (crossover_child, phase_operators.cuh:185)
       if (r.status == ST_OK && warp_locals_defined(s, w.out.node, r.nodes)) {
-        warp_copy(w.out.node, w.out.cval, r.nodes, r.constants, w.child.node, w.child.cval);
-        w.child.n = r.nodes;
-        w.child.nc = r.constants;
+        child = w.out;
+        child.n = r.nodes;
+        child.nc = r.constants;
+        crossed = true;
         break;
       }
     }
@@ -277,20 +286,20 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bo
   stamp[1] = clock64();
   // ---- mutate_child
   {
-    Rng m(seed ^ (0x124ab512bf01ULL + uint64_t(child)));
+    Rng m(seed ^ (0x124ab512bf01ULL + uint64_t(index)));
     if (m.unit() < s.mutation_probability) {
       if (s.uniform_phase) (void)m.bounded(1);
-      const int dest = warp_choose_site(w.child, m, s.counted, kNoClass);
+      const int dest = warp_choose_site(child, m, s.counted, kNoClass);
       if (dest >= 0) {
-        const uint64_t a = w.child.node[dest];
-        const int end = warp_subtree_end(w.child, dest), depth = w_depth(a);
+        const uint64_t a = child.node[dest];
+        const int end = warp_subtree_end(child, dest), depth = w_depth(a);
         if (end < 0 || depth < 1) return 6;
         const int entry = w_entry(a);
         const int incoming = s.site_depth ? w_sval(a) - 1 : 0;
         if (incoming < 0 || incoming > s.site_depth) return 6;
         const int logical = s.site_depth - incoming;
         const int replaced = end - dest;
-        const int whole = s.maxv - (w.child.n - replaced), phase = kCapacity - (w.child.n - replaced);
+        const int whole = s.maxv - (child.n - replaced), phase = kCapacity - (child.n - replaced);
         const int available = whole < phase ? whole : phase, uncapped = available < kCapacity ? available : kCapacity;
         const bool capped = s.mutation_max_nodes > 0 && s.mutation_max_nodes < uncapped;
         const int bounded = capped ? s.mutation_max_nodes : uncapped;
@@ -311,16 +320,18 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bo
         } else {
           w.gen.n = g.nodes;
           w.gen.nc = g.constants;
-          const GenResult r = warp_splice(w.child, dest, end, w.gen, 0, w.gen.n, w.out, s.stride, s.slot_max_depth,
-                                          s.site_depth);
+          const SRow to = crossed ? w.child : w.out;
+          const GenResult r = warp_splice(child, within || crossed, dest, end, w.gen, 0, w.gen.n, to, s.stride,
+                                          s.slot_max_depth, s.site_depth);
           if (r.status != ST_OK) return 8;
           // a mutation that reads a grammar local before assigning it is
           // dropped and the crossed child stands (mutate_child,
           // phase_operators.cuh:240-241)
-          if (warp_locals_defined(s, w.out.node, r.nodes)) {
-            warp_copy(w.out.node, w.out.cval, r.nodes, r.constants, w.child.node, w.child.cval);
-            w.child.n = r.nodes;
-            w.child.nc = r.constants;
+          if (warp_locals_defined(s, to.node, r.nodes)) {
+            child = to;
+            child.n = r.nodes;
+            child.nc = r.constants;
+            mutated = true;
           }
         }
       }
@@ -330,30 +341,32 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bo
   // phase_population_cpu.cpp:283-290): the first elite_count children are
   // the best members, each reusing its own completed result (an identical
   // program: the same result as the parent or member the reference finds)
-  if (s.generational && child < s.elite_count) {
-    const int src = s.elites[child];
+  if (s.generational && index < s.elite_count) {
+    const int src = s.elites[index];
     const int32_t l = s.len[src];
     for (int i = lane; i < len_nodes(l); i += 32)
-      s.cnode[size_t(child) * s.stride + i] = s.node[size_t(src) * s.stride + i];
+      s.cnode[size_t(index) * s.stride + i] = s.node[size_t(src) * s.stride + i];
     for (int i = lane; i < len_consts(l); i += 32)
-      s.ccval[size_t(child) * s.stride + i] = s.cval[size_t(src) * s.stride + i];
-    if (lane == 0) s.clen[child] = l;
+      s.ccval[size_t(index) * s.stride + i] = s.cval[size_t(src) * s.stride + i];
+    if (lane == 0) s.clen[index] = l;
     *reuse_out = src;
     return 0;
   }
   // ---- compare_child: identical construction records and constants
-  bool equal = w.child.n == w.parent.n && w.child.nc == w.parent.nc;
-  if (equal) {
+  bool equal = child.n == w.parent.n && child.nc == w.parent.nc;
+  if (equal && (crossed || mutated)) {
     bool mine = true;
-    for (int i = lane; i < w.child.n; i += 32) mine &= w_origin(w.child.node[i]) == w_origin(w.parent.node[i]);
-    for (int i = lane; i < w.child.nc; i += 32) mine &= w.child.cval[i] == w.parent.cval[i];
+    for (int i = lane; i < child.n; i += 32) mine &= w_origin(child.node[i]) == w_origin(w.parent.node[i]);
+    for (int i = lane; i < child.nc; i += 32) mine &= child.cval[i] == w.parent.cval[i];
     equal = __all_sync(kFull, mine);
   }
   if (equal) *reuse_out = parent;
   // ---- publish the child row
-  for (int i = lane; i < w.child.n; i += 32) s.cnode[size_t(child) * s.stride + i] = w.child.node[i];
-  for (int i = lane; i < w.child.nc; i += 32) s.ccval[size_t(child) * s.stride + i] = w.child.cval[i];
-  if (lane == 0) s.clen[child] = make_len(w.child.n, w.child.nc);
+  for (int i = lane; i < child.n; i += 32) s.cnode[size_t(index) * s.stride + i] = child.node[i];
+  for (int i = lane; i < child.nc; i += 32) s.ccval[size_t(index) * s.stride + i] = child.cval[i];
+  if (lane == 0) s.clen[index] = make_len(child.n, child.nc);
+  w.child.n = child.n;  // the caller's statistics
+  w.child.nc = child.nc;
   return 0;
 }
 
