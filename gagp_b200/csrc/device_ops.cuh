@@ -43,6 +43,24 @@ constexpr unsigned kFull = 0xffffffffu;
 // domains) draw with 32-bit arithmetic only (Rng::bounded).
 constexpr uint64_t kSmallBound = uint64_t(1) << 16;
 
+// A range u of 1 .. 2^16 and what a bounded draw over it needs.  With
+// m = 2^32 mod u, a draw v = hi * 2^32 + lo has v mod u =
+// ((hi mod u) * m + lo mod u) mod u, and the rejection bound (2^64 - u) mod u is
+// m^2 mod u (every intermediate below 2^32).  One division gives
+// q = floor((2^32 - 1) / u); floor(x q / 2^32) is then at most one below
+// floor(x / u), because q >= 2^32 / u - 1.
+struct SmallRange {
+  uint32_t u, q, m;
+  __device__ __forceinline__ explicit SmallRange(uint32_t range) : u(range), q(0xffffffffu / range) {
+    const uint32_t t = 0xffffffffu - q * u;
+    m = t + 1 == u ? 0 : t + 1;
+  }
+  __device__ __forceinline__ uint32_t mod(uint32_t x) const {
+    const uint32_t r = x - __umulhi(x, q) * u;
+    return r >= u ? r - u : r;
+  }
+};
+
 // SplitMix64 stream with rejection-sampled bounds
 // (DGrammarRandom, cpp/src/evolution/repro/gpu/device/grammar_random.cuh:10-51).
 struct Rng {
@@ -54,27 +72,17 @@ struct Rng {
     v = (v ^ (v >> 27)) * 0x94d049bb133111ebULL;
     return v ^ (v >> 31);
   }
-  __device__ __forceinline__ uint64_t bounded(uint64_t upper) {
-    if (upper - 1 < uint64_t(kSmallBound)) {
-      // the same rejection bound and residue from 32-bit arithmetic, with no
-      // table load on the generator's dependent chain: with m = 2^32 mod u, a
-      // draw v = hi * 2^32 + lo has v mod u = ((hi mod u) * m + lo mod u) mod u
-      // and the bound (2^64 - u) mod u is m^2 mod u (every intermediate below
-      // 2^32 for u <= 2^16).  One division gives q = floor((2^32 - 1) / u);
-      // floor(x q / 2^32) is then at most one below floor(x / u), because
-      // q >= 2^32 / u - 1.  Only a draw below 2^16 can be below the bound.
-      const uint32_t u = uint32_t(upper), q = 0xffffffffu / u, t = 0xffffffffu - q * u;
-      const uint32_t m = t + 1 == u ? 0 : t + 1;
-      auto mod = [u, q](uint32_t x) -> uint32_t {
-        const uint32_t r = x - __umulhi(x, q) * u;
-        return r >= u ? r - u : r;
-      };
-      for (;;) {
-        const uint64_t v = next();
-        if (v < kSmallBound && v < mod(m * m)) continue;
-        return mod(mod(uint32_t(v >> 32)) * m + mod(uint32_t(v)));
-      }
+  // 32-bit arithmetic only, with no table load on the dependent chain; only a
+  // draw below 2^16 can be below the rejection bound
+  __device__ __forceinline__ uint32_t bounded(const SmallRange& r) {
+    for (;;) {
+      const uint64_t v = next();
+      if (v < kSmallBound && v < r.mod(r.m * r.m)) continue;
+      return r.mod(r.mod(uint32_t(v >> 32)) * r.m + r.mod(uint32_t(v)));
     }
+  }
+  __device__ __forceinline__ uint64_t bounded(uint64_t upper) {
+    if (upper - 1 < uint64_t(kSmallBound)) return bounded(SmallRange(uint32_t(upper)));
     const uint64_t threshold = (0 - upper) % upper;
     for (;;) {
       const uint64_t v = next();
@@ -494,6 +502,25 @@ __device__ __forceinline__ bool site_matches(uint64_t w, uint32_t cls) {
 __device__ __forceinline__ int warp_nth_bit(unsigned mask, unsigned rank) {
   const unsigned lane = lane_id();
   return __ffs(__ballot_sync(kFull, (mask >> lane & 1u) && unsigned(__popc(mask & ((1u << lane) - 1u))) == rank)) - 1;
+}
+
+// The variation sites of a row of at most 64 nodes (of class `cls`, of any when
+// cls == kNoClass), kept so that a draw among them reads the row only once:
+// crossover attempts draw from the same row again and again.
+struct SiteSet {
+  unsigned low, high;
+  SmallRange range;
+};
+__device__ __forceinline__ SiteSet warp_sites(const SRow& t, uint32_t cls) {
+  const int i = lane_id(), j = i + 32;
+  const unsigned low = __ballot_sync(kFull, i < t.n && site_matches(t.node[i], cls));
+  const unsigned high = __ballot_sync(kFull, j < t.n && site_matches(t.node[j], cls));
+  return SiteSet{low, high, SmallRange(max(1u, unsigned(__popc(low) + __popc(high))))};
+}
+__device__ __forceinline__ int choose_site(const SiteSet& sites, Rng& random) {
+  if (!(sites.low | sites.high)) return -1;
+  const unsigned rank = random.bounded(sites.range), first = unsigned(__popc(sites.low));
+  return rank < first ? warp_nth_bit(sites.low, rank) : 32 + warp_nth_bit(sites.high, rank - first);
 }
 
 // choose_site (phase_operators.cuh:55-83 and the counted warp variant

@@ -261,11 +261,20 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bo
   const int total = w.parent.n;
   const bool gated = s.crossover_probability < 1 && random.unit() >= s.crossover_probability;
   if (!gated) {
-    if (s.uniform_phase) (void)random.bounded(1);
+    if (s.uniform_phase) (void)random.next();  // bounded(1) over the row's one phase
+    const bool small = s.counted && w.parent.n <= 64 && w.donor.n <= 64;
+    const SiteSet sites = warp_sites(w.parent, kNoClass);
+    uint32_t donor_class = small ? w_class(w.donor.node[0]) : 0u;
+    SiteSet donor_sites = warp_sites(w.donor, donor_class);
     for (int attempt = 0; attempt < s.attempts; ++attempt) {
-      const int dest = warp_choose_site(w.parent, random, s.counted, kNoClass);
+      const int dest = small ? choose_site(sites, random) : warp_choose_site(w.parent, random, s.counted, kNoClass);
       if (dest < 0) break;
-      const int src = warp_choose_site(w.donor, random, s.counted, w_class(w.parent.node[dest]));
+      const uint32_t cls = w_class(w.parent.node[dest]);
+      if (small && cls != donor_class) {
+        donor_class = cls;
+        donor_sites = warp_sites(w.donor, cls);
+      }
+      const int src = small ? choose_site(donor_sites, random) : warp_choose_site(w.donor, random, s.counted, cls);
       if (src < 0) continue;
       const int ae = warp_subtree_end(w.parent, dest), be = warp_subtree_end(w.donor, src);
       if (ae < 0 || be < 0) return 3;
@@ -288,8 +297,9 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bo
   {
     Rng m(seed ^ (0x124ab512bf01ULL + uint64_t(index)));
     if (m.unit() < s.mutation_probability) {
-      if (s.uniform_phase) (void)m.bounded(1);
-      const int dest = warp_choose_site(child, m, s.counted, kNoClass);
+      if (s.uniform_phase) (void)m.next();
+      const int dest = s.counted && child.n <= 64 ? choose_site(warp_sites(child, kNoClass), m)
+                                                  : warp_choose_site(child, m, s.counted, kNoClass);
       if (dest >= 0) {
         const uint64_t a = child.node[dest];
         const int end = warp_subtree_end(child, dest), depth = w_depth(a);
