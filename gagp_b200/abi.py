@@ -116,6 +116,19 @@ class Verdict(C.Structure):
                 "solved": self.correct == self.cases}
 
 
+def verdict_summaries(verdicts, count: int) -> List[dict]:
+    """``summary()`` of the first ``count`` entries of a ``Verdict`` array."""
+    v = np.frombuffer(verdicts, dtype=_VERDICT, count=count)
+    n = v["cases"].astype(np.float64)
+    return [{"cases": a, "correct": b, "wrong": c, "runtime_errors": d, "mean_loss": e, "solved": f}
+            for a, b, c, d, e, f in zip(n.tolist(), v["correct"].astype(np.float64).tolist(),
+                                        (n - v["correct"]).tolist(), v["runtime_errors"].astype(np.float64).tolist(),
+                                        (v["loss"] / n).tolist(), (v["correct"] == v["cases"]).tolist())]
+
+
+_VERDICT = np.dtype(Verdict)
+
+
 class SearchResult(C.Structure):
     _fields_ = [("generations", C.c_int32), ("history_best_fitness", C.POINTER(C.c_double)),
                 ("history_mean_fitness", C.POINTER(C.c_double)), ("history_best_wrong", C.POINTER(C.c_int32)),
@@ -166,13 +179,14 @@ class GrammarBlob:
         self.tables = t
         n = len(t.expressions)
         self.expressions = (Expression * n)()
-        for i, e in enumerate(t.expressions):
-            x = self.expressions[i]
-            x.kind, x.node_kind, x.opcode, x.operand, x.arity = e.kind, e.node_kind, e.opcode, e.operand, e.arity
-            x.fuel, x.merge_fuel, x.type, x.target, x.scope_count = e.fuel, e.merge_fuel, e.type, e.target, e.scope_count
-            for k in range(MAX_ARITY):
-                x.children[k] = e.children[k]
-                x.child_scope[k] = e.child_scope[k]
+        if n:  # one array of the fields, not one assignment per field
+            fields = np.array([(e.kind, e.node_kind, e.opcode, e.operand, e.arity, e.fuel, e.merge_fuel, e.type,
+                                e.target, e.scope_count, *e.children[:MAX_ARITY], *e.child_scope[:MAX_ARITY])
+                               for e in t.expressions], dtype=np.int64)
+            words = np.frombuffer(self.expressions, dtype=np.int32).reshape(n, -1)
+            words[:, :10 + MAX_ARITY] = fields[:, :10 + MAX_ARITY]
+            scopes = np.frombuffer(self.expressions, dtype=np.int8).reshape(n, -1)
+            scopes[:, 4 * (10 + MAX_ARITY):4 * (10 + MAX_ARITY) + MAX_ARITY] = fields[:, 10 + MAX_ARITY:]
         self.productions = (Production * max(1, len(t.productions)))()
         for i, (x, w) in enumerate(t.productions):
             self.productions[i].expression, self.productions[i].weight = x, w

@@ -18,6 +18,7 @@
 #include <map>
 #include <tuple>
 #include <memory>
+#include <new>
 #include <mutex>
 #include <numeric>
 #include <string>
@@ -126,7 +127,7 @@ struct gagp_engine {
   // stream-ordered pool of the searches' device blocks: admission and
   // retirement neither allocate from the driver nor synchronize the device
   cudaMemPool_t pool = nullptr;
-  // pinned staging of result downloads (grown on demand)
+  // pinned staging of result downloads and row evaluations (grown on demand)
   char* pinned = nullptr;
   size_t pinned_bytes = 0;
   // VM autotuner: per batch shape, the fast VM's cases per lane, chosen by
@@ -949,6 +950,18 @@ Plan plan_search(const gagp_grammar* g, const gagp_cases* c, const gagp_search_c
   p.hist_nodes = L.take(4 * H); p.hist_node = L.take(8 * S * H); p.hist_cval = L.take(8 * S * H);
   p.hist_len = L.take(4 * H); p.counters = L.take(8 * GAGP_COUNTERS);
   return p;
+}
+
+// The engine's pinned staging, grown to `bytes`.  Nothing is in flight in it:
+// every user waits for its copies before it returns.
+gagp_status pinned_at_least(gagp_engine* e, size_t bytes) {
+  if (bytes <= e->pinned_bytes) return GAGP_OK;
+  if (e->pinned) cudaFreeHost(e->pinned);
+  e->pinned = nullptr;
+  e->pinned_bytes = 0;
+  CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&e->pinned), bytes));
+  e->pinned_bytes = bytes;
+  return GAGP_OK;
 }
 
 template <class T>
@@ -2028,7 +2041,7 @@ struct EvalPlan {
   Layout L;
   size_t desc, ex, info, minimum, local_types, regions, inputs, expected, lists, node, cval, len, code, code_len, kpool,
       code_temps, vm_acc, bc, bc_len, bc_locals, bc_consts, fitness, wrong, errors, counters, round, fast, exact,
-      general, counts, off, region_list, region_ws;
+      general, counts, off, region_list, region_ws, packed, results_end;
   int stride, code_stride, bc_stride;
   size_t region_words;  // bounded-region workspace per lane (0: the grammar has none)
 };
@@ -2047,25 +2060,34 @@ EvalPlan plan_eval(const gagp_grammar* g, const gagp_cases* c, int rows) {
   const int E = g->expression_count, C = c->case_count;
   const size_t R = size_t(std::max(1, rows)), S = size_t(p.stride);
   auto& L = p.L;
+  // downloaded with one copy: the results and the device's error word
+  p.fitness = L.take(8 * R); p.wrong = L.take(4 * R); p.errors = L.take(4 * R); p.round = L.take(16);
+  p.results_end = L.total;
+  // uploaded with one copy, from the error word to the packed rows: the
+  // counters come zeroed with it
+  p.counters = L.take(8 * GAGP_COUNTERS); p.counts = L.take(4 * kRowCountWords);
   p.desc = L.take(sizeof(gb::SearchDesc));
   p.ex = L.take(sizeof(gagp_expression) * E);
-  p.info = L.take(sizeof(gb::ExprInfo) * E);
-  p.minimum = L.take(sizeof(uint32_t));
   p.local_types = L.take(sizeof(int32_t) * GAGP_MAX_LOCALS);
+  p.info = L.take(sizeof(gb::ExprInfo) * E);
   p.regions = L.take(sizeof(gb::RegionInfo) * size_t(std::max(1, g->region_count)));
   p.inputs = L.take(sizeof(int64_t) * size_t(std::max(1, c->input_count)) * C);
   p.expected = L.take(sizeof(int64_t) * C);
   p.lists = L.take(sizeof(int64_t) * size_t(std::max<int64_t>(1, c->list_values ? c->list_value_count : 0)));
+  p.off = L.take(8);
+  // the packed rows lie where the lowering writes the bytecode afterwards: a
+  // row's 10 bytes per node and 12 more against 20 bytes per bytecode word,
+  // of which a row has at least as many as it has nodes and at least 4
+  p.bc = L.take(20 * R * p.bc_stride);
+  p.packed = p.bc;
+  p.bc_len = L.take(4 * R); p.bc_locals = L.take(4 * R);
+  p.bc_consts = L.take(8 * R * p.bc_stride);
+  p.minimum = L.take(sizeof(uint32_t));
   p.node = L.take(8 * S * R); p.cval = L.take(8 * S * R); p.len = L.take(4 * R);
   p.code = L.take(8 * R * p.code_stride); p.code_len = L.take(4 * R); p.kpool = L.take(8 * R * S);
   p.code_temps = L.take(4 * R); p.vm_acc = L.take(16 * R);
-  p.bc = L.take(20 * R * p.bc_stride); p.bc_len = L.take(4 * R); p.bc_locals = L.take(4 * R);
-  p.bc_consts = L.take(8 * R * p.bc_stride);
-  p.fitness = L.take(8 * R); p.wrong = L.take(4 * R); p.errors = L.take(4 * R);
-  p.counters = L.take(8 * GAGP_COUNTERS); p.round = L.take(16);
   p.fast = L.take(sizeof(gb::ProgramRef) * R); p.exact = L.take(sizeof(gb::ProgramRef) * R);
   p.general = L.take(sizeof(gb::ProgramRef) * R);
-  p.counts = L.take(4 * kRowCountWords); p.off = L.take(8);
   p.region_words = 0;
   for (int r = 0; r < g->region_count; ++r)
     if (g->regions[r].traversal == 0)
@@ -2097,27 +2119,60 @@ gagp_status eval_check(const gagp_grammar* g, const gagp_cases* c, const gagp_se
     const int n = rows->node_counts[r], nc = rows->constant_counts[r];
     if (n < 1 || n > maxv || nc < 0 || nc > n || n > rows->stride)
       return fail(GAGP_INVALID_ARGUMENT, "row " + std::to_string(r) + " outside the node budget");
-    for (int i = 0; i < n; ++i) {
-      const int o = rows->origins[size_t(r) * rows->stride + i];
-      if (o < 0 || o >= g->expression_count) return fail(GAGP_INVALID_ARGUMENT, "row origin out of range");
-    }
+    const int32_t* o = rows->origins + size_t(r) * rows->stride;
+    uint32_t bad = 0;  // without an exit in the loop: vectorised
+    for (int i = 0; i < n; ++i) bad |= uint32_t(o[i]) >= uint32_t(g->expression_count);
+    if (bad) return fail(GAGP_INVALID_ARGUMENT, "row origin out of range");
   }
   return GAGP_OK;
+}
+
+// The staging bytes of one row evaluation: what is uploaded (the plan's
+// uploaded areas and the packed rows) and the results.
+struct EvalStaging {
+  size_t constants, starts, origins, packed_bytes;  // the packed rows' parts, from EvalPlan::packed
+  size_t up_bytes, bytes;
+};
+
+EvalStaging eval_staging(const EvalPlan& p, const gagp_rows* rows) {
+  size_t nodes = 0, constants = 0;
+  for (int r = 0; r < rows->count; ++r) {
+    nodes += size_t(rows->node_counts[r]);
+    constants += size_t(rows->constant_counts[r]);
+  }
+  EvalStaging s{};
+  s.constants = 0;
+  s.starts = 8 * constants;
+  s.origins = s.starts + 12 * size_t(rows->count);
+  s.packed_bytes = s.origins + 2 * nodes;
+  s.up_bytes = p.packed + s.packed_bytes - p.round;
+  s.bytes = std::max(s.up_bytes, p.results_end);
+  return s;
 }
 
 // Fills `region` (device, plan.L.total bytes) and evaluates every row on
 // `stream`; results are copied to the host arrays (`wrong` and `errors`, the
 // cases that ended in a runtime error, may be null).  No device allocation.
-gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g, const gagp_cases* c,
-                         const gagp_search_config* cfg, const gagp_rows* rows, double* fitness, uint32_t* wrong,
-                         uint32_t* errors, cudaStream_t stream, int sm_count, size_t max_smem) {
+// `staging` holds eval_staging().bytes host bytes, 16-byte aligned.
+// The rows go up packed -- 16-bit construction expressions and the constants
+// that exist, a sixth of the node words and constant slots they become -- and
+// one kernel unpacks them.  Host loops over node words, zeroed vectors, 16 MB
+// of pageable copies and an allocation per call took most of the 5.8 ms of
+// 16384 rows of 60 slots on 2000 cases (now 2.3 ms); 15 small copies and
+// memsets a third of the 153 us of 32 rows on 21 cases (now 105 us).
+gagp_status eval_rows_in(char* region, char* staging, const EvalStaging& sz, const EvalPlan& p, const gagp_grammar* g,
+                         const gagp_cases* c, const gagp_search_config* cfg, const gagp_rows* rows, double* fitness,
+                         uint32_t* wrong, uint32_t* errors, cudaStream_t stream, int sm_count, size_t max_smem) {
   const int E = g->expression_count, C = c->case_count, NI = c->input_count, R = rows->count;
   if (R == 0) return GAGP_OK;
   char* b = region;
-  std::vector<gb::ExprInfo> info(E);
+  auto host = [&](size_t off) { return staging + (off - p.round); };  // where the device's `off` is staged
+  std::memset(host(p.round), 0, p.desc - p.round);  // error word and counters
+  gb::ExprInfo* info = reinterpret_cast<gb::ExprInfo*>(host(p.info));
+  std::memcpy(host(p.ex), g->expressions, sizeof(gagp_expression) * E);
   for (int i = 0; i < E; ++i) {
     const gagp_expression& x = g->expressions[i];
-    gb::ExprInfo& f = info[i];
+    gb::ExprInfo f{};
     f.kind = int8_t(x.kind);
     f.node_kind = int8_t(x.node_kind);
     f.arity = int8_t(x.kind == gb::EK_REFERENCE ? 0 : x.arity);
@@ -2127,28 +2182,33 @@ gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g,
     f.target = x.target;
     f.site_nt = -1;
     f.site_class = -1;
+    info[i] = f;
   }
-  std::vector<int64_t> inputs(size_t(std::max(1, NI)) * C, 0);
+  int64_t* inputs = reinterpret_cast<int64_t*>(host(p.inputs));
   for (int j = 0; j < NI; ++j)
     for (int k = 0; k < C; ++k) inputs[size_t(j) * C + k] = c->inputs[size_t(k) * NI + j];
-  std::vector<int32_t> local_types(GAGP_MAX_LOCALS, GAGP_TAG_INVALID);
-  for (int j = 0; j < g->local_count; ++j) local_types[j] = g->local_types[j];
-  // rows as node words: evaluation reads the construction expression, arity
-  // and constant flag only
-  const size_t S = size_t(p.stride);
-  std::vector<uint64_t> node(S * R, 0);
-  std::vector<int64_t> cval(S * R, 0);
-  std::vector<int32_t> len(R);
-  for (int r = 0; r < R; ++r) {
-    const int n = rows->node_counts[r], nc = rows->constant_counts[r];
-    for (int i = 0; i < n; ++i) {
-      const int o = rows->origins[size_t(r) * rows->stride + i];
-      const gagp_expression& x = g->expressions[o];
-      node[S * r + i] = uint64_t(uint32_t(o)) | (uint64_t(uint32_t(x.arity) & 0xfu) << 48) |
-                        (uint64_t(x.kind == gb::EK_CONSTANT) << 52) | (uint64_t(gb::kNoClass) << 53);
+  std::memcpy(host(p.expected), c->expected, sizeof(int64_t) * C);
+  int32_t* local_types = reinterpret_cast<int32_t*>(host(p.local_types));
+  for (int j = 0; j < GAGP_MAX_LOCALS; ++j)
+    local_types[j] = j < g->local_count ? g->local_types[j] : int32_t(GAGP_TAG_INVALID);
+  const std::vector<gb::RegionInfo> regions = region_infos(g);
+  if (!regions.empty())
+    std::memcpy(host(p.regions), regions.data(), sizeof(gb::RegionInfo) * regions.size());
+  {
+    char* packed = host(p.packed);
+    int64_t* constants = reinterpret_cast<int64_t*>(packed + sz.constants);
+    gb::PackedRow* starts = reinterpret_cast<gb::PackedRow*>(packed + sz.starts);
+    uint16_t* origins = reinterpret_cast<uint16_t*>(packed + sz.origins);
+    uint32_t at_node = 0, at_constant = 0;
+    for (int r = 0; r < R; ++r) {
+      const int n = rows->node_counts[r], nc = rows->constant_counts[r];
+      const int32_t* o = rows->origins + size_t(r) * rows->stride;
+      starts[r] = gb::PackedRow{at_node, at_constant, int32_t(n | (nc << 16))};
+      for (int i = 0; i < n; ++i) origins[at_node + i] = uint16_t(o[i]);
+      if (nc) std::memcpy(constants + at_constant, rows->constants + size_t(r) * rows->stride, 8 * size_t(nc));
+      at_node += uint32_t(n);
+      at_constant += uint32_t(nc);
     }
-    for (int k = 0; k < nc; ++k) cval[S * r + k] = rows->constants[size_t(r) * rows->stride + k];
-    len[r] = n | (nc << 16);
   }
   gb::SearchDesc d{};
   d.ex = at<gagp_expression>(b, p.ex);
@@ -2204,25 +2264,13 @@ gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g,
   d.counters = at<uint64_t>(b, p.counters);
   d.round = at<int32_t>(b, p.round);
   const int32_t off[2] = {0, R};
-  auto up = [&](size_t at_off, const void* src, size_t bytes) {
-    return cudaMemcpyAsync(b + at_off, src, bytes, cudaMemcpyHostToDevice, stream);
-  };
-  CUDA_TRY(up(p.desc, &d, sizeof d));
-  CUDA_TRY(up(p.ex, g->expressions, sizeof(gagp_expression) * E));
-  CUDA_TRY(up(p.info, info.data(), sizeof(gb::ExprInfo) * E));
-  CUDA_TRY(up(p.local_types, local_types.data(), sizeof(int32_t) * GAGP_MAX_LOCALS));
-  const std::vector<gb::RegionInfo> regions = region_infos(g);
-  CUDA_TRY(up(p.regions, regions.data(), sizeof(gb::RegionInfo) * regions.size()));
-  CUDA_TRY(up(p.inputs, inputs.data(), sizeof(int64_t) * inputs.size()));
-  CUDA_TRY(up(p.expected, c->expected, sizeof(int64_t) * C));
-  if (n_lists) CUDA_TRY(up(p.lists, c->list_values, sizeof(int64_t) * size_t(n_lists)));
-  CUDA_TRY(up(p.node, node.data(), 8 * node.size()));
-  CUDA_TRY(up(p.cval, cval.data(), 8 * cval.size()));
-  CUDA_TRY(up(p.len, len.data(), 4 * len.size()));
-  CUDA_TRY(up(p.off, off, sizeof off));
-  CUDA_TRY(cudaMemsetAsync(b + p.counters, 0, 8 * GAGP_COUNTERS, stream));
-  CUDA_TRY(cudaMemsetAsync(b + p.round, 0, 16, stream));
-  CUDA_TRY(cudaMemsetAsync(b + p.counts, 0, 4 * kRowCountWords, stream));
+  std::memcpy(host(p.off), off, sizeof off);
+  std::memcpy(host(p.desc), &d, sizeof d);
+  if (n_lists) std::memcpy(host(p.lists), c->list_values, sizeof(int64_t) * size_t(n_lists));
+  CUDA_TRY(cudaMemcpyAsync(b + p.round, staging, sz.up_bytes, cudaMemcpyHostToDevice, stream));
+  gb::k_unpack_rows<<<blocks_for(size_t(R) * 32, 256), 256, 0, stream>>>(
+      at<gb::SearchDesc>(b, p.desc), at<int64_t>(b, p.packed + sz.constants),
+      at<gb::PackedRow>(b, p.packed + sz.starts), at<uint16_t>(b, p.packed + sz.origins));
   const gb::SearchDesc* dd = at<gb::SearchDesc>(b, p.desc);
   const int32_t* doff = at<int32_t>(b, p.off);
   gb::ProgramRef* fast = at<gb::ProgramRef>(b, p.fast);
@@ -2247,12 +2295,13 @@ gagp_status eval_rows_in(char* region, const EvalPlan& p, const gagp_grammar* g,
         dd, 0, lists.region, counts + 4, reinterpret_cast<unsigned long long*>(counts + 12), C, kRowRegionLanes,
         at<int64_t>(b, p.region_ws), p.region_words);
   CUDA_TRY(cudaGetLastError());
-  int32_t round[4];
-  CUDA_TRY(cudaMemcpyAsync(round, b + p.round, sizeof round, cudaMemcpyDeviceToHost, stream));
-  CUDA_TRY(cudaMemcpyAsync(fitness, b + p.fitness, 8 * size_t(R), cudaMemcpyDeviceToHost, stream));
-  if (wrong) CUDA_TRY(cudaMemcpyAsync(wrong, b + p.wrong, 4 * size_t(R), cudaMemcpyDeviceToHost, stream));
-  if (errors) CUDA_TRY(cudaMemcpyAsync(errors, b + p.errors, 4 * size_t(R), cudaMemcpyDeviceToHost, stream));
+  CUDA_TRY(cudaMemcpyAsync(staging, b, p.results_end, cudaMemcpyDeviceToHost, stream));
   CUDA_TRY(cudaStreamSynchronize(stream));
+  int32_t round[4];
+  std::memcpy(round, staging + p.round, sizeof round);
+  std::memcpy(fitness, staging + p.fitness, 8 * size_t(R));
+  if (wrong) std::memcpy(wrong, staging + p.wrong, 4 * size_t(R));
+  if (errors) std::memcpy(errors, staging + p.errors, 4 * size_t(R));
   if (round[3]) return fail(GAGP_DEVICE_ERROR, "row evaluation failed on the device (code " + std::to_string(round[3]) + ")");
   return GAGP_OK;
 }
@@ -2421,6 +2470,38 @@ static gagp_status batch_advance_body(gagp_engine* e, const int32_t* ids, int32_
   return st;
 }
 
+// Row evaluation in a block of the engine's pool with its pinned staging.
+// Past the two limits the block is allocated and freed for the call alone,
+// and the staging is pageable: the engine keeps no more than these for row
+// evaluation, and at that size an allocation is small next to the work.
+constexpr size_t kEvalPoolBytes = size_t(256) << 20, kEvalPinnedBytes = size_t(64) << 20;
+
+static gagp_status eval_rows_on(gagp_engine* e, const gagp_grammar* grammar, const gagp_cases* cases,
+                                const gagp_search_config* config, const gagp_rows* rows, double* fitness,
+                                uint32_t* wrong, uint32_t* errors) {
+  const EvalPlan p = plan_eval(grammar, cases, rows->count);
+  const EvalStaging sz = eval_staging(p, rows);
+  std::unique_ptr<char[]> pageable;
+  char* staging = nullptr;
+  if (sz.bytes <= kEvalPinnedBytes) {
+    if (const gagp_status st = pinned_at_least(e, sz.bytes); st != GAGP_OK) return st;
+    staging = e->pinned;
+  } else {
+    pageable.reset(new (std::nothrow) char[sz.bytes]);
+    if (!(staging = pageable.get())) return fail(GAGP_OUT_OF_MEMORY, "host staging of a row evaluation");
+  }
+  const bool pooled = p.L.total <= kEvalPoolBytes;
+  char* region = nullptr;
+  if (pooled) CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&region), p.L.total, e->pool, e->stream));
+  else CUDA_TRY(cudaMalloc(&region, p.L.total));
+  const gagp_status st = eval_rows_in(region, staging, sz, p, grammar, cases, config, rows, fitness, wrong, errors,
+                                      e->stream, e->sm_count, e->max_smem);
+  if (st != GAGP_OK) cudaStreamSynchronize(e->stream);  // the staging may still be read
+  if (pooled) cudaFreeAsync(region, e->stream);
+  else cudaFree(region);
+  return st;
+}
+
 // Entry points that launch work refuse a poisoned engine and poison it
 // after a device error that left a CUDA error pending, as search_run does.
 static gagp_status poison_after(gagp_engine* e, gagp_status st) {
@@ -2522,13 +2603,7 @@ gagp_status gagp_b200_evaluate_rows(gagp_engine* e, const gagp_grammar* grammar,
   gagp_status st = eval_check(grammar, cases, config, rows);
   if (st != GAGP_OK) return st;
   CUDA_TRY(cudaSetDevice(e->device));
-  const EvalPlan p = plan_eval(grammar, cases, rows->count);
-  char* region = nullptr;
-  CUDA_TRY(cudaMalloc(&region, p.L.total));
-  st = eval_rows_in(region, p, grammar, cases, config, rows, fitness, wrong, nullptr, e->stream, e->sm_count,
-                    e->max_smem);
-  cudaFree(region);
-  return st;
+  return eval_rows_on(e, grammar, cases, config, rows, fitness, wrong, nullptr);
 }
 
 gagp_status gagp_b200_judge_rows(gagp_engine* e, const gagp_grammar* grammar, const gagp_cases* cases,
@@ -2541,12 +2616,7 @@ gagp_status gagp_b200_judge_rows(gagp_engine* e, const gagp_grammar* grammar, co
   const int R = rows->count, C = cases->case_count;
   std::vector<double> fitness(size_t(std::max(1, R)));
   std::vector<uint32_t> wrong(size_t(std::max(1, R))), errors(size_t(std::max(1, R)));
-  const EvalPlan p = plan_eval(grammar, cases, R);
-  char* region = nullptr;
-  CUDA_TRY(cudaMalloc(&region, p.L.total));
-  st = eval_rows_in(region, p, grammar, cases, config, rows, fitness.data(), wrong.data(), errors.data(), e->stream,
-                    e->sm_count, e->max_smem);
-  cudaFree(region);
+  st = eval_rows_on(e, grammar, cases, config, rows, fitness.data(), wrong.data(), errors.data());
   if (st != GAGP_OK) return st;
   // run.cpp's judge_case from the fitness terms: a case is correct exactly
   // when it is not wrong; an Int-expected case whose value is not an Int is
@@ -2586,8 +2656,13 @@ gagp_status gagp_b200_evaluate_rows_static(const gagp_grammar* grammar, const ga
   CUDA_TRY(cudaGetDevice(&device));
   StaticDevice* d = nullptr;
   if ((st = static_scratch_on(device, &d)) != GAGP_OK) return st;
-  return eval_rows_in(d->scratch, p, grammar, cases, config, rows, fitness, wrong, nullptr,
-                      static_cast<cudaStream_t>(stream), d->sm_count, d->max_smem);
+  const EvalStaging sz = eval_staging(p, rows);
+  std::unique_ptr<char[]> staging(new (std::nothrow) char[sz.bytes]);
+  if (!staging) return fail(GAGP_OUT_OF_MEMORY, "host staging of a row evaluation");
+  st = eval_rows_in(d->scratch, staging.get(), sz, p, grammar, cases, config, rows, fitness, wrong, nullptr,
+                    static_cast<cudaStream_t>(stream), d->sm_count, d->max_smem);
+  if (st != GAGP_OK) cudaStreamSynchronize(static_cast<cudaStream_t>(stream));  // the staging may still be read
+  return st;
 }
 
 gagp_status gagp_b200_search_result(gagp_engine* e, int32_t id, gagp_search_result* out) {
@@ -2624,13 +2699,7 @@ gagp_status gagp_b200_search_result(gagp_engine* e, int32_t id, gagp_search_resu
                o_hl = L.take(4 * size_t(H)), o_fit = L.take(8 * size_t(P)), o_wr = L.take(4 * size_t(P)),
                o_nodes = L.take(4 * size_t(P)), o_nc = L.take(4 * size_t(P)), o_cc = L.take(4 * size_t(P)),
                o_org = L.take(4 * size_t(P) * W), o_con = L.take(8 * size_t(P) * W), o_cnt = L.take(8 * 4);
-  if (L.total > e->pinned_bytes) {
-    if (e->pinned) cudaFreeHost(e->pinned);
-    e->pinned = nullptr;
-    e->pinned_bytes = 0;
-    CUDA_TRY(cudaMallocHost(reinterpret_cast<void**>(&e->pinned), L.total));
-    e->pinned_bytes = L.total;
-  }
+  if (const gagp_status st = pinned_at_least(e, L.total); st != GAGP_OK) return st;
   char* hb = e->pinned;
   auto fetch = [&](size_t off, const void* src, size_t bytes) -> cudaError_t {
     e->d2h_bytes += bytes;

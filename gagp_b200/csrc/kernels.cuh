@@ -1697,6 +1697,34 @@ __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThr
   }
 }
 
+// ------------------------------------------------------------ row evaluation
+struct PackedRow {
+  uint32_t node, constant;  // the row's first construction expression and constant
+  int32_t len;              // its node and constant counts, as make_len packs them
+};
+static_assert(sizeof(PackedRow) == 12, "packed rows are uploaded as 12 bytes each");
+
+// The packed rows of a row evaluation as node words, constants and lengths,
+// a warp per row: evaluation reads the construction expression, the arity and
+// the constant flag only.  Bound by the launch at a few rows and by the 16
+// bytes written per node at many.
+__global__ void k_unpack_rows(const SearchDesc* desc, const int64_t* __restrict__ constants,
+                              const PackedRow* __restrict__ rows, const uint16_t* __restrict__ origins) {
+  const int r = int((size_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  const SearchDesc& s = *desc;
+  if (r >= s.P) return;
+  const PackedRow row = rows[r];
+  const int n = len_nodes(row.len), nc = len_consts(row.len);
+  const gagp_expression* __restrict__ ex = s.ex;
+  for (int i = lane; i < n; i += 32) {
+    const int o = origins[row.node + i];
+    s.node[size_t(r) * s.stride + i] = uint64_t(uint32_t(o)) | (uint64_t(uint32_t(ex[o].arity) & 0xfu) << 48) |
+                                       (uint64_t(ex[o].kind == EK_CONSTANT) << 52) | (uint64_t(kNoClass) << 53);
+  }
+  for (int k = lane; k < nc; k += 32) s.cval[size_t(r) * s.stride + k] = constants[row.constant + k];
+  if (lane == 0) s.len[r] = row.len;
+}
+
 // ------------------------------------------------------------ result export
 // The final population ranked as the reference ranks it (by ranking key,
 // ties by member index, selection.cpp:10-20): a member's rank is the number

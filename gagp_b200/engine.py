@@ -219,7 +219,7 @@ class Engine:
         cfg = task.settings.struct()
         out = (abi.Verdict * max(1, rows.count))()
         _check(load_library().gagp_b200_judge_rows(self.handle, g.ref(), cases.ref(), C.byref(cfg), rows.ref(), out))
-        return [out[i].summary() for i in range(rows.count)]
+        return abi.verdict_summaries(out, rows.count)
 
     def judge_best(self, task: LoadedTask, result: dict) -> dict:
         """The judgement of a search result's best program on the task's test
