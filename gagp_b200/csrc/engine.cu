@@ -1727,7 +1727,7 @@ gagp_status launch_vm_fast(gagp_engine* e, const BatchView& v, int mode, cudaStr
                            const int32_t* counts, const VmPlan& plan) {
   const int warps = 8;
   const int temp_stride = gb::kMaxTemps * plan.lanes * 32;
-  const int code_stride = (v.max_code_stride + 1) & ~1;  // uint2 slots, in int64 units
+  const int code_stride = ((v.max_code_stride + 1) & ~1) + 2;  // uint2 slots and two end words, in int64 units
   const int const_stride = v.max_stride;
   const size_t smem = size_t(warps) * (temp_stride + code_stride + const_stride) * sizeof(int64_t);
   // persistent: as many blocks as fit on every SM at once
@@ -2283,7 +2283,7 @@ gagp_status eval_rows_in(char* region, char* staging, const EvalStaging& sz, con
   const int warps = 8;
   const int lanes = d.vm_cases_per_lane;
   const int temp_stride = gb::kMaxTemps * lanes * 32;
-  const int code_stride = (p.code_stride + 1) & ~1;
+  const int code_stride = ((p.code_stride + 1) & ~1) + 2;  // and two end words
   const size_t smem = size_t(warps) * (temp_stride + code_stride + p.stride) * sizeof(int64_t);
   if (smem > max_smem - 1024) return fail(GAGP_DECLINED, "program too long for the VM's shared memory");
   const int per_sm = std::max(1, std::min(4, int((max_smem - 1024) / smem)));

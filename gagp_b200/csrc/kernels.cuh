@@ -11,7 +11,7 @@
 #include <cooperative_groups.h>
 
 #include "operators.cuh"
-#include "vm.cuh"
+#include "accumulator.cuh"
 #include "exact.cuh"
 
 namespace gb {
@@ -409,51 +409,75 @@ __global__ void __launch_bounds__(kRegionThreads) k_vm_region(const SearchDesc* 
 
 // Fast VM: persistent warps over the fast list.  Per warp shared memory:
 // temporaries (kMaxTemps x K x 32), the staged code (code_stride) and
-// constants (stride).
-template <int K>
-__device__ __forceinline__ void run_k(const SearchDesc& s, int slot, const VmWarpSmem& w, int case_begin,
-                                      int case_end, int64_t& loss, uint32_t& wrong, uint64_t& ops) {
-  switch (s.n_inputs) {
-    case 1: run_accumulator<K, 1>(s, slot, w, case_begin, case_end, loss, wrong, ops); break;
-    case 2: run_accumulator<K, 2>(s, slot, w, case_begin, case_end, loss, wrong, ops); break;
-    default: run_accumulator<K, 0>(s, slot, w, case_begin, case_end, loss, wrong, ops); break;
-  }
+// constants (stride).  Work items are (program, group of tiles of 32 K
+// cases), program-major, so that a round with fewer programs than resident
+// warps still fills the GPU; a group's tiles share the staging of the
+// program, and groups grow while every warp keeps kVmItems items.  Each group
+// adds its loss and wrong count to the program's accumulators and the last to
+// finish stores the program's result (integer sums: the order does not
+// matter).
+// (Items a warp: 16384 programs on 2000 cases, a whole call: 8 1.54 ms, a warp
+// of long programs runs on alone; 16 1.44; 32 1.46, every tile staged anew.)
+constexpr int kVmItems = 16;
+template <int K, int NIN>
+__device__ __forceinline__ void run_group(const SearchDesc& s, int slot, const VmWarpSmem& w, const uint8_t* entries,
+                                          int len, int case_begin, int case_end, int64_t& loss, uint32_t& wrong) {
+  stage_program<K, NIN>(s, slot, w, entries, len);
+  for (uint32_t c = case_begin; c < uint32_t(case_end); c += 32 * K)
+    run_accumulator<K, NIN>(s, w, c, min(uint32_t(case_end), c + 32 * K), loss, wrong);
 }
 // One instantiation per cases-per-lane K (each with its own register
-// budget); the engine's autotuner picks K per batch shape.  Work items are
-// (program, tile of 32 K cases), program-major, so that a round with fewer
-// programs than resident warps still fills the GPU; each tile adds its loss
-// and wrong count to the program's accumulators and the last tile to finish
-// stores the program's result (integer sums: the order does not matter).
+// budget); the engine's autotuner picks K per batch shape.
 template <int K>
-__global__ void __launch_bounds__(256, K == 4 ? 2 : 4) k_vm_fast(const SearchDesc* descs, int mode, const ProgramRef* list,
+__global__ void __launch_bounds__(256, K == 4 ? 3 : 4) k_vm_fast(const SearchDesc* descs, int mode, const ProgramRef* list,
                                                  const int32_t* list_count, int temp_stride, int code_stride,
                                                  int const_stride, int tiles_max) {
   extern __shared__ __align__(16) int64_t smem_vm[];
+  __shared__ uint8_t entries[kStageEntries];
+  if (threadIdx.x < kStageEntries) entries[threadIdx.x] = uint8_t(stage_entry(threadIdx.x));
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int warps = blockDim.x >> 5;
   const size_t per_warp = size_t(temp_stride) + size_t(code_stride) + size_t(const_stride);  // int64 units
   int64_t* base = smem_vm + size_t(warp) * per_warp;
   const VmWarpSmem w{base, reinterpret_cast<uint2*>(base + temp_stride), base + temp_stride + code_stride};
-  const long long items = (long long)(*list_count) * tiles_max;
-  for (long long item = (long long)blockIdx.x * warps + warp; item < items; item += (long long)gridDim.x * warps) {
-    const ProgramRef p = list[item / tiles_max];
-    const int case0 = int(item % tiles_max) * 32 * K;
+  const long long count = *list_count, step = (long long)gridDim.x * warps;
+  const int group = int(max(1LL, min((long long)tiles_max, count * tiles_max / (kVmItems * step))));  // tiles
+  const int groups = (tiles_max + group - 1) / group;
+  const long long cases = (long long)group * (32 * K);
+  // the warp's items, first and then every `step` further on: program and
+  // group counted along, for a 64-bit division per item cost more than staging
+  const long long first = (long long)blockIdx.x * warps + warp;
+  long long program = first / groups;
+  int g = int(first % groups);
+  const long long program_step = step / groups;
+  const int g_step = int(step % groups);
+  for (; program < count; program += program_step, g += g_step) {
+    if (g >= groups) {
+      g -= groups;
+      if (++program >= count) break;
+    }
+    const ProgramRef p = list[program];
+    const long long case0 = g * cases;
     const SearchDesc& s = descs[p.search];
     if (case0 >= s.C) continue;
+    const int case1 = int(min((long long)s.C, case0 + cases));
+    const int len = s.code_len[p.slot];
     int64_t loss = 0;
     uint32_t wrong = 0;
-    uint64_t ops = 0;
-    run_k<K>(s, p.slot, w, case0, min(s.C, case0 + 32 * K), loss, wrong, ops);
+    switch (s.n_inputs) {
+      case 1: run_group<K, 1>(s, p.slot, w, entries, len, int(case0), case1, loss, wrong); break;
+      case 2: run_group<K, 2>(s, p.slot, w, entries, len, int(case0), case1, loss, wrong); break;
+      default: run_group<K, 0>(s, p.slot, w, entries, len, int(case0), case1, loss, wrong); break;
+    }
     loss = warp_sum(loss);
     wrong = warp_sum(wrong);
     if (lane == 0) {
-      const unsigned tiles = unsigned((s.C + 32 * K - 1) / (32 * K));
       // accumulator programs never fail; the program's instructions over all
       // its cases are counted once
-      if (add_tile_result(s, mode, p.slot, tiles, loss, wrong, 0))
+      if (add_tile_result(s, mode, p.slot, unsigned((s.C + cases - 1) / cases), loss, wrong, 0))
         atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[3]),
-                  (unsigned long long)s.code_len[p.slot] * (unsigned long long)s.C);
+                  (unsigned long long)len * (unsigned long long)s.C);
     }
   }
 }
