@@ -1724,7 +1724,7 @@ VmPlan plan_vm(gagp_engine* e, const BatchView& v, bool may_measure) {
 }
 
 gagp_status launch_vm_fast(gagp_engine* e, const BatchView& v, int mode, cudaStream_t stream, const gb::ProgramRef* fast,
-                           const int32_t* counts, const VmPlan& plan) {
+                           const int32_t* counts, const VmPlan& plan, int share = 1) {  // of the GPU: one part in `share`
   const int warps = 8;
   const int temp_stride = gb::kMaxTemps * plan.lanes * 32;
   const int code_stride = ((v.max_code_stride + 1) & ~1) + 2;  // uint2 slots and two end words, in int64 units
@@ -1736,7 +1736,7 @@ gagp_status launch_vm_fast(gagp_engine* e, const BatchView& v, int mode, cudaStr
                           : plan.lanes == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gb::k_vm_fast<2>, warps * 32, smem)
                                             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gb::k_vm_fast<4>, warps * 32, smem);
   if (occ != cudaSuccess) return fail(GAGP_DEVICE_ERROR, std::string("VM occupancy: ") + cudaGetErrorString(occ));
-  const int blocks = e->sm_count * std::max(1, per_sm);
+  const int blocks = std::max(1, e->sm_count * std::max(1, per_sm) / share);
   cudaEvent_t mark_start = nullptr, mark_stop = nullptr;
   if (plan.measure_key) {
     mark_start = take_event(e);
@@ -1874,7 +1874,13 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
                    v.exact_possible);
     }
     if (!shared_fast)
-      if (const gagp_status st2 = launch_vm_fast(e, v, 1, st, e->d_fast + lo, counts, vm); st2 != GAGP_OK) return st2;
+      // a quarter of the GPU per range: a grid that fills it would keep the
+      // other ranges' lowering blocks waiting for the first range's VM (a
+      // large scalar search 308 / 263 us per round with the whole, 295 / 252
+      // with a half or a quarter, 305 / 258 with an eighth)
+      if (const gagp_status st2 = launch_vm_fast(e, v, 1, st, e->d_fast + lo, counts, vm, chunks == 1 ? 1 : chunks / 2);
+          st2 != GAGP_OK)
+        return st2;
     if (chunks > 1) {
       CUDA_TRY(cudaEventRecord(e->chunk_done[c], st));
       CUDA_TRY(cudaStreamWaitEvent(e->stream, e->chunk_done[c], 0));
@@ -1975,7 +1981,8 @@ gagp_status capture_round(gagp_engine* e, const BatchView& v, RoundGraph* out) {
     return st;
   }
   if (ended != cudaSuccess) return fail(GAGP_DEVICE_ERROR, std::string("round capture: ") + cudaGetErrorString(ended));
-  const cudaError_t made = cudaGraphInstantiate(&out->exec, graph, 0);
+  // (the kernels keep the priorities of the streams they were captured from)
+  const cudaError_t made = cudaGraphInstantiate(&out->exec, graph, cudaGraphInstantiateFlagUseNodePriority);
   cudaGraphDestroy(graph);
   if (made != cudaSuccess) return fail(GAGP_DEVICE_ERROR, std::string("round graph: ") + cudaGetErrorString(made));
   return GAGP_OK;
