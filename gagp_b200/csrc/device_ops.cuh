@@ -61,17 +61,30 @@ struct SmallRange {
   }
 };
 
+__device__ __forceinline__ uint64_t splitmix_next(uint64_t& state) {
+  uint64_t v = (state += 0x9e3779b97f4a7c15ULL);
+  v = (v ^ (v >> 30)) * 0xbf58476d1ce4e5b9ULL;
+  v = (v ^ (v >> 27)) * 0x94d049bb133111ebULL;
+  return v ^ (v >> 31);
+}
+// A draw below `upper` past 2^16, out of line: two 64-bit divisions.
+struct Drawn {
+  uint64_t value, state;
+};
+__device__ __noinline__ Drawn draw_wide(uint64_t state, uint64_t upper) {
+  const uint64_t threshold = (0 - upper) % upper;
+  for (;;) {
+    const uint64_t v = splitmix_next(state);
+    if (v >= threshold) return Drawn{v % upper, state};
+  }
+}
+
 // SplitMix64 stream with rejection-sampled bounds
 // (DGrammarRandom, cpp/src/evolution/repro/gpu/device/grammar_random.cuh:10-51).
 struct Rng {
   uint64_t state;
   __device__ explicit Rng(uint64_t seed) : state(seed) {}
-  __device__ __forceinline__ uint64_t next() {
-    uint64_t v = (state += 0x9e3779b97f4a7c15ULL);
-    v = (v ^ (v >> 30)) * 0xbf58476d1ce4e5b9ULL;
-    v = (v ^ (v >> 27)) * 0x94d049bb133111ebULL;
-    return v ^ (v >> 31);
-  }
+  __device__ __forceinline__ uint64_t next() { return splitmix_next(state); }
   // 32-bit arithmetic only, with no table load on the dependent chain; only a
   // draw below 2^16 can be below the rejection bound
   __device__ __forceinline__ uint32_t bounded(const SmallRange& r) {
@@ -83,11 +96,9 @@ struct Rng {
   }
   __device__ __forceinline__ uint64_t bounded(uint64_t upper) {
     if (upper - 1 < uint64_t(kSmallBound)) return bounded(SmallRange(uint32_t(upper)));
-    const uint64_t threshold = (0 - upper) % upper;
-    for (;;) {
-      const uint64_t v = next();
-      if (v >= threshold) return v % upper;
-    }
+    const Drawn d = draw_wide(state, upper);
+    state = d.state;
+    return d.value;
   }
   __device__ __forceinline__ int64_t integer(int64_t lo, int64_t hi) {
     const uint64_t sign = 1ULL << 63;
@@ -526,37 +537,48 @@ __device__ __forceinline__ int choose_site(const SiteSet& sites, Rng& random) {
 // choose_site (phase_operators.cuh:55-83 and the counted warp variant
 // :95-117): the same count, draws and prefix-ordered rank; reservoir draws
 // visit matching sites in prefix order.  Every lane returns the same site.
-__device__ inline int warp_choose_site(const SRow& t, Rng& random, bool counted, uint32_t cls) {
+// Out of line (a row of more than 64 nodes, or reservoir draws); returns the
+// site (Drawn::value, -1 for none) and the stream's state.
+__device__ __noinline__ Drawn choose_site_of(const uint64_t* node, int n, uint64_t state, bool counted, uint32_t cls) {
   const int lane = lane_id();
+  Rng random(state);
   if (counted) {
     unsigned count = 0;
-    for (int chunk = 0; chunk < t.n; chunk += 32) {
+#pragma unroll 1
+    for (int chunk = 0; chunk < n; chunk += 32) {
       const int i = chunk + lane;
-      count += __popc(__ballot_sync(kFull, i < t.n && site_matches(t.node[i], cls)));
+      count += __popc(__ballot_sync(kFull, i < n && site_matches(node[i], cls)));
     }
-    if (!count) return -1;
+    if (!count) return Drawn{~0ULL, random.state};
     unsigned rank = unsigned(random.bounded(count));
-    for (int chunk = 0; chunk < t.n; chunk += 32) {
+#pragma unroll 1
+    for (int chunk = 0; chunk < n; chunk += 32) {
       const int i = chunk + lane;
-      const unsigned mask = __ballot_sync(kFull, i < t.n && site_matches(t.node[i], cls));
+      const unsigned mask = __ballot_sync(kFull, i < n && site_matches(node[i], cls));
       const unsigned c = __popc(mask);
-      if (rank < c) return chunk + warp_nth_bit(mask, rank);
+      if (rank < c) return Drawn{uint64_t(chunk + warp_nth_bit(mask, rank)), random.state};
       rank -= c;
     }
-    return -1;
+    return Drawn{~0ULL, random.state};
   }
   int selected = -1;
   unsigned count = 0;
-  for (int chunk = 0; chunk < t.n; chunk += 32) {
+#pragma unroll 1
+  for (int chunk = 0; chunk < n; chunk += 32) {
     const int i = chunk + lane;
-    unsigned mask = __ballot_sync(kFull, i < t.n && site_matches(t.node[i], cls));
+    unsigned mask = __ballot_sync(kFull, i < n && site_matches(node[i], cls));
     while (mask) {
       const int bit = __ffs(mask) - 1;
       mask &= mask - 1;
       if (random.bounded(++count) == 0) selected = chunk + bit;
     }
   }
-  return selected;
+  return Drawn{uint64_t(int64_t(selected)), random.state};
+}
+__device__ __forceinline__ int warp_choose_site(const SRow& t, Rng& random, bool counted, uint32_t cls) {
+  const Drawn d = choose_site_of(t.node, t.n, random.state, counted, cls);
+  random.state = d.state;
+  return int(int64_t(d.value));
 }
 
 // phase_subtree_end (device/phase_variation.cuh:81-91, warp form :213-229).
@@ -565,6 +587,7 @@ __device__ inline int warp_subtree_end(const SRow& t, int start) {
   // than its root
   if (start < 0 || start >= t.n) return -1;
   const int lane = lane_id(), depth = w_depth(t.node[start]);
+#pragma unroll 1
   for (int chunk = start + 1; chunk < t.n; chunk += 32) {
     const int i = chunk + lane;
     const unsigned hit = __ballot_sync(kFull, i < t.n && w_depth(t.node[i]) <= depth);
@@ -576,6 +599,7 @@ __device__ inline int warp_subtree_end(const SRow& t, int start) {
 // Constant nodes among row positions [0, first) and [0, second), first <= second.
 __device__ __forceinline__ void warp_count_constants2(const SRow& t, int first, int second, int* a, int* b) {
   int ca = 0, cb = 0;
+#pragma unroll 1
   for (int chunk = 0; chunk < second; chunk += 32) {
     const int i = chunk + lane_id();
     const bool c = i < second && w_const(t.node[i]);
@@ -610,18 +634,21 @@ __device__ inline GenResult warp_splice(const SRow& base, bool base_within, int 
   if (length > stride) { r.status = ST_CAPACITY; return r; }  // never reached: callers bound by the node budget
   const int ddepth = w_depth(a) - w_depth(b), dsval = w_sval(a) - w_sval(b);
   int maxd = 0, maxs = 0;
+#pragma unroll 1
   for (int i = src + lane_id(); i < donor_end; i += 32) {
     const uint64_t w = w_shift(donor.node[i], ddepth, dsval);
     maxd = max(maxd, w_depth(w));
     maxs = max(maxs, w_sval(w));
   }
   if (!base_within)
+#pragma unroll 1
     for (int i = lane_id(); i < base.n; i += 32)
       if (i < dest || i >= end) {
         maxd = max(maxd, w_depth(base.node[i]));
         maxs = max(maxs, w_sval(base.node[i]));
       }
   if (__any_sync(kFull, maxd > max_depth || (site_limit && maxs > site_limit))) { r.status = ST_CAPACITY; return r; }
+#pragma unroll 1
   for (int i = lane_id(); i < length; i += 32) {
     uint64_t w;
     if (i >= dest && i < dest + inserted) {
@@ -636,8 +663,11 @@ __device__ inline GenResult warp_splice(const SRow& base, bool base_within, int 
   warp_count_constants2(base, dest, end, &bb, &be);
   warp_count_constants2(donor, src, donor_end, &db, &de);
   const int dc = de - db;
+#pragma unroll 1
   for (int k = lane_id(); k < bb; k += 32) out.cval[k] = base.cval[k];
+#pragma unroll 1
   for (int k = lane_id(); k < dc; k += 32) out.cval[bb + k] = donor.cval[db + k];
+#pragma unroll 1
   for (int k = lane_id(); k < base.nc - be; k += 32) out.cval[bb + dc + k] = base.cval[be + k];
   __syncwarp();
   r.status = ST_OK;

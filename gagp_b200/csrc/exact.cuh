@@ -177,6 +177,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   {
     const bool unit = s.unit_fuel;
     uint32_t open = 1, fuel = 0, seen = 0;
+#pragma unroll 1
     for (int base = 0; base < n; base += 32) {
       const int i = base + lane;
       uint32_t charge = 0;
@@ -299,11 +300,13 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
     const_count = __shfl_sync(kFull, const_count, 0);
   }
   // ---- subtree ends (as in lower_accumulator_emit) and parents
+#pragma unroll 1
   for (int base = 0; base < n; base += 32) {
     const int i = base + lane;
     const int r = i < n ? m.start[i] : 0;
     int e = n;
     bool found = i >= n;
+#pragma unroll 1
     for (int cb = base; cb < n && __any_sync(kFull, !found); cb += 32) {
       const int j = cb + lane;
       const int open = j < n ? m.start[j] : 0x7fffffff;
@@ -322,6 +325,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   if (m.end[0] != n) return -1;
   {
     int rank = 0;
+#pragma unroll 1
     for (int base = 0; base < n; base += 32) {
       const int i = base + lane;
       const bool is_const = i < n && m.kind[i] == N_CONST;
@@ -357,6 +361,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   };
   // ---- bound reads: the nearest traversal body (element, index or state)
   // or let body around the node that binds its number
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     if (m.kind[i] != N_BOUND) continue;
     const int b = m.aux[i];
@@ -378,6 +383,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   __syncwarp();
   // their types: the traversal's binding, or the let's value (a let's value
   // may itself be read through another let, so outer ones come first)
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     if (m.kind[i] != N_BOUND) continue;
     int x = i, t = GAGP_TAG_INVALID;
@@ -401,6 +407,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   // both branches)
   {
     uint32_t not_flat = 0;
+#pragma unroll 1
     for (int base = 0; base < n; base += 32) {
       const int i = base + lane;
       bool flat = true;
@@ -465,6 +472,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   uint32_t kept = 0;
   {
     uint32_t assigned = 0, read = 0;
+#pragma unroll 1
     for (int i = lane; i < n; i += 32) {
       const uint8_t kind = m.kind[i];
       if ((kind == N_ASSIGN || kind == N_FOR) && m.aux[i] < n_inputs) assigned |= 1u << m.aux[i];
@@ -476,6 +484,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   }
   auto kept_length = [&](int i) -> bool { return m.kind[i] == N_SLOT && m.aux[i] < n_inputs && (kept >> m.aux[i] & 1u); };
   __syncwarp();
+#pragma unroll 1
   for (int i = lane; i < n; i += 32)
     if (m.kind[i] == N_OP1 && m.aux[i] == X_LEN && kept_length(i + 1)) m.kind[i] = N_LEN;
   // a search's rows are definitely assigned: generation, crossover, mutation
@@ -496,6 +505,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
     return end;
   };
   // ---- fused comparisons and selects
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     if (m.kind[i] != N_IF) continue;
     const int c0 = i + 1, c1 = m.end[c0], end = m.end[i];
@@ -510,6 +520,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
     m.flags[i] |= uint8_t(NF_SELECT | (next_if(c1, end) < end ? NF_PICK : 0));
   }
   __syncwarp();
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     bool inside = false;
     for (int x = i; x > 0 && !inside; x = m.par[x]) inside = m.kind[m.par[x]] == N_IF && (m.flags[m.par[x]] & NF_SELECT);
@@ -519,6 +530,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   auto alias = [&](int i) -> bool { return m.mark[i] & NM_ALIAS; };
   // ---- words
   uint32_t total_words = 0;
+#pragma unroll 1
   for (int base = 0; base < n; base += 32) {
     const int i = base + lane;
     uint32_t own = 0;
@@ -551,14 +563,17 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   if (lane == 0) m.words[n] = int16_t(min(total_words, 32767u));
   const int count = int(total_words) + 1;  // and the appended RETURN, or the end of a statement program
   if (count > kExactWords || count + 2 > word_cap) return -1;
+#pragma unroll 1
   for (int k = lane; k < count; k += 32) m.cw[k] = 0;
   __syncwarp();
+#pragma unroll 1
   for (int i = lane; i < n; i += 32)
     if (m.kind[i] == N_BOUND && m.kind[m.aux[i]] == N_TRAVERSE && (m.flags[i] >> 6) == 1) m.mark[m.aux[i]] |= NM_INDEX;
   __syncwarp();
   auto size = [&](int i) { return m.words[m.end[i]] - m.words[i]; };
   // ---- first words and temporaries: offsets from the parent, then sums
   // along the path from the root
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     if (i == 0) { m.start[0] = 0; m.pos[0] = 0; }
     const int a = w_arity(node[i]);
@@ -593,6 +608,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   }
   __syncwarp();
   int top = 0;  // slots in use
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     int at = 0, held = 0, depth = 0;
     for (int x = i; x > 0; x = m.par[x]) {
@@ -627,6 +643,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
     const int which = m.flags[i] >> 6;  // of a traversal: 0 element, 1 index, 2 state
     return uint32_t(base_slot + m.slot[aux] + (m.kind[aux] == N_LET || which == 2 ? 0 : 3 + which));
   };
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) m.pos[i] = uint8_t(alias(i) ? leaf_slot(i) : uint32_t(base_slot + m.slot[i]));
   __syncwarp();
   auto operand = [&](int i) -> uint32_t { return m.pos[i]; };
@@ -673,6 +690,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
     atomicAdd(&m.cw[k], cost + (exact_control(op) ? 1u << 31 : 0u));
   };
   int rank = 0;
+#pragma unroll 1
   for (int base = 0; base < n; base += 32) {
     const int i = base + lane;
     const bool live = i < n;

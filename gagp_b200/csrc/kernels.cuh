@@ -748,7 +748,13 @@ __global__ void __launch_bounds__(256) k_member_index(const SearchDesc* descs, c
 // block first copies that search's generator image (image_bytes) into
 // shared memory after the rows: a generation step is a chain of dependent
 // table lookups, each a shared-memory load instead of a global one.
-__global__ void __launch_bounds__(128, 6) k_vary(const SearchDesc* descs, const int32_t* off, int n, int stride_max,
+// Bound by latency, of instruction fetches first: its warps are each somewhere
+// else in 130 KB of code (4.7 of the 12 cycles an instruction waits, with 24
+// warps an SM), so loops over a row's nodes are not unrolled and rare draws
+// are out of line (174 KB before).  Five blocks an SM and 96 registers: six
+// spill 200 bytes a thread, four are no faster (large scalar search 274 / 250
+// us per round, generational 165 / 176; six 273 / 247 and 173 / 186).
+__global__ void __launch_bounds__(128, 5) k_vary(const SearchDesc* descs, const int32_t* off, int n, int stride_max,
                                                  int32_t* next_item, int lo, int hi, int collect_stats, int staged,
                                                  int image_bytes) {
   extern __shared__ __align__(16) char smem_rows[];

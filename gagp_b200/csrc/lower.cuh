@@ -734,6 +734,7 @@ __device__ inline int lower_accumulator_emit(LowerScratch& m, int n, uint2* code
   const int lane = threadIdx.x & 31;
   // open slots before node i: 1 + sum over earlier nodes of (arity - 1)
   int carry = 1;
+#pragma unroll 1
   for (int base = 0; base < n; base += 32) {
     const int i = base + lane;
     const int v = i < n ? int(m.arity[i]) - 1 : 0;
@@ -749,11 +750,13 @@ __device__ inline int lower_accumulator_emit(LowerScratch& m, int n, uint2* code
   // a subtree ends at the first later node with fewer open slots: for 32
   // nodes at a time, every lane holds one later node's slot count and each
   // node's question is answered by one ballot per chunk
+#pragma unroll 1
   for (int base = 0; base < n; base += 32) {
     const int i = base + lane;
     const int r = i < n ? m.start[i] : 0;
     int e = n;
     bool found = i >= n;
+#pragma unroll 1
     for (int cb = base; cb < n && __any_sync(kFull, !found); cb += 32) {
       const int j = cb + lane;
       const int slots = j < n ? m.start[j] : 0x7fffffff;
@@ -851,6 +854,7 @@ __device__ inline int lower_accumulator_emit(LowerScratch& m, int n, uint2* code
   // children's offsets from itself, then pointer jumping adds up the paths
   // in about log2(depth) rounds instead of one sweep per level.
   if (lane == 0) { m.start[0] = 0; m.temp_base[0] = 0; m.depth[0] = 1; m.anc[0] = -1; }
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     const int a = m.arity[i];
     if (!a) continue;
@@ -873,6 +877,7 @@ __device__ inline int lower_accumulator_emit(LowerScratch& m, int n, uint2* code
     }
   }
   __syncwarp();
+#pragma unroll 1
   for (int i = lane; i < n; i += 32)
     if (m.arity[i] && m.anc[i] == -2) fail = true;  // unreachable from the root
   if (__any_sync(kFull, fail)) return -1;
@@ -880,6 +885,7 @@ __device__ inline int lower_accumulator_emit(LowerScratch& m, int n, uint2* code
   // and a write step per node slot, so every read sees a consistent pair
   for (int round = 0; round < 10; ++round) {
     bool more = false;
+#pragma unroll 1
     for (int base = 0; base < n; base += 32) {
       const int i = base + lane;
       const bool live = i < n && m.arity[i] && m.anc[i] >= 0;
@@ -903,9 +909,11 @@ __device__ inline int lower_accumulator_emit(LowerScratch& m, int n, uint2* code
     }
     if (!__any_sync(kFull, more)) break;
   }
+#pragma unroll 1
   for (int i = lane; i < n; i += 32)
     if (m.arity[i] && m.anc[i] >= 0) fail = true;  // deeper than 2^10 levels: impossible for admitted rows
   // ---- every non-leaf node writes its spills and its own words
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) {
     const int a = m.arity[i];
     if (!a) continue;
@@ -1017,6 +1025,7 @@ __device__ inline int lower_accumulator_warp(const SearchDesc& s, const uint64_t
   const ExprInfo* __restrict__ info = s.info;
   bool total = true;
   int bytecode = 0, constants = 0;
+#pragma unroll 1
   for (int base = 0; base < n; base += 32) {
     const int i = base + lane;
     const uint64_t w = i < n ? node[i] : 0;
@@ -1043,6 +1052,7 @@ __device__ inline int lower_accumulator_warp(const SearchDesc& s, const uint64_t
     }
     constants += __popc(const_mask);
   }
+#pragma unroll 1
   for (int k = lane; k < nc; k += 32) kpool[k] = cval[k];
   total = __all_sync(kFull, total);
   for (int o = 16; o; o >>= 1) bytecode += __shfl_xor_sync(kFull, bytecode, o);

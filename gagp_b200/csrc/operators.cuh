@@ -55,10 +55,23 @@ __device__ inline void warp_tournaments(const SearchDesc& s, Rng& random, int* p
     // a segmented shuffle reduction, then each winner from its lane
     int seg = 1;
     while (seg < p) seg <<= 1;
-    int mine = 0;
-    for (int j = 0; j < total; ++j) {
-      const int d = int(random.bounded_fixed(uint64_t(s.P), s.bounded_threshold, s.mod_magic));
-      if ((j < p ? j : seg + j - p) == lane) mine = d;
+    // draw j is a function of the counter j steps on, so the lanes take a
+    // draw each; only when one is rejected (a chance of P / 2^64) are they
+    // taken in order
+    const int draw = lane < seg ? lane : p + lane - seg;
+    Rng ahead(random.state + uint64_t(draw) * 0x9e3779b97f4a7c15ULL);
+    const uint64_t v = ahead.next();
+    uint64_t drawn = v - __umul64hi(v, s.mod_magic) * uint64_t(s.P);
+    while (drawn >= uint64_t(s.P)) drawn -= uint64_t(s.P);
+    int mine = int(drawn);
+    if (__any_sync(kFull, lane < 2 * seg && (lane < seg ? lane : lane - seg) < p && v < s.bounded_threshold)) {
+#pragma unroll 1
+      for (int j = 0; j < total; ++j) {
+        const int d = int(random.bounded_fixed(uint64_t(s.P), s.bounded_threshold, s.mod_magic));
+        if ((j < p ? j : seg + j - p) == lane) mine = d;
+      }
+    } else {
+      random.state += uint64_t(total) * 0x9e3779b97f4a7c15ULL;
     }
     const int position = lane < seg ? lane : lane - seg;
     const bool live = lane < 2 * seg && position < p;
@@ -81,9 +94,11 @@ __device__ inline void warp_tournaments(const SearchDesc& s, Rng& random, int* p
     return;
   }
   Entrant best[2] = {{0, 0, 0, false}, {0, 0, 0, false}};
+#pragma unroll 1
   for (int base = 0; base < total; base += 32) {
     const int n = min(32, total - base);
     int mine = 0;
+#pragma unroll 1
     for (int j = 0; j < n; ++j) {
       const int d = int(random.bounded_fixed(uint64_t(s.P), s.bounded_threshold, s.mod_magic));
       if (j == lane) mine = d;
@@ -133,6 +148,7 @@ __device__ inline void load_members(const SearchDesc& s, int a, SRow& to_a, int 
   const uint64_t* nb = s.node + size_t(b) * s.stride;
   const int64_t* ca = s.cval + size_t(a) * s.stride;
   const int64_t* cb = s.cval + size_t(b) * s.stride;
+#pragma unroll 2
   for (int i = lane_id(); i < s.stride; i += 32) {
     const uint64_t x = na[i], y = nb[i];
     const int64_t u = ca[i], v = cb[i];
@@ -157,7 +173,9 @@ __device__ inline void load_members(const SearchDesc& s, int a, SRow& to_a, int 
 __device__ inline uint64_t warp_row_hash(const uint64_t* node, const int64_t* cval, int n, int nc) {
   const int lane = lane_id();
   uint64_t acc = 0;
+#pragma unroll 1
   for (int i = lane; i < n; i += 32) acc += mix64(uint64_t(w_origin(node[i])) | (uint64_t(i) << 32));
+#pragma unroll 1
   for (int i = lane; i < nc; i += 32) acc += mix64(uint64_t(cval[i]) ^ mix64(0x5bd1e995ULL + uint64_t(i)));
 #pragma unroll
   for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
@@ -171,7 +189,9 @@ __device__ inline bool warp_rows_equal(const uint64_t* an, const int64_t* ac, in
                                        const int64_t* bc, int b_n, int b_nc) {
   if (a_n != b_n || a_nc != b_nc) return false;
   bool same = true;
+#pragma unroll 1
   for (int i = lane_id(); i < a_n; i += 32) same &= w_origin(an[i]) == w_origin(bn[i]);
+#pragma unroll 1
   for (int i = lane_id(); i < a_nc; i += 32) same &= ac[i] == bc[i];
   return __all_sync(kFull, same);
 }
@@ -255,6 +275,7 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bo
   // be deeper than the depth limit, and then every splice that keeps the deep
   // part is rejected)
   bool within = true;
+#pragma unroll 1
   for (int i = lane; i < w.parent.n; i += 32)
     within &= w_depth(w.parent.node[i]) <= s.slot_max_depth && (!s.site_depth || w_sval(w.parent.node[i]) <= s.site_depth);
   within = __all_sync(kFull, within);
@@ -354,8 +375,10 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bo
   if (s.generational && index < s.elite_count) {
     const int src = s.elites[index];
     const int32_t l = s.len[src];
+#pragma unroll 1
     for (int i = lane; i < len_nodes(l); i += 32)
       s.cnode[size_t(index) * s.stride + i] = s.node[size_t(src) * s.stride + i];
+#pragma unroll 1
     for (int i = lane; i < len_consts(l); i += 32)
       s.ccval[size_t(index) * s.stride + i] = s.cval[size_t(src) * s.stride + i];
     if (lane == 0) s.clen[index] = l;
@@ -366,13 +389,17 @@ __device__ inline int warp_vary_child(const SearchDesc& s, const char* image, bo
   bool equal = child.n == w.parent.n && child.nc == w.parent.nc;
   if (equal && (crossed || mutated)) {
     bool mine = true;
+#pragma unroll 1
     for (int i = lane; i < child.n; i += 32) mine &= w_origin(child.node[i]) == w_origin(w.parent.node[i]);
+#pragma unroll 1
     for (int i = lane; i < child.nc; i += 32) mine &= child.cval[i] == w.parent.cval[i];
     equal = __all_sync(kFull, mine);
   }
   if (equal) *reuse_out = parent;
   // ---- publish the child row
+#pragma unroll 1
   for (int i = lane; i < child.n; i += 32) s.cnode[size_t(index) * s.stride + i] = child.node[i];
+#pragma unroll 1
   for (int i = lane; i < child.nc; i += 32) s.ccval[size_t(index) * s.stride + i] = child.cval[i];
   if (lane == 0) s.clen[index] = make_len(child.n, child.nc);
   w.child.n = child.n;  // the caller's statistics
