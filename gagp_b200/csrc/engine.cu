@@ -86,6 +86,7 @@ struct gagp_engine {
   static constexpr int kChunks = 8;
   cudaStream_t chunk_stream[kChunks] = {};
   cudaEvent_t chunk_fork = nullptr, chunk_done[kChunks] = {};
+  cudaEvent_t vm_fork = nullptr, vm_done[2] = {};
   std::map<int, std::unique_ptr<Search>> searches;
   int next_id = 1;
   uint64_t arena_limit = 0, arena_used = 0;
@@ -1219,6 +1220,8 @@ gagp_status gagp_b200_engine_create(int32_t device, uint64_t arena_bytes, gagp_e
   CUDA_TRY(cudaEventCreateWithFlags(&e->join, cudaEventDisableTiming));
   CUDA_TRY(cudaEventCreateWithFlags(&e->indexed, cudaEventDisableTiming));
   CUDA_TRY(cudaEventCreateWithFlags(&e->chunk_fork, cudaEventDisableTiming));
+  for (cudaEvent_t* ev : {&e->vm_fork, &e->vm_done[0], &e->vm_done[1]})
+    CUDA_TRY(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
   for (int c = 0; c < gagp_engine::kChunks; ++c) {
     CUDA_TRY(cudaStreamCreateWithPriority(&e->chunk_stream[c], cudaStreamNonBlocking, greatest));
     CUDA_TRY(cudaEventCreateWithFlags(&e->chunk_done[c], cudaEventDisableTiming));
@@ -1277,6 +1280,8 @@ void gagp_b200_engine_destroy(gagp_engine* e) {
   if (e->join) cudaEventDestroy(e->join);
   if (e->indexed) cudaEventDestroy(e->indexed);
   if (e->chunk_fork) cudaEventDestroy(e->chunk_fork);
+  for (cudaEvent_t ev : {e->vm_fork, e->vm_done[0], e->vm_done[1]})
+    if (ev) cudaEventDestroy(ev);
   for (int c = 0; c < gagp_engine::kChunks; ++c) {
     if (e->chunk_stream[c]) cudaStreamDestroy(e->chunk_stream[c]);
     if (e->chunk_done[c]) cudaEventDestroy(e->chunk_done[c]);
@@ -1756,15 +1761,35 @@ gagp_status launch_vm_fast(gagp_engine* e, const BatchView& v, int mode, cudaStr
   return GAGP_OK;
 }
 
-// The exact VM and the bounded-region kernel over a round's shared lists
-// (nothing for a batch whose programs never need them).
-gagp_status launch_vm_exact(gagp_engine* e, const BatchView& v, int mode) {
-  if (v.exact_possible) {
+// The VMs over a round's shared lists, side by side -- their programs are
+// different ones: the accumulator VM (`fast`, null where the ranges ran it),
+// and for a batch whose programs may need them the exact VM and the
+// bounded-region kernel.  One after the other, the two with few or no
+// programs cost 5 to 7 us each.
+gagp_status launch_vms(gagp_engine* e, const BatchView& v, int mode, const VmPlan* fast) {
+  auto run_fast = [&](cudaStream_t st) {
+    return launch_vm_fast(e, v, mode, st, e->d_fast, e->d_counts + kSharedFast, *fast);
+  };
+  if (!v.exact_possible) return fast ? run_fast(e->stream) : GAGP_OK;
+  CUDA_TRY(cudaEventRecord(e->vm_fork, e->stream));
+  if (v.regions) {
+    CUDA_TRY(cudaStreamWaitEvent(e->chunk_stream[1], e->vm_fork, 0));
+    if (const gagp_status st = vm_region_launch(e, e->chunk_stream[1], v, mode); st != GAGP_OK) return st;
+    CUDA_TRY(cudaEventRecord(e->vm_done[1], e->chunk_stream[1]));
+  }
+  if (fast) {
+    CUDA_TRY(cudaStreamWaitEvent(e->chunk_stream[0], e->vm_fork, 0));
+    if (const gagp_status st = run_fast(e->chunk_stream[0]); st != GAGP_OK) return st;
+    CUDA_TRY(cudaEventRecord(e->vm_done[0], e->chunk_stream[0]));
+  }
+  {
     Timed t(e, KN_VM_EXACT);
     vm_exact_launch(e->sm_count, e->stream, v.d_desc, mode, engine_lists(e, e->d_fast, kSharedFast),
                     e->d_counts + kExactNext, v.max_C, v.exact_heavy);
   }
-  return v.regions ? vm_region_launch(e, e->stream, v, mode) : GAGP_OK;
+  if (fast) CUDA_TRY(cudaStreamWaitEvent(e->stream, e->vm_done[0], 0));
+  if (v.regions) CUDA_TRY(cudaStreamWaitEvent(e->stream, e->vm_done[1], 0));
+  return GAGP_OK;
 }
 
 gagp_status launch_start(gagp_engine* e, const BatchView& v) {
@@ -1777,10 +1802,7 @@ gagp_status launch_start(gagp_engine* e, const BatchView& v) {
   }
   VmPlan start_plan;
   start_plan.lanes = v.max_lanes;
-  if (const gagp_status st = launch_vm_fast(e, v, 0, e->stream, e->d_fast, e->d_counts + kSharedFast, start_plan);
-      st != GAGP_OK)
-    return st;
-  if (const gagp_status st = launch_vm_exact(e, v, 0); st != GAGP_OK) return st;
+  if (const gagp_status st = launch_vms(e, v, 0, &start_plan); st != GAGP_OK) return st;
   { Timed t(e, KN_KEYS); gb::k_member_keys<<<blocks_for(v.total_members, 128), 128, 0, e->stream>>>(v.d_desc, v.d_member_off, v.n); }
   { Timed t(e, KN_START); gb::k_start<<<v.n, 256, 0, e->stream>>>(v.d_desc, v.n); }
   return cudaPeekAtLastError() == cudaSuccess ? GAGP_OK : fail(GAGP_DEVICE_ERROR, cudaGetErrorString(cudaGetLastError()));
@@ -1848,7 +1870,7 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
   // one of the accumulator VM too.  A per-range launch, mostly empty, would
   // still wait for SM room (shared memory) behind the other ranges' VM
   // blocks, on its range's critical path.
-  const bool shared_fast = chunks > 1 && v.exact_heavy;
+  const bool shared_fast = v.exact_possible && (chunks == 1 || v.exact_heavy);
   int per_sm = 0;
   CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gb::k_vary, warps * 32, vary_smem));
   for (int c = 0; c < chunks; ++c) {
@@ -1886,11 +1908,7 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
       CUDA_TRY(cudaStreamWaitEvent(e->stream, e->chunk_done[c], 0));
     }
   }
-  if (shared_fast)
-    if (const gagp_status st2 = launch_vm_fast(e, v, 1, e->stream, e->d_fast, e->d_counts + kSharedFast, vm);
-        st2 != GAGP_OK)
-      return st2;
-  if (const gagp_status st2 = launch_vm_exact(e, v, 1); st2 != GAGP_OK) return st2;
+  if (const gagp_status st2 = launch_vms(e, v, 1, shared_fast ? &vm : nullptr); st2 != GAGP_OK) return st2;
   if (v.generational) {
     // every child becomes the member of its index (reproduce's swap), after
     // the reused children have read their sources' results and the history
@@ -1904,12 +1922,18 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
       Timed t(e, KN_PLACE);
       gb::k_gen_place<<<blocks_for(v.total_members, 256), 256, 0, e->stream>>>(v.d_desc, v.d_member_off, v.n);
     }
+    // the rows' copies and the round's end beside each other: neither reads
+    // what the other writes
+    CUDA_TRY(cudaEventRecord(e->fork, e->stream));
+    CUDA_TRY(cudaStreamWaitEvent(e->draws, e->fork, 0));
+    { Timed t(e, KN_STREAM, e->draws); gb::k_gen_finish<<<v.n, 256, 0, e->draws>>>(v.d_desc, v.n); }
+    CUDA_TRY(cudaEventRecord(e->drawn, e->draws));
     {
       Timed t(e, KN_COMMIT);
       gb::k_commit<<<blocks_for(size_t(v.total_members) * gb::kCommitLanes, 256), 256, 0, e->stream>>>(
           v.d_desc, v.d_member_off, v.n);
     }
-    { Timed t(e, KN_STREAM); gb::k_gen_finish<<<v.n, 256, 0, e->stream>>>(v.d_desc, v.n); }
+    CUDA_TRY(cudaStreamWaitEvent(e->stream, e->drawn, 0));
     return cudaPeekAtLastError() == cudaSuccess ? GAGP_OK : fail(GAGP_DEVICE_ERROR, cudaGetErrorString(cudaGetLastError()));
   }
   {
