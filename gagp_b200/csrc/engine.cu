@@ -1660,9 +1660,11 @@ void vm_exact_launch(int sm_count, cudaStream_t stream, const gb::SearchDesc* de
 // Lowering of batch items [lo, hi).
 void lower_launch(cudaStream_t stream, const gb::SearchDesc* descs, const int32_t* off, int n, int mode,
                   const gb::LowerLists& lists, int lo, int hi, bool exact) {
-  const int blocks = blocks_for(hi - lo, gb::kLowerWarps);
-  if (exact) gb::k_lower<true><<<blocks, gb::kLowerWarps * 32, 0, stream>>>(descs, off, n, mode, lists, lo, hi);
-  else gb::k_lower<false><<<blocks, gb::kLowerWarps * 32, 0, stream>>>(descs, off, n, mode, lists, lo, hi);
+  constexpr int with = gb::kLowerWarps<true>, without = gb::kLowerWarps<false>;
+  if (exact)
+    gb::k_lower<true><<<blocks_for(hi - lo, with), with * 32, 0, stream>>>(descs, off, n, mode, lists, lo, hi);
+  else
+    gb::k_lower<false><<<blocks_for(hi - lo, without), without * 32, 0, stream>>>(descs, off, n, mode, lists, lo, hi);
 }
 // The engine's program lists; accumulator programs to `fast`, counted in
 // counter word `fast_word`.

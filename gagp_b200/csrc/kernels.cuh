@@ -90,20 +90,26 @@ struct LowerLists {
 // (exact_possible in the engine), so the other lowerings, with their shared
 // memory and local arrays, stay out of the kernel and a row the accumulator
 // lowering rejects is one the reference's compiler rejects too.
-constexpr int kLowerWarps = 4;
+// Rows a block: a block's slowest row keeps its place, so without the exact
+// lowerings one (a large scalar search 273 / 246 us per round with four rows,
+// 266 / 241 with two, 264 / 240 with one); with them, whose local arrays make
+// a block's start dear, two (list 341, 330 and 349 us).
+template <bool Exact>
+constexpr int kLowerWarps = Exact ? 2 : 1;
 union LowerSmem {
   LowerScratch fast;
   ExactScratch exact;
 };
 template <bool Exact>
-__global__ void __launch_bounds__(kLowerWarps * 32, Exact ? 7 : 8)
+__global__ void __launch_bounds__(kLowerWarps<Exact> * 32, Exact ? 14 : 32)
     k_lower(const SearchDesc* descs, const int32_t* off, int n, int mode, LowerLists lists, int lo, int hi) {
   using Scratch = typename std::conditional<Exact, LowerSmem, LowerScratch>::type;
-  __shared__ Scratch scratch[kLowerWarps];
+  __shared__ Scratch scratch[kLowerWarps<Exact>];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   LowerScratch& fast_scratch = reinterpret_cast<LowerScratch&>(scratch[warp]);
   const int total_items = min(off[n], hi);
-  for (int item = lo + blockIdx.x * kLowerWarps + warp; item < total_items; item += gridDim.x * kLowerWarps) {
+  for (int item = lo + blockIdx.x * kLowerWarps<Exact> + warp; item < total_items;
+       item += gridDim.x * kLowerWarps<Exact>) {
     const int si = find_search(off, n, item);
     const SearchDesc& s = descs[si];
     if (!search_live(s)) continue;
