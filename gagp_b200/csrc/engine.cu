@@ -1831,7 +1831,7 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
   // run-generator output at its end instead (k_gen_finish)
   if (!v.generational) {
     CUDA_TRY(cudaStreamWaitEvent(e->draws, e->fork, 0));
-    { Timed t(e, KN_STREAM, e->draws); gb::k_stream<<<v.n, 256, 0, e->draws>>>(v.d_desc, v.n); }
+    { Timed t(e, KN_STREAM, e->draws); gb::k_stream<<<v.n, gb::kStreamThreads, 0, e->draws>>>(v.d_desc, v.n); }
     if (v.max_B >= gb::kClusterMinChildren) {
       // the placement levels follow from the draws alone: found here, beside
       // the variation, so the placement itself only compares and writes keys

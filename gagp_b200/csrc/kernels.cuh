@@ -571,21 +571,65 @@ __device__ __forceinline__ long long* stream_ptrs(const SearchDesc& s) { return 
 // 2B+1 draws (as far as the ring allows).  Launched on a side stream so the
 // generation overlaps the round's variation, lowering and evaluation; the
 // placement kernel waits for it and only generates what redraws add.
-__global__ void k_stream(const SearchDesc* descs, int n) {
-  __shared__ uint64_t mt[312], nw[312];
+//
+// Thread t keeps words t and t + 156 of the state: the new ones need, besides
+// the thread's own, only the next thread's old pair -- a shuffle, or shared
+// memory at a warp's edge -- and the last thread, whose next words are the
+// first thread's, forms word 0 itself.  One barrier per 312 outputs (three,
+// with the state in shared memory, took 108 us for 32768 draws beside the
+// variation, and the placement levels wait for them).
+constexpr int kStreamThreads = 160;
+__global__ void __launch_bounds__(kStreamThreads) k_stream(const SearchDesc* descs, int n) {
+  __shared__ uint64_t edge_lo[2][kStreamThreads / 32], edge_hi[2][kStreamThreads / 32], second[2];
   const SearchDesc& s = descs[blockIdx.x];
   if (!search_live(s)) return;
-  for (int i = threadIdx.x; i < 312; i += blockDim.x) mt[i] = s.mt[i];
-  __syncthreads();
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const bool on = t < 156;
+  uint64_t lo = on ? s.mt[t] : 0, hi = on ? s.mt[t + 156] : 0;
   const long long rp = stream_ptrs(s)[0];
   long long wp = stream_ptrs(s)[1];
   const long long need = (long long)s.B * s.replacement_size + 1;
-  while (wp - rp < need && wp - rp + 312 <= s.stream_capacity) {
-    mt_block(s, mt, nw, wp);
+  const int cap = s.stream_capacity;
+  int at = int((wp + t) % cap);
+  int buf = 0;
+  __syncthreads();  // every thread has read the position
+  while (wp - rp < need && wp - rp + 312 <= cap) {
+    if (lane == 0) {
+      edge_lo[buf][warp] = lo;
+      edge_hi[buf][warp] = hi;
+    }
+    if (t == 1) second[buf] = lo;
+    __syncthreads();
+    uint64_t next_lo = __shfl_down_sync(kFull, lo, 1), next_hi = __shfl_down_sync(kFull, hi, 1);
+    if (lane == 31 && warp + 1 < kStreamThreads / 32) {
+      next_lo = edge_lo[buf][warp + 1];
+      next_hi = edge_hi[buf][warp + 1];
+    }
+    if (t == 155) {
+      next_lo = edge_hi[buf][0];
+      next_hi = mt_mix(edge_lo[buf][0], second[buf], edge_hi[buf][0]);
+    }
+    lo = mt_mix(lo, next_lo, hi);
+    hi = mt_mix(hi, next_hi, lo);
+    if (on) {
+      int far = at + 156;
+      if (far >= cap) far -= cap;
+      const uint64_t a = mt_temper(lo), b = mt_temper(hi);
+      s.stream[at] = a;
+      s.stream[far] = b;
+      s.stream_mod[at] = mod_p(a, s.mod_magic, uint32_t(s.P));
+      s.stream_mod[far] = mod_p(b, s.mod_magic, uint32_t(s.P));
+    }
+    at += 312;
+    if (at >= cap) at -= cap;
     wp += 312;
+    buf ^= 1;
   }
-  for (int i = threadIdx.x; i < 312; i += blockDim.x) s.mt[i] = mt[i];
-  if (threadIdx.x == 0) stream_ptrs(s)[1] = wp;
+  if (on) {
+    s.mt[t] = lo;
+    s.mt[t + 156] = hi;
+  }
+  if (t == 0) stream_ptrs(s)[1] = wp;
 }
 
 // The `count` best members in ranking order (smallest (key, member) first),
