@@ -159,11 +159,11 @@ cudaError_t copy_d2h(gagp_engine* e, void* dst, const void* src, size_t bytes) {
 namespace {
 
 enum KernelId {
-  KN_INIT, KN_LOWER, KN_VM_FAST, KN_KEYS, KN_START, KN_RECORD, KN_VARY, KN_CHILD, KN_PLACE,
+  KN_INIT, KN_LOWER, KN_VM_FAST, KN_KEYS, KN_START, KN_RECORD, KN_VARY, KN_PLACE,
   KN_COMMIT, KN_STREAM, KN_LEVELS, KN_VM_EXACT, KN_INDEX, KN_COUNT
 };
 const char* const kKernelNames[KN_COUNT] = {"k_init_population", "k_lower", "k_vm_fast",
-                                            "k_member_keys", "k_start", "k_record", "k_vary", "k_child_results",
+                                            "k_member_keys", "k_start", "k_record", "k_vary",
                                             "k_place", "k_commit", "k_stream", "k_place_levels", "k_vm_exact",
                                             "k_member_index"};
 
@@ -1915,10 +1915,6 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
     // every child becomes the member of its index (reproduce's swap), after
     // the reused children have read their sources' results and the history
     // entry has read the members
-    {
-      Timed t(e, KN_CHILD);
-      gb::k_child_results<<<blocks_for(v.total_children, 128), 128, 0, e->stream>>>(v.d_desc, v.d_child_off, v.n);
-    }
     CUDA_TRY(cudaStreamWaitEvent(e->stream, e->join, 0));
     {
       Timed t(e, KN_PLACE);

@@ -71,6 +71,28 @@ __global__ void k_init_population(const SearchDesc* descs, const int32_t* off, i
   s.len[i] = make_len(g.nodes, g.constants);
 }
 
+// Packed ranking key: (-fitness, wrong, nodes); smaller is better.
+__device__ __forceinline__ uint64_t pack_key(const SearchDesc& s, double fitness, uint32_t wrong, uint32_t nodes) {
+  const uint64_t loss = uint64_t(-fitness);
+  if (!s.has_wrong) return loss;
+  return (loss << s.key_shift_wrong) | (uint64_t(wrong) << s.key_shift_nodes) | uint64_t(nodes);
+}
+
+// A child that reuses member `source`'s result (an unchanged parent, an
+// identical member): its statistics and key, by one lane.  The members'
+// statistics stand until the round's commit.
+__device__ inline void reuse_result(const SearchDesc& s, int b, int source) {
+  s.c_fitness[b] = s.fitness[source];
+  s.c_wrong[b] = s.wrong[source];
+  s.c_nodes[b] = s.nodes[source];
+  s.c_key[b] = s.key[source];
+  atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[1]), 1ULL);
+  // the generational evaluate copies a reused member's case counts too
+  // (HostPhasePopulation::evaluate, phase_population_cpu.cpp:252-253), so
+  // its program-case total covers every member
+  if (s.generational) atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[2]), (unsigned long long)s.C);
+}
+
 // ----------------------------------------------------------- lowering
 // Where lowered programs are listed, with each list's size: accumulator
 // programs, register code, reference bytecode for the per-thread
@@ -119,7 +141,10 @@ __global__ void __launch_bounds__(kLowerWarps<Exact> * 32, Exact ? 14 : 32)
       const int32_t l = s.len[slot];
       t = LRow{s.node + size_t(slot) * s.stride, s.cval + size_t(slot) * s.stride, len_nodes(l), len_consts(l)};
     } else {
-      if (!s.c_eval[slot]) continue;
+      if (!s.c_eval[slot]) {
+        if (lane == 0 && s.c_reuse[slot] >= 0) reuse_result(s, slot, s.c_reuse[slot]);
+        continue;
+      }
       const int32_t l = s.clen[slot];
       t = LRow{s.cnode + size_t(slot) * s.stride, s.ccval + size_t(slot) * s.stride, len_nodes(l), len_consts(l)};
       // a child its parent does not cover reuses an identical current
@@ -132,6 +157,7 @@ __global__ void __launch_bounds__(kLowerWarps<Exact> * 32, Exact ? 14 : 32)
           if (lane == 0) {
             s.c_reuse[slot] = m;
             s.c_eval[slot] = 0;
+            reuse_result(s, slot, m);
           }
           continue;
         }
@@ -200,12 +226,18 @@ __global__ void __launch_bounds__(kLowerWarps<Exact> * 32, Exact ? 14 : 32)
 
 __device__ __forceinline__ void store_result(const SearchDesc& s, int mode, int slot, int64_t loss, uint32_t wrong) {
   const double f = -double(loss);
+  const uint32_t w = s.has_wrong ? wrong : 0;
   if (mode == 0) {
     s.fitness[slot] = f;
-    s.wrong[slot] = s.has_wrong ? wrong : 0;
+    s.wrong[slot] = w;
   } else {
+    // a child's ranking key too (evolve.cpp:403-413): with the reused
+    // children's, formed as they are lowered, the placement reads keys only
+    const uint32_t nodes = s.has_wrong ? ranking_nodes(s, s.cnode + size_t(slot) * s.stride, len_nodes(s.clen[slot])) : 0;
     s.c_fitness[slot] = f;
-    s.c_wrong[slot] = s.has_wrong ? wrong : 0;
+    s.c_wrong[slot] = w;
+    s.c_nodes[slot] = nodes;
+    s.c_key[slot] = pack_key(s, f, w, nodes);
   }
 }
 
@@ -486,13 +518,6 @@ __global__ void __launch_bounds__(256, K == 4 ? 3 : 4) k_vm_fast(const SearchDes
                   (unsigned long long)len * (unsigned long long)s.C);
     }
   }
-}
-
-// Packed ranking key: (-fitness, wrong, nodes); smaller is better.
-__device__ __forceinline__ uint64_t pack_key(const SearchDesc& s, double fitness, uint32_t wrong, uint32_t nodes) {
-  const uint64_t loss = uint64_t(-fitness);
-  if (!s.has_wrong) return loss;
-  return (loss << s.key_shift_wrong) | (uint64_t(wrong) << s.key_shift_nodes) | uint64_t(nodes);
 }
 
 // Member statistics after the initial evaluation.
@@ -883,54 +908,6 @@ constexpr int kClusterThreads = 1024;
 constexpr int kClusterPer = 2;
 constexpr int kClusterMinChildren = 4096;
 
-// A child's result and ranking key before any placement (evolve.cpp:403-413):
-// an unchanged genotype takes its parent's.  Returns the key; reports a
-// reuse through `reused`.
-__device__ inline uint64_t child_result_of(const SearchDesc& s, int b, bool* reused) {
-  const int source = s.c_reuse[b];
-  double f;
-  uint32_t w, nodes;
-  *reused = source >= 0;
-  if (source >= 0) {
-    f = s.fitness[source];
-    w = s.wrong[source];
-    nodes = s.nodes[source];
-  } else {
-    f = s.c_fitness[b];
-    w = s.c_wrong[b];
-    nodes = s.has_wrong ? ranking_nodes(s, s.cnode + size_t(b) * s.stride, len_nodes(s.clen[b])) : 0;
-  }
-  s.c_fitness[b] = f;
-  s.c_wrong[b] = w;
-  s.c_nodes[b] = nodes;
-  const uint64_t key = pack_key(s, f, w, nodes);
-  s.c_key[b] = key;
-  return key;
-}
-__device__ inline void child_result(const SearchDesc& s, int b) {
-  bool reused;
-  child_result_of(s, b, &reused);
-  if (reused) {
-    atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[1]), 1ULL);
-    // the generational evaluate copies a reused member's case counts too
-    // (HostPhasePopulation::evaluate, phase_population_cpu.cpp:252-253), so
-    // its program-case total covers every member
-    atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[2]), (unsigned long long)s.C);
-  }
-}
-
-// Results of all children of a generational round, thread per child.
-__global__ void k_child_results(const SearchDesc* descs, const int32_t* off, int n) {
-  const int item = blockIdx.x * blockDim.x + threadIdx.x;
-  if (item >= off[n]) return;
-  const int si = find_search(off, n, item);
-  const SearchDesc& s = descs[si];
-  if (!search_live(s)) return;
-  const int b = item - off[si];
-  child_result(s, b);
-}
-
-
 // Windowed placement step over lanes [seg_begin, seg_end) of a window whose
 // children's draws do not overlap (every lane's members differ from every
 // earlier active lane's): victims from the current keys equal the
@@ -1042,27 +1019,12 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
   }
   for (int i = tid; i < 312; i += blockDim.x) mt[i] = s.mt[i];
   __syncthreads();
-  // the children's results and keys: formed here for a round the cluster
-  // kernel leaves out
   constexpr int kPerThread = Per;
   constexpr bool kKeep = Per <= 4;  // the children's keys stay in registers
   uint64_t kept[kKeep ? Per : 1];
   if constexpr (kKeep) {
-    int reused_here = 0;
 #pragma unroll
-    for (int t = 0; t < Per; ++t) {
-      const int b = tid * Per + t;
-      kept[t] = ~0ULL;
-      if (b < B) {
-        bool reused = false;
-        kept[t] = B < kClusterMinChildren ? child_result_of(s, b, &reused) : s.c_key[b];
-        reused_here += reused;
-      }
-    }
-    for (int o = 16; o; o >>= 1) reused_here += __shfl_xor_sync(kFull, reused_here, o);
-    if ((tid & 31) == 0 && reused_here)
-      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[1]), (unsigned long long)reused_here);
-    __syncthreads();  // the windowed path reads every child's key
+    for (int t = 0; t < Per; ++t) kept[t] = tid * Per + t < B ? s.c_key[tid * Per + t] : ~0ULL;
   }
   const long long rp = stream_ptrs(s)[0];
   long long wp = stream_ptrs(s)[1];
@@ -1601,25 +1563,10 @@ __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThr
   const int P = s.P, B = s.B, cap = s.stream_capacity;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const long long rp = stream_ptrs(s)[0], wp = stream_ptrs(s)[1];
-  // the children's results and keys, formed before any decision so that the
-  // single-block placement finds them too
   const int begin = (rank * kClusterThreads + tid) * kClusterPer;
   uint64_t kv[kClusterPer];  // the children's keys
-  if (B >= kClusterMinChildren) {
-    int reused_here = 0;
 #pragma unroll
-    for (int t = 0; t < kClusterPer; ++t) {
-      kv[t] = ~0ULL;
-      if (begin + t < B) {
-        bool reused;
-        kv[t] = child_result_of(s, begin + t, &reused);
-        reused_here += reused;
-      }
-    }
-    for (int o = 16; o; o >>= 1) reused_here += __shfl_xor_sync(kFull, reused_here, o);
-    if (lane == 0 && reused_here)
-      atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[1]), (unsigned long long)reused_here);
-  }
+  for (int t = 0; t < kClusterPer; ++t) kv[t] = begin + t < B ? s.c_key[begin + t] : ~0ULL;
   // the levels come from k_place_levels, run earlier in this round
   if (!cluster_placement_applies(s, rp, wp) || s.level_plan[0] != s.round[0] + 1) {
     if (rank == 0 && tid == 0) *s.place_state = 0;
@@ -1890,7 +1837,7 @@ __global__ void k_commit(const SearchDesc* descs, const int32_t* off, int n) {
 // ----------------------------------------------------------- generational
 // The generational schedule's placement (reproduce, phase_population_cpu.cpp:
 // 269-312, then the next evaluate's reuse, :243-265): child i becomes member
-// i with its result.  Runs after k_child_results, which read the members'
+// i with its result.  Runs after the lowering, which read the members'
 // results for the reused children; k_commit then copies the rows.
 __global__ void k_gen_place(const SearchDesc* descs, const int32_t* off, int n) {
   const int item = blockIdx.x * blockDim.x + threadIdx.x;
