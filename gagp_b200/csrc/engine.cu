@@ -1463,9 +1463,8 @@ gagp_status gagp_b200_search_create(gagp_engine* e, const gagp_grammar* g, const
   d.mod_magic = ~0ULL / uint64_t(s->P);
   d.bounded_threshold = (0 - uint64_t(s->P)) % uint64_t(s->P);
   d.round_seed = at<uint64_t>(b, p.round_seed);
-  d.best = at<int32_t>(b, p.best); d.placed = at<int32_t>(b, p.placed); d.round = at<int32_t>(b, p.round);
+  d.best = at<int32_t>(b, p.best); d.placed = at<int32_t>(b, p.placed); d.place_state = at<int32_t>(b, p.place_state); d.round = at<int32_t>(b, p.round);
   d.elites = at<int32_t>(b, p.elites);
-  d.place_state = at<int32_t>(b, p.place_state);
   d.child_level = at<int16_t>(b, p.child_level); d.level_plan = at<int32_t>(b, p.level_plan);
   d.hist_sum = at<int64_t>(b, p.hist_sum); d.hist_fitness = at<double>(b, p.hist_fitness);
   d.hist_wrong = at<uint32_t>(b, p.hist_wrong); d.hist_nodes = at<uint32_t>(b, p.hist_nodes);
@@ -1545,6 +1544,7 @@ struct BatchView {
   int max_code_stride = 2;
   int max_C = 1, max_inputs = 0;
   int max_B = 0;                     // the largest round of the batch
+  bool levels_small = false, levels_large = false;  // which of the level kernels the batch's rounds need
   bool exact_heavy = false;          // some search's programs mostly need the exact VM
   bool exact_possible = false;       // some search's programs may need it
   bool regions = false;              // some search's grammar has bounded regions
@@ -1606,6 +1606,7 @@ gagp_status make_batch_view(gagp_engine* e, const std::vector<Search*>& list, Ba
   v->max_code_stride = 2;
   v->max_lanes = 1;
   v->max_B = 0;
+  v->levels_small = v->levels_large = false;
   v->max_C = 1;
   v->max_inputs = 0;
   v->exact_heavy = v->exact_possible = false;
@@ -1629,6 +1630,7 @@ gagp_status make_batch_view(gagp_engine* e, const std::vector<Search*>& list, Ba
     v->max_code_stride = std::max(v->max_code_stride, s->desc.code_stride);
     v->max_draws = std::max(v->max_draws, (long long)s->B * s->desc.replacement_size + 1);
     v->max_B = std::max(v->max_B, s->B);
+    (gb::levels_small(s->desc) ? v->levels_small : v->levels_large) = true;
   }
   return ensure_lists(e, size_t(std::max(v->total_members, v->total_children)));
 }
@@ -1832,9 +1834,13 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
   if (!v.generational) {
     CUDA_TRY(cudaStreamWaitEvent(e->draws, e->fork, 0));
     { Timed t(e, KN_STREAM, e->draws); gb::k_stream<<<v.n, gb::kStreamThreads, 0, e->draws>>>(v.d_desc, v.n); }
-    if (v.max_B >= gb::kClusterMinChildren) {
-      // the placement levels follow from the draws alone: found here, beside
-      // the variation, so the placement itself only compares and writes keys
+    // the placement levels follow from the draws alone: found here, beside
+    // the variation, so the placement itself only compares and writes keys
+    if (v.levels_small) {
+      Timed t(e, KN_LEVELS, e->draws);
+      gb::k_place_levels_small<<<v.n, gb::kClusterThreads, 0, e->draws>>>(v.d_desc, v.n);
+    }
+    if (v.levels_large) {
       Timed t(e, KN_LEVELS, e->draws);
       const int local_P = (v.max_P + gb::kPlaceCtas - 1) / gb::kPlaceCtas;
       gb::k_place_levels<<<v.n * gb::kPlaceCtas, gb::kClusterThreads, 2 * size_t(local_P) * sizeof(int32_t) + 16,
@@ -1936,11 +1942,11 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
   }
   {
     Timed t(e, KN_PLACE);
-    // member keys plus as many 16-bit staged draws as fit (B * replacement + slack)
+    // member keys, then the 16-bit staged draws (B * replacement + slack, as
+    // many as fit) or the child placed on each member
     const size_t limit = e->max_smem - 16384;  // static shared memory of k_place: ~13 KB
-    // keys, then either the level owners (4 bytes per member) or the staged draws
     size_t bytes = size_t(v.max_P + 1) * sizeof(uint64_t) +
-                   std::max(size_t(v.max_P) * sizeof(int32_t) + 64, size_t(v.max_draws + 64) * sizeof(uint16_t));
+                   std::max(size_t(v.max_P) * sizeof(int16_t) + 64, size_t(v.max_draws + 64) * sizeof(uint16_t));
     bytes = std::min(bytes, limit);
     CUDA_TRY(cudaStreamWaitEvent(e->stream, e->join, 0));
     CUDA_TRY(cudaStreamWaitEvent(e->stream, e->drawn, 0));

@@ -900,13 +900,15 @@ __global__ void k_status(const SearchDesc* descs, int n, int32_t* out) {
   out[i] = (s.round[2] ? 1 : 0) | (s.round[3] ? 2 : 0);
 }
 
-// Cluster placement shape (k_place_levels, k_place_cluster): kPlaceCtas
-// blocks of kClusterThreads threads, kClusterPer children per thread, for
-// rounds of at least kClusterMinChildren children.
+// Shape of the cluster that finds a large round's placement levels
+// (k_place_levels): kPlaceCtas blocks of kClusterThreads threads, kClusterPer
+// children per thread.  Rounds that one block holds take one
+// (k_place_levels_small).
 constexpr int kPlaceCtas = 8;
 constexpr int kClusterThreads = 1024;
 constexpr int kClusterPer = 2;
-constexpr int kClusterMinChildren = 4096;
+constexpr int kLevelsSmall = kClusterThreads * kClusterPer;  // children
+constexpr int kClusterMinChildren = 4096;  // rounds the cluster places (k_place_cluster)
 
 // Windowed placement step over lanes [seg_begin, seg_end) of a window whose
 // children's draws do not overlap (every lane's members differ from every
@@ -968,10 +970,11 @@ __device__ __forceinline__ int latest_overlap(int d0, int d1) {
 // memory of the launch (member keys, then the level owners or staged draws).
 //
 // Level-parallel path (replacement size 2): without a redraw child j draws
-// stream positions 2j and 2j+1.  A child is ready once it is the earliest
-// unplaced child drawing each of its members; the ready children of a level
-// draw disjoint members, so they read exactly the keys the sequential loop
-// would and place at once.  The best member before each child is then a
+// stream positions 2j and 2j+1, and its level follows from the draws alone: a
+// child is ready once it is the earliest unplaced child drawing each of its
+// members (k_place_levels, run beside the variation).  The ready children of
+// a level draw disjoint members, so they read exactly the keys the sequential
+// loop would and place at once.  The best member before each child is then a
 // prefix minimum of (key, member) in child order; a child whose victim is
 // that best member would have redrawn (both its draws are the best member),
 // and then the round is replayed on the exact windowed path.
@@ -987,36 +990,38 @@ __device__ __forceinline__ bool key_before(uint64_t ka, int va, uint64_t kb, int
   return ka < kb || (ka == kb && va < vb);
 }
 // Per: children per thread of the level-parallel path, the fewest that hold
-// the search's round (1 up to 1024 children, 4 up to 4096, 16 beyond).  What
-// bounds it is latency: two barriers a level, and the children's keys.  With
-// 16 children per thread whatever the round, 64 of the 1024 threads placed a
-// round of 1024 children and loaded each level's keys from global memory:
-// 64 us, and 9 us more for a kernel that formed their results.  With up to 4,
-// rounds below kClusterMinChildren form their children's results here and the
-// keys stay in registers: 21 us.
+// the search's round (1 up to 1024 children, 4 up to 4096; past that the
+// cluster places).  Bound by latency: a barrier and two shared-memory keys per
+// level, some 11 levels.  Finding the levels here with two atomics and two
+// barriers each, and copying the placed members' statistics (k_commit does),
+// took a round of 1024 children 15 us and one of 2048 31, 9 and 14 now.
+// With 16 children a thread for larger rounds, a child's key had to come from
+// global memory each time: 88 us for 16384 against the cluster's 36.
 struct PlaceShared {
   uint64_t mt[312], nw[312];
   uint64_t ck_stage[1024];
   uint64_t scan_key[32];
   int scan_idx[32];
   long long pos, wp;
-  int best, fail, ready_count[2], redraw_at;
+  int best, fail, redraw_at;
 };
+// Whether a round of search s has placement levels: replacement size 2 and
+// the whole round's draws in the stream.
+__device__ __forceinline__ bool levels_apply(const SearchDesc& s, long long rp, long long wp) {
+  return s.replacement_size == 2 && s.B <= kPlaceCtas * kClusterThreads * kClusterPer && wp - rp >= 2LL * s.B + 1;
+}
 template <int Per>
 __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, uint64_t* keys, int dyn_bytes,
-                                         int cluster_state) {
+                                         bool replay) {
   uint64_t (&mt)[312] = sh.mt, (&nw)[312] = sh.nw, (&ck_stage)[1024] = sh.ck_stage, (&scan_key)[32] = sh.scan_key;
-  int (&scan_idx)[32] = sh.scan_idx, (&ready_count)[2] = sh.ready_count;
+  int (&scan_idx)[32] = sh.scan_idx;
   long long &shared_pos = sh.pos, &shared_wp = sh.wp;
   int &shared_best = sh.best, &shared_fail = sh.fail, &redraw_at = sh.redraw_at;
   const long long t0 = clock64();
   const int P = s.P, B = s.B, rs = s.replacement_size, cap = s.stream_capacity;
   const int tid = threadIdx.x;
   int32_t* __restrict__ placed = s.placed;
-  for (int m = tid; m < P; m += blockDim.x) {
-    keys[m] = s.key[m];
-    placed[m] = -1;
-  }
+  for (int m = tid; m < P; m += blockDim.x) keys[m] = s.key[m];
   for (int i = tid; i < 312; i += blockDim.x) mt[i] = s.mt[i];
   __syncthreads();
   constexpr int kPerThread = Per;
@@ -1035,13 +1040,15 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
   }
   const long long t1 = clock64();
   // ---------------------------------------------------- level-parallel path
-  // owner area after the keys, 16-byte aligned, with 64 bytes of slack for
-  // the per-thread 16-byte reads of the staged draws
-  int32_t* owner = reinterpret_cast<int32_t*>(keys + P + (P & 1));
-  const bool parallel_path = cluster_state == 0 && rs == 2 && blockDim.x == kPlaceThreads &&
-                             B <= kPlaceThreads * kPerThread &&
-                             wp - rp >= need &&
-                             dyn_bytes >= int(sizeof(uint64_t)) * (P + 1) + int(sizeof(int32_t)) * P + 64;
+  // after the keys, 16-byte aligned: first the staged draws, with 64 bytes
+  // of slack for the per-thread 16-byte reads of them, then the child placed
+  // on each member
+  uint16_t* const stage = reinterpret_cast<uint16_t*>(keys + P + (P & 1));
+  int16_t* const on = reinterpret_cast<int16_t*>(stage);
+  const int after = dyn_bytes - int(sizeof(uint64_t)) * (P + 1) - 64;
+  const bool parallel_path = !replay && levels_apply(s, rp, wp) && s.level_plan[0] == s.round[0] + 1 &&
+                             blockDim.x == kPlaceThreads && B <= kPlaceThreads * kPerThread &&
+                             after >= int(sizeof(int16_t)) * max(P, 2 * B);
   bool parallel_done = false;
   if (parallel_path) {
     // thread tid owns children [16 tid, 16 tid + 16): cand[t] holds child
@@ -1054,11 +1061,10 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
       if constexpr (kKeep) return kept[t];
       else return ckey[begin + t];
     };
-    // the 2B draws (residues < P <= 65536), staged as 16-bit values in the
-    // owner area with coalesced loads, then read back per thread: child j's
-    // pair is the 32-bit word j
+    // the 2B draws (residues < P <= 65536), staged as 16-bit values with
+    // coalesced loads, then read back per thread: child j's pair is the
+    // 32-bit word j
     {
-      uint16_t* stage = reinterpret_cast<uint16_t*>(owner);
       const uint32_t* __restrict__ smod = s.stream_mod;
       for (int i = tid; i < 2 * B; i += blockDim.x) {
         int pos = base + i;
@@ -1066,12 +1072,28 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
         stage[i] = uint16_t(smod[pos]);
       }
     }
+    // the children's levels, two a word (rows of child_level are padded)
+    uint32_t level_pair[(kPerThread + 1) / 2];
+    {
+      const uint32_t* pairs = reinterpret_cast<const uint32_t*>(s.child_level);
+      if constexpr (kPerThread == 1) {
+        level_pair[0] = begin < B ? uint32_t(uint16_t(s.child_level[begin])) : 0xffffu;
+      } else {
+#pragma unroll
+        for (int q = 0; q < kPerThread / 4; ++q) {
+          const uint2 v = begin + 4 * q < B ? *reinterpret_cast<const uint2*>(pairs + begin / 2 + 2 * q)
+                                            : make_uint2(~0u, ~0u);
+          level_pair[2 * q] = v.x;
+          level_pair[2 * q + 1] = v.y;
+        }
+      }
+    }
     __syncthreads();
     uint32_t cand[kPerThread];
-    uint32_t pending = 0;
     {
+      const uint32_t* words = reinterpret_cast<const uint32_t*>(stage);
       if constexpr (kPerThread % 4 == 0) {
-        const uint4* pairs = reinterpret_cast<const uint4*>(owner) + size_t(begin) / 4;
+        const uint4* pairs = reinterpret_cast<const uint4*>(words) + size_t(begin) / 4;
 #pragma unroll
         for (int q = 0; q < kPerThread / 4; ++q) {
           const uint4 v = begin < B ? pairs[q] : make_uint4(0, 0, 0, 0);
@@ -1082,77 +1104,45 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
         }
       } else {
 #pragma unroll
-        for (int t = 0; t < kPerThread; ++t)
-          cand[t] = begin + t < B ? reinterpret_cast<const uint32_t*>(owner)[begin + t] : 0;
+        for (int t = 0; t < kPerThread; ++t) cand[t] = begin + t < B ? words[begin + t] : 0;
       }
 #pragma unroll
-      for (int t = 0; t < kPerThread; ++t) {
-        if (begin + t < B) pending |= 1u << t;
-        else cand[t] = 0;
-      }
+      for (int t = 0; t < kPerThread; ++t)
+        if (begin + t >= B) {
+          cand[t] = 0;
+          level_pair[t / 2] |= 0xffffu << (16 * (t & 1));  // no level
+        }
     }
-    __syncthreads();  // the owner area is reset below
-    // owner[m]: the earliest child of the current level that drew member m,
-    // tagged with the level so that no per-level reset is needed (a later
-    // level's tag is smaller than every earlier one's)
-    for (int m = tid; m < P; m += blockDim.x) owner[m] = 0x7fffffff;
-    if (tid == 0) {
-      ready_count[0] = ready_count[1] = 0;
-      redraw_at = 0x7fffffff;
-    }
+    __syncthreads();  // the staged draws give way to the placed children
+    for (int m = tid; m < P; m += blockDim.x) on[m] = -1;
+    if (tid == 0) redraw_at = 0x7fffffff;
     __syncthreads();
-    int levels_run = 0, left = B;
+    const int levels_run = s.level_plan[1];
     const long long level_start = clock64();
-    for (int level = 0; level <= B; ++level) {
-      ++levels_run;
-      const int tag = (0x7fff - level) << 16;
+    for (int level = 0; level < levels_run; ++level) {
 #pragma unroll
-      for (int t = 0; t < kPerThread; ++t)
-        if (pending >> t & 1) {
-          atomicMin(&owner[cand[t] & 0xffff], tag | (begin + t));
-          atomicMin(&owner[cand[t] >> 16], tag | (begin + t));
-        }
-      __syncthreads();
-      // children owning both their members are placed at this level; they
-      // touch disjoint members, so their order within the level is free
-      uint32_t ready = 0;
+      for (int h = 0; h < kPerThread; h += kBatch) {
+        uint32_t ready = 0;
 #pragma unroll
-      for (int t = 0; t < kPerThread; ++t)
-        if ((pending >> t & 1) && owner[cand[t] & 0xffff] == (tag | (begin + t)) &&
-            owner[cand[t] >> 16] == (tag | (begin + t)))
-          ready |= 1u << t;
-      if (ready) {
+        for (int u = 0; u < kBatch; ++u)
+          if ((level_pair[(h + u) / 2] >> (16 * ((h + u) & 1)) & 0xffffu) == uint32_t(level)) ready |= 1u << u;
+        uint64_t kv[kBatch];
 #pragma unroll
-        for (int h = 0; h < kPerThread; h += kBatch) {
-          uint64_t kv[kBatch];
+        for (int u = 0; u < kBatch; ++u) kv[u] = (ready >> u & 1) ? key_of(h + u) : 0;
 #pragma unroll
-          for (int u = 0; u < kBatch; ++u) kv[u] = (ready >> (h + u) & 1) ? key_of(h + u) : 0;
-#pragma unroll
-          for (int u = 0; u < kBatch; ++u)
-            if (ready >> (h + u) & 1) {
-              const int d0 = int(cand[h + u] & 0xffff), d1 = int(cand[h + u] >> 16);
-              const uint64_t k0 = keys[d0], k1 = keys[d1];
-              // worst of the pair: the second replaces the first when the first is better
-              const int v = (k0 < k1 || (k0 == k1 && d0 < d1)) ? d1 : d0;
-              keys[v] = kv[u];
-              placed[v] = begin + h + u;
-              cand[h + u] = uint32_t(v);
-            }
-        }
-        pending &= ~ready;
+        for (int u = 0; u < kBatch; ++u)
+          if (ready >> u & 1) {
+            const int d0 = int(cand[h + u] & 0xffff), d1 = int(cand[h + u] >> 16);
+            const uint64_t k0 = keys[d0], k1 = keys[d1];
+            // worst of the pair: the second replaces the first when the first is better
+            const int v = (k0 < k1 || (k0 == k1 && d0 < d1)) ? d1 : d0;
+            keys[v] = kv[u];
+            on[v] = int16_t(begin + h + u);
+            cand[h + u] = uint32_t(v);
+          }
       }
-      {
-        // one shared-memory atomic per warp, not per thread
-        int placed_here = __popc(ready);
-        for (int o = 16; o; o >>= 1) placed_here += __shfl_xor_sync(kFull, placed_here, o);
-        if ((tid & 31) == 0 && placed_here) atomicAdd(&ready_count[level & 1], placed_here);
-      }
-      if (tid == 0) ready_count[(level + 1) & 1] = 0;  // read by every thread before this level's first barrier
       __syncthreads();
-      left -= ready_count[level & 1];
-      if (left == 0) break;
     }
-    const int level_left = left;
     if (tid == 0)
       atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[14]), (unsigned long long)(clock64() - level_start));
     // best member before each child (child order): each thread's minimum of
@@ -1230,7 +1220,7 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
     parallel_done = redraw_at == 0x7fffffff;
     if (tid == 0)  // levels of the parallel path; a replay adds 2^20
       atomicAdd(reinterpret_cast<unsigned long long*>(&s.counters[7]),
-                (unsigned long long)(B - level_left >= 0 ? levels_run : 0) + (parallel_done ? 0ULL : (1ULL << 20)));
+                (unsigned long long)levels_run + (parallel_done ? 0ULL : (1ULL << 20)));
     if (parallel_done) {
       if (tid == 0) {
         int fv = best0;
@@ -1247,15 +1237,15 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
         shared_pos = pos + 1;
         shared_wp = wp;
       }
+      for (int m = tid; m < P; m += blockDim.x) placed[m] = on[m];
     } else {
       // replay the round on the exact windowed path from the round's keys
-      for (int m = tid; m < P; m += blockDim.x) {
-        keys[m] = s.key[m];
-        placed[m] = -1;
-      }
+      for (int m = tid; m < P; m += blockDim.x) keys[m] = s.key[m];
     }
     __syncthreads();
   }
+  if (!parallel_done)
+    for (int m = tid; m < P; m += blockDim.x) placed[m] = -1;
   // ---------------------------------------------------- windowed path
   uint16_t* draws = reinterpret_cast<uint16_t*>(keys + P);
   const int slots = (dyn_bytes - int(sizeof(uint64_t)) * P) / int(sizeof(uint16_t));
@@ -1371,36 +1361,6 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
     stream_ptrs(s)[1] = shared_wp;
   }
   for (int i = tid; i < 312; i += blockDim.x) s.mt[i] = mt[i];
-  {
-    // placed members take their child's statistics; four members' loads in flight at once
-    const double* __restrict__ cfit = s.c_fitness;
-    const uint32_t* __restrict__ cwrong = s.c_wrong;
-    const uint32_t* __restrict__ cnodes = s.c_nodes;
-    const int stride = blockDim.x;
-    for (int m0 = tid; m0 < P; m0 += 4 * stride) {
-      int c[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) c[u] = m0 + u * stride < P ? placed[m0 + u * stride] : -1;
-      double f[4];
-      uint32_t w[4], nd[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (c[u] >= 0) {
-          f[u] = cfit[c[u]];
-          w[u] = cwrong[c[u]];
-          nd[u] = cnodes[c[u]];
-        }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (c[u] >= 0) {
-          const int m = m0 + u * stride;
-          s.key[m] = keys[m];
-          s.fitness[m] = f[u];
-          s.wrong[m] = w[u];
-          s.nodes[m] = nd[u];
-        }
-    }
-  }
   if (tid == 0) {
     const int r = s.round[0] + 1;
     s.round[0] = r;
@@ -1422,32 +1382,10 @@ __global__ void __launch_bounds__(kPlaceThreads, 1) k_place(const SearchDesc* de
   __shared__ PlaceShared sh;
   const SearchDesc& s = descs[blockIdx.x];
   if (!search_live(s)) return;
-  const int cluster_state = after_cluster ? *s.place_state : 0;
-  if (cluster_state == 1) return;
-  if (s.B <= kPlaceThreads) place_round<1>(s, sh, place_keys, dyn_bytes, cluster_state);
-  else if (s.B <= 4 * kPlaceThreads) place_round<4>(s, sh, place_keys, dyn_bytes, cluster_state);
-  else place_round<16>(s, sh, place_keys, dyn_bytes, cluster_state);
-}
-
-// Cluster placement: the level-parallel placement above, spread over a
-// cluster of kPlaceCtas blocks that share their shared memory.  Member m
-// lives in block m % kPlaceCtas (its key and level owner); thread g of the
-// cluster owns children [2g, 2g + 2), so the blocks hold the children in
-// order.  Each level is two cluster barriers: level-tagged atomicMin on the
-// owning block's owner word, then the ready children place (remote key
-// reads and writes).  The running best before each child is a scan inside
-// each block plus a prefix over the blocks' totals.  When a child would have
-// redrawn, nothing is written back (place_state 2) and k_place replays the
-// round on the exact path; a batch of fewer than kClusterMinChildren
-// children, another replacement size or a stream short of draws is left to
-// k_place (place_state 0), whose single block is then as fast.  On success
-// this kernel finishes the round as k_place does (statistics, best member,
-// stream position, next seed).
-// Whether a round of search s is placed by the cluster (the same answer in
-// every block and in both cluster kernels of the round).
-__device__ __forceinline__ bool cluster_placement_applies(const SearchDesc& s, long long rp, long long wp) {
-  return s.replacement_size == 2 && s.B >= kClusterMinChildren && s.B <= kPlaceCtas * kClusterThreads * kClusterPer &&
-         wp - rp >= 2LL * s.B + 1;
+  const int state = after_cluster ? *s.place_state : 0;
+  if (state == 1) return;
+  if (s.B <= kPlaceThreads) place_round<1>(s, sh, place_keys, dyn_bytes, state == 2);
+  else place_round<4>(s, sh, place_keys, dyn_bytes, state == 2);
 }
 
 // The children's two drawn members for this round, from the run generator's
@@ -1465,18 +1403,69 @@ __device__ __forceinline__ uint32_t child_draws(const SearchDesc& s, int base, i
 // is placed: its level is one more than the largest level among those, which
 // depends on the draws alone.  So this runs on the side stream, once the run
 // generator has topped up the stream, while the children are still being
-// varied and evaluated; k_place_cluster then only compares and writes keys,
-// level by level.  Levels are found as the placement would find them: each
-// level, every pending child claims both its members with a level-tagged
-// atomicMin on the owning block's owner word (member m lives in block
-// m % kPlaceCtas), and a child that owns both is at this level.  The owner
-// words alternate between two arrays by level parity: a thread that has
-// moved on to level L + 1 claims in the other array, so its claims never
+// varied and evaluated; k_place then only compares and writes keys, level by
+// level.  Levels are found as the placement would find them: each level,
+// every pending child claims both its members with a level-tagged atomicMin
+// on the member's owner word, and a child that owns both is at this level.
+// The owner words alternate between two arrays by level parity: a thread that
+// has moved on to level L + 1 claims in the other array, so its claims never
 // disturb a slower thread still checking level L (and the array of level L
 // is claimed again only after barrier L + 1, which every check of level L
 // precedes).  The levels are therefore the exact longest-path levels,
 // whatever the timing.
 // level_plan: [0] the round + 1 the levels belong to, [1] their number.
+//
+// In one block, for rounds of at most kLevelsSmall children whose two banks
+// fit its shared memory.
+__host__ __device__ __forceinline__ bool levels_small(const SearchDesc& s) { return s.B <= kLevelsSmall && s.P <= kLevelsSmall; }
+__global__ void __launch_bounds__(kClusterThreads) k_place_levels_small(const SearchDesc* descs, int n) {
+  __shared__ int32_t owner[2][kLevelsSmall];
+  const SearchDesc& s = descs[blockIdx.x];
+  if (!search_live(s) || !levels_small(s)) return;
+  const int P = s.P, B = s.B, tid = threadIdx.x;
+  const long long rp = stream_ptrs(s)[0], wp = stream_ptrs(s)[1];
+  if (!levels_apply(s, rp, wp)) return;
+  for (int m = tid; m < P; m += blockDim.x) owner[0][m] = owner[1][m] = 0x7fffffff;
+  const int base = int(rp % s.stream_capacity);
+  uint32_t cand[kClusterPer];
+  uint32_t pending = 0;
+#pragma unroll
+  for (int t = 0; t < kClusterPer; ++t) {
+    const int j = tid + t * kClusterThreads;
+    cand[t] = 0;
+    if (j < B) {
+      cand[t] = child_draws(s, base, j);
+      pending |= 1u << t;
+    }
+  }
+  __syncthreads();
+  int level = 0;
+  for (; level <= B; ++level) {
+    const int tag = (0x7fff - level) << 16;
+    int32_t* const claims = owner[level & 1];
+#pragma unroll
+    for (int t = 0; t < kClusterPer; ++t)
+      if (pending >> t & 1) {
+        atomicMin(&claims[cand[t] & 0xffff], tag | (tid + t * kClusterThreads));
+        atomicMin(&claims[cand[t] >> 16], tag | (tid + t * kClusterThreads));
+      }
+    if (!__syncthreads_or(pending != 0)) break;
+#pragma unroll
+    for (int t = 0; t < kClusterPer; ++t) {
+      const int mine = tag | (tid + t * kClusterThreads);
+      if ((pending >> t & 1) && claims[cand[t] & 0xffff] == mine && claims[cand[t] >> 16] == mine) {
+        s.child_level[tid + t * kClusterThreads] = int16_t(level);
+        pending &= ~(1u << t);
+      }
+    }
+  }
+  if (tid == 0) {
+    s.level_plan[1] = level;  // levels 0 .. level - 1 hold every child
+    s.level_plan[0] = s.round[0] + 1;
+  }
+}
+// In a cluster of kPlaceCtas blocks that share their shared memory, for the
+// others: member m's owner words live in block m % kPlaceCtas.
 __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThreads, 1)
     k_place_levels(const SearchDesc* descs, int n) {
   extern __shared__ __align__(16) int32_t lv_owner[];
@@ -1488,7 +1477,7 @@ __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThr
   const int P = s.P, B = s.B;
   const int tid = threadIdx.x, lane = tid & 31;
   const long long rp = stream_ptrs(s)[0], wp = stream_ptrs(s)[1];
-  if (!cluster_placement_applies(s, rp, wp)) return;
+  if (levels_small(s) || !levels_apply(s, rp, wp)) return;
   const int local_P = (P + kPlaceCtas - 1) / kPlaceCtas;
   for (int i = tid; i < 2 * local_P; i += blockDim.x) lv_owner[i] = 0x7fffffff;
   if (tid == 0) ready_count[0] = ready_count[1] = ready_count[2] = 0;
@@ -1511,7 +1500,8 @@ __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThr
   int* counter0 = cluster.map_shared_rank(ready_count, 0);
   int16_t* __restrict__ level_of = s.child_level;
   cluster.sync();
-  // one cluster barrier per level (count slots rotate as in k_place_cluster)
+  // one cluster barrier per level; three count slots rotate: a level adds to
+  // its own, reads the one before's and clears the next
   int left = B, level = 0;
   for (; level <= B; ++level) {
     const int tag = (0x7fff - level) << 16, par = level & 1;
@@ -1547,6 +1537,18 @@ __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThr
   cluster.sync();  // no block leaves while another may still read its shared memory
 }
 
+// Cluster placement: the level-parallel placement of place_round, spread over
+// a cluster of kPlaceCtas blocks that share their shared memory, for rounds
+// of at least kClusterMinChildren children.  Member m's key lives in block
+// m % kPlaceCtas; thread g of the cluster owns children [2g, 2g + 2), so the
+// blocks hold the children in order.  Each level is a cluster barrier after
+// the level's children have placed (remote key reads and writes).  The
+// running best before each child is a scan inside each block plus a prefix
+// over the blocks' totals.  When a child would have redrawn (place_state 2)
+// k_place replays the round on the exact path; another replacement size or a
+// stream short of draws is left to k_place (place_state 0).  On success this
+// kernel finishes the round as k_place does (best member, stream position,
+// next seed).
 __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThreads, 1)
     k_place_cluster(const SearchDesc* descs, int n) {
   extern __shared__ __align__(16) uint64_t cl_keys[];
@@ -1568,7 +1570,7 @@ __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThr
 #pragma unroll
   for (int t = 0; t < kClusterPer; ++t) kv[t] = begin + t < B ? s.c_key[begin + t] : ~0ULL;
   // the levels come from k_place_levels, run earlier in this round
-  if (!cluster_placement_applies(s, rp, wp) || s.level_plan[0] != s.round[0] + 1) {
+  if (B < kClusterMinChildren || !levels_apply(s, rp, wp) || s.level_plan[0] != s.round[0] + 1) {
     if (rank == 0 && tid == 0) *s.place_state = 0;
     return;  // the same decision in every block
   }
@@ -1684,23 +1686,6 @@ __global__ void __cluster_dims__(kPlaceCtas, 1, 1) __launch_bounds__(kClusterThr
     }
   cluster.sync();
   const bool done = redraw_at == 0x7fffffff;
-  if (done) {
-    // this block's members take their child's statistics
-    const double* __restrict__ cfit = s.c_fitness;
-    const uint32_t* __restrict__ cwrong = s.c_wrong;
-    const uint32_t* __restrict__ cnodes = s.c_nodes;
-    for (int i = tid; i < local_P; i += blockDim.x) {
-      const int m = i * kPlaceCtas + rank;
-      if (m >= P) continue;
-      const int c = placed[m];
-      if (c >= 0) {
-        s.key[m] = keys[i];
-        s.fitness[m] = cfit[c];
-        s.wrong[m] = cwrong[c];
-        s.nodes[m] = cnodes[c];
-      }
-    }
-  }
   if (rank == 0 && tid == 0) {
     *s.place_state = done ? 1 : 2;
     if (done) {
@@ -1831,7 +1816,15 @@ __global__ void k_commit(const SearchDesc* descs, const int32_t* off, int n) {
   int64_t* cto = s.cval + size_t(m) * s.stride;
   for (int i = lane; i < len_nodes(l); i += kCommitLanes) to[i] = from[i];
   for (int i = lane; i < len_consts(l); i += kCommitLanes) cto[i] = cfrom[i];
-  if (lane == 0) s.len[m] = l;
+  if (lane == 0) {
+    s.len[m] = l;
+    if (!s.generational) {  // k_gen_place has copied these
+      s.fitness[m] = s.c_fitness[b];
+      s.wrong[m] = s.c_wrong[b];
+      s.nodes[m] = s.c_nodes[b];
+      s.key[m] = s.c_key[b];
+    }
+  }
 }
 
 // ----------------------------------------------------------- generational
