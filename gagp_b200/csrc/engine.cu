@@ -1991,8 +1991,8 @@ gagp_status check_errors(gagp_engine* e, const std::vector<Search*>& list) {
 }
 
 // One round of a fixed batch captured as a CUDA graph (its fork/join over the
-// side and range streams included), so that a sequence of rounds costs one
-// graph launch each instead of ~30 stream operations.  The round's kernels
+// side and range streams included), so that rounds timed one by one
+// (batch_advance) are not timed with their launches.  The round's kernels
 // read everything that changes between rounds from device memory, so the
 // same graph serves every round of the batch.
 struct RoundGraph {
@@ -2015,34 +2015,29 @@ gagp_status capture_round(gagp_engine* e, const BatchView& v, RoundGraph* out) {
   if (made != cudaSuccess) return fail(GAGP_DEVICE_ERROR, std::string("round graph: ") + cudaGetErrorString(made));
   return GAGP_OK;
 }
-// `rounds` rounds of a batch: graph replays, or direct launches while
-// per-kernel timing is on (its events are recorded per launch).
+// `rounds` rounds of a batch, launched one after another: the host is ahead of
+// the device (10 to 40 stream operations a round), and instantiating a graph
+// of the round costs some 300 us for nothing in return -- 24 rounds of P = 777
+// 2.73 ms replayed, 2.40 launched; 50 generational rounds 9.65 and 8.93; 128
+// large scalar rounds 31.6 and 31.1; a served mix 98 and 85.
 gagp_status launch_rounds(gagp_engine* e, const BatchView& v, int rounds) {
   if (rounds <= 0) return GAGP_OK;
-  if (e->profiling || rounds == 1) {
-    for (int r = 0; r < rounds; ++r) {
-      const gagp_status st = launch_round(e, v);
-      if (st != GAGP_OK) return st;
-    }
-    return GAGP_OK;
-  }
   // an untuned batch shape times its VM candidates on the first rounds
   int r = 0;
-  while (r < rounds && e->vm_tune[vm_key(v.max_C, v.max_inputs)].chosen < 0 && r < 3 * kTuneRounds) {
-    const gagp_status st = launch_round(e, v);
-    if (st != GAGP_OK) return st;
-    ++r;
-  }
+  if (!e->profiling && rounds > 1)
+    while (r < rounds && e->vm_tune[vm_key(v.max_C, v.max_inputs)].chosen < 0 && r < 3 * kTuneRounds) {
+      const gagp_status st = launch_round(e, v);
+      if (st != GAGP_OK) return st;
+      ++r;
+    }
   if (r) {
     CUDA_TRY(cudaStreamSynchronize(e->stream));
     harvest(e);
   }
-  if (r >= rounds) return GAGP_OK;
-  RoundGraph g;
-  const gagp_status st = capture_round(e, v, &g);
-  if (st != GAGP_OK) return st;
-  for (; r < rounds; ++r) CUDA_TRY(cudaGraphLaunch(g.exec, e->stream));
-  CUDA_TRY(cudaStreamSynchronize(e->stream));  // the graph is destroyed on return
+  for (; r < rounds; ++r) {
+    const gagp_status st = launch_round(e, v);
+    if (st != GAGP_OK) return st;
+  }
   return GAGP_OK;
 }
 
