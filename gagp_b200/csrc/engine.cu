@@ -1812,6 +1812,8 @@ gagp_status launch_start(gagp_engine* e, const BatchView& v) {
   return cudaPeekAtLastError() == cudaSuccess ? GAGP_OK : fail(GAGP_DEVICE_ERROR, cudaGetErrorString(cudaGetLastError()));
 }
 
+// Rounds of at least this many children are split into ranges.
+constexpr int kRangedChildren = 4096;
 gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = true) {
   const VmPlan vm = plan_vm(e, v, may_measure);
   // the run-generator top-up overlaps everything up to the placement
@@ -1852,7 +1854,7 @@ gagp_status launch_round(gagp_engine* e, const BatchView& v, bool may_measure = 
   // of the variation warps; range c's accumulator list starts at item lo
   CUDA_TRY(cudaMemsetAsync(e->d_counts, 0, kCountWords * sizeof(int32_t), e->stream));
   CUDA_TRY(cudaEventRecord(e->chunk_fork, e->stream));
-  const int chunks = v.total_children >= 4096 ? gagp_engine::kChunks : 1;
+  const int chunks = v.total_children >= kRangedChildren ? gagp_engine::kChunks : 1;
   const int warps = 4;
   // a range whose children all belong to one search stages that search's
   // generator image in shared memory (when it is small enough to keep the
@@ -2015,11 +2017,16 @@ gagp_status capture_round(gagp_engine* e, const BatchView& v, RoundGraph* out) {
   if (made != cudaSuccess) return fail(GAGP_DEVICE_ERROR, std::string("round graph: ") + cudaGetErrorString(made));
   return GAGP_OK;
 }
-// `rounds` rounds of a batch, launched one after another: the host is ahead of
-// the device (10 to 40 stream operations a round), and instantiating a graph
-// of the round costs some 300 us for nothing in return -- 24 rounds of P = 777
-// 2.73 ms replayed, 2.40 launched; 50 generational rounds 9.65 and 8.93; 128
-// large scalar rounds 31.6 and 31.1; a served mix 98 and 85.
+// `rounds` rounds of a batch.  Most runs launch them one after another: the
+// host is ahead of the device (10 to 40 stream operations a round), and
+// instantiating a graph of the round costs some 300 us a run for nothing in
+// return -- 24 rounds of P = 777 2.73 ms replayed, 2.40 launched; 50
+// generational rounds of 8 ranges 9.65 and 8.93; a served mix 98 and 85.  Long
+// runs of rounds split into ranges replay one: where the process created its
+// context with the default 8 hardware queues, ranges launched from 11 streams
+// wait for one another (128 rounds of P = 16384 33.9 ms replayed, 36.3
+// launched; with 32 queues 33.4 and 33.0).
+constexpr int kReplayRounds = 64;
 gagp_status launch_rounds(gagp_engine* e, const BatchView& v, int rounds) {
   if (rounds <= 0) return GAGP_OK;
   // an untuned batch shape times its VM candidates on the first rounds
@@ -2033,6 +2040,14 @@ gagp_status launch_rounds(gagp_engine* e, const BatchView& v, int rounds) {
   if (r) {
     CUDA_TRY(cudaStreamSynchronize(e->stream));
     harvest(e);
+  }
+  if (!e->profiling && v.total_children >= kRangedChildren && rounds - r >= kReplayRounds) {
+    RoundGraph g;
+    const gagp_status st = capture_round(e, v, &g);
+    if (st != GAGP_OK) return st;
+    for (; r < rounds; ++r) CUDA_TRY(cudaGraphLaunch(g.exec, e->stream));
+    CUDA_TRY(cudaStreamSynchronize(e->stream));  // the graph is destroyed on return
+    return GAGP_OK;
   }
   for (; r < rounds; ++r) {
     const gagp_status st = launch_round(e, v);
