@@ -626,8 +626,7 @@ def run_batch_workload(args, rank: int, world: int):
     """Batching: 64 independent searches, half scalar regressions and half
     list programs (populations log-uniform 256..8192, 16..1000 cases, 64
     generations, seeds 0..63) run as one batch (one launch sequence per
-    round, rounds replayed from a CUDA graph) against the plain path (each
-    search alone, one after another)."""
+    round) against the plain path (each search alone, one after another)."""
     from gagp_b200 import build
     from gagp_b200.engine import Engine
     dist = init_ranks(world, rank_info()[2])

@@ -254,10 +254,10 @@ class Server:
 
     submit() queues a search; every step() admits queued requests in arrival
     order while their device bytes fit `memory_budget`, runs up to
-    `rounds_per_step` rounds of every running search in one batched launch
-    sequence (a captured round replayed) and retires the
-    finished ones; result() returns a finished request's history and final
-    population exactly as Search.result() does for the search run alone."""
+    `rounds_per_step` rounds of every running search, one batched launch
+    sequence each, and retires the finished ones; result() returns a finished
+    request's history and final population exactly as Search.result() does
+    for the search run alone."""
 
     def __init__(self, engine: Engine, memory_budget: int = 0, max_active: int = 0, rounds_per_step: int = 1):
         h = C.c_void_p()

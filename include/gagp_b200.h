@@ -307,7 +307,9 @@ gagp_status gagp_b200_search_progress(gagp_engine* engine, int32_t search, int32
  * that reused their parent's result, [2] evaluated (program, case) pairs,
  * [3] accumulator-VM instructions executed over all cases (added when a
  * program's last case tile finishes), [24] bytecode instructions the exact
- * VM executed (the reference's fuel consumed by those programs), [4..6] SM
+ * VM executed (the reference's instructions of those programs; a straight
+ * stretch counts as it is entered, so a case that fails may count the rest
+ * of its stretch), [4..6] SM
  * clock cycles of
  * the placement phases (stream generation, draw staging, placement),
  * [7] placement levels (+2^20 per sequential replay), [8] and [10..23]
@@ -421,8 +423,8 @@ gagp_status gagp_b200_server_create(gagp_engine* engine, uint64_t memory_budget,
                                     gagp_server** out);
 void gagp_b200_server_destroy(gagp_server* server);
 /* Rounds each step runs (1..4096, default 1) before it reads the searches'
- * states: the batch's round is captured once and replayed, and the host
- * reads states and retires searches once per step.  A search that finishes
+ * states: the host launches the rounds, then reads states and retires
+ * searches once per step.  A search that finishes
  * within a step waits for the step's end; results do not depend on it. */
 gagp_status gagp_b200_server_set_rounds_per_step(gagp_server* server, int32_t rounds);
 /* Queues a search request (the blobs are copied).  Declines at once what
