@@ -9,7 +9,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libgagp_b200.so")
 SOURCES = ["engine.cu"]
-HEADERS = ["search_state.h", "device_ops.cuh", "operators.cuh", "lower.cuh", "vm.cuh", "accumulator.cuh", "exact.cuh", "kernels.cuh"]
+HEADERS = ["search_state.h", "device_ops.cuh", "operators.cuh", "lower.cuh", "vm_choice.cuh", "vm.cuh", "accumulator.cuh", "exact.cuh", "kernels.cuh"]
 NVCC_FLAGS = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "-shared", "-diag-suppress", "550"]
 

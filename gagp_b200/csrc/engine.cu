@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "vm_choice.cuh"
 
 namespace {
 
@@ -794,73 +795,9 @@ std::vector<char> gen_image(const gagp_grammar* g, const std::vector<gb::ExprInf
   return img;
 }
 
-// Instructions (and constants) the lowering can emit for a row of at most
-// `maxv` nodes, the appended RETURN included: a leaf or operation emits 1, a
-// value if 2 (its jumps), and/or 5, and a traversal at most 36 of its own
-// beside its four children, so at most 8 per node of a row holding
-// traversals (36 + 4 children over 5 nodes).  A for_range emits 23 of its
-// own; its body's root is a block node that emits none and is no other
-// loop's body root, so at most 12 per node of a row holding loops.  A
-// bounded region emits its BOUNDED_REGION and at most 13 record
-// instructions beside at least five children: at most 3 per node.
-// Program, block and nil nodes emit nothing, an if_stmt 2 and an assign,
-// a return or a local read 1.
-int bytecode_bound(const gagp_grammar* g, int maxv) {
-  int per_node = 1;
-  for (int i = 0; i < g->expression_count; ++i) {
-    const int nk = g->expressions[i].node_kind;
-    if (g->expressions[i].kind == gb::EK_OPERATION)
-      per_node = std::max(per_node, nk == gb::TK_FOR_RANGE ? 12 : nk == gb::TK_TRAVERSE ? 8 : nk == gb::TK_REGION ? 3
-                                    : nk == gb::TK_IF ? 2
-                                    : (nk == gb::TK_AND || nk == gb::TK_OR) ? 5 : 1);
-  }
-  return per_node * maxv + 2;
-}
-
 // Instructions of a program's bytecode row, rounded so that a row also holds
 // register code in 16-byte words.
-int bytecode_stride(const gagp_grammar* g, int maxv) { return int(align_up(size_t(bytecode_bound(g, maxv)), 4)); }
-
-// Whether a grammar's programs mostly need the exact VM: it holds
-// traversals or bound reads, or operations that can raise a runtime error
-// (modulo and division by zero, list builtins).
-// Whether every instruction a program of `g` can emit costs one unit of
-// fuel: the accumulator VM's timeout proof counts instructions.
-bool unit_fuel(const gagp_grammar* g) {
-  if (g->return_fuel != 1) return false;
-  for (int r = 0; r < g->region_count; ++r)
-    if (g->regions[r].fuel_profile) return false;
-  for (int i = 0; i < g->expression_count; ++i)
-    if (g->expressions[i].fuel != 1 || g->expressions[i].merge_fuel != 1) return false;
-  return true;
-}
-
-bool exact_heavy(const gagp_grammar* g) {
-  if (gb::is_statement_tag(g->slot_type)) return true;  // statement programs run on the exact VM only
-  if (!unit_fuel(g)) return true;                       // so do programs with fuel charges other than 1
-  for (int i = 0; i < g->expression_count; ++i) {
-    const gagp_expression& e = g->expressions[i];
-    if (e.kind == gb::EK_BOUND) return true;
-    if (e.kind != gb::EK_OPERATION) continue;
-    if (e.node_kind == gb::TK_TRAVERSE) return true;
-    if (e.node_kind == gb::TK_OPERATION &&
-        gb::accumulator_op_of(e.node_kind, e.opcode, e.operand) == gb::A_COUNT)
-      return true;
-  }
-  return false;
-}
-
-// Whether any program of a grammar can need the exact VM.  A program of
-// accumulator operations goes there only when its bytecode may exceed the
-// fuel or when it needs more than kMaxTemps temporaries.  The fewest nodes of
-// a tree of need k are T(k) = 1 + min(2 T(k-1), 3 T(k-2)) (two children of
-// need k-1, or an if over three of need k-2), T(0) = 2, T(1) = 5: a seventh
-// temporary takes T(7) = 135 nodes.
-bool exact_possible(const gagp_grammar* g, int fuel) {
-  static_assert(gb::kMaxTemps == 6, "the node bound is the seventh temporary's");
-  const int maxv = g->max_nodes - g->fixed_nodes;
-  return exact_heavy(g) || maxv >= 135 || bytecode_bound(g, maxv) > fuel;
-}
+int bytecode_stride(const gagp_grammar* g, int maxv) { return int(align_up(size_t(gb::bytecode_bound(g, maxv)), 4)); }
 
 // Device copy of the traversal table.
 std::vector<gb::RegionInfo> region_infos(const gagp_grammar* g) {
@@ -1319,8 +1256,8 @@ gagp_status gagp_b200_search_create(gagp_engine* e, const gagp_grammar* g, const
   s->stride = p.stride;
   s->fixed_nodes = g->fixed_nodes;
   s->has_wrong = cfg->metric != GAGP_METRIC_LEGACY;
-  s->exact_heavy = exact_heavy(g);
-  s->exact_possible = exact_possible(g, cfg->fuel);
+  s->exact_heavy = gb::exact_heavy(g);
+  s->exact_possible = gb::exact_possible(g, cfg->fuel);
   s->region_words = 0;
   for (int r = 0; r < g->region_count; ++r)
     if (g->regions[r].traversal == 0)
@@ -1425,7 +1362,7 @@ gagp_status gagp_b200_search_create(gagp_engine* e, const gagp_grammar* g, const
   d.depth_count = g->depth_count; d.logical_count = g->logical_depth_count; d.site_depth = g->site_depth;
   d.root_expression = g->root_expression; d.slot_max_depth = g->slot_max_depth; d.slot_type = g->slot_type;
   d.result_type = result_type_of(g);
-  d.unit_fuel = unit_fuel(g) ? 1 : 0;
+  d.unit_fuel = gb::unit_fuel(g) ? 1 : 0;
   d.local_count = g->local_count; d.max_nodes = g->max_nodes; d.fixed_nodes = g->fixed_nodes;
   d.return_fuel = g->return_fuel;
   d.P = s->P; d.B = s->B; d.maxv = s->maxv; d.stride = p.stride;
@@ -2266,7 +2203,7 @@ gagp_status eval_rows_in(char* region, char* staging, const EvalStaging& sz, con
   d.n_ex = E;
   d.slot_type = g->slot_type;
   d.result_type = result_type_of(g);
-  d.unit_fuel = unit_fuel(g) ? 1 : 0;
+  d.unit_fuel = gb::unit_fuel(g) ? 1 : 0;
   d.local_count = g->local_count;
   d.max_nodes = g->max_nodes;
   d.fixed_nodes = g->fixed_nodes;
@@ -2323,7 +2260,7 @@ gagp_status eval_rows_in(char* region, char* staging, const EvalStaging& sz, con
   const gb::LowerLists lists{fast, at<gb::ProgramRef>(b, p.exact), at<gb::ProgramRef>(b, p.general),
                              at<gb::ProgramRef>(b, p.region_list), R, counts, counts + 1, counts + 2, counts + 3,
                              counts + 4};
-  const bool exact = exact_possible(g, cfg->fuel);
+  const bool exact = gb::exact_possible(g, cfg->fuel);
   lower_launch(stream, dd, doff, 1, 0, lists, 0, R, exact);
   const int warps = 8;
   const int lanes = d.vm_cases_per_lane;

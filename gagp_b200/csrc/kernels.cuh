@@ -109,7 +109,7 @@ struct LowerLists {
 // the accumulator program when the row is total and fits the fuel, else
 // register code for the exact VM, else the reference bytecode (lane 0).
 // Exact false: no program of the batch can need the exact VM
-// (exact_possible in the engine), so the other lowerings, with their shared
+// (exact_possible in vm_choice.cuh), so the other lowerings, with their shared
 // memory and local arrays, stay out of the kernel and a row the accumulator
 // lowering rejects is one the reference's compiler rejects too.
 // Rows a block: a block's slowest row keeps its place, so without the exact

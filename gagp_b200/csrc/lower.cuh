@@ -1012,6 +1012,17 @@ __host__ __device__ __forceinline__ uint32_t accumulator_op_of(int node_kind, in
   }
 }
 
+// Whether an accumulator program can hold a node: a leaf that is a constant or
+// an Int/Bool input (a bound read, of a traversal's binder say, needs the exact
+// VM), or an operation with an accumulator operation.
+__host__ __device__ __forceinline__ bool accumulator_leaf(int node_kind) {
+  return node_kind == TK_CONSTANT || node_kind == TK_LOCAL;
+}
+__host__ __device__ __forceinline__ bool accumulator_takes(int node_kind, int opcode, int operand, int arity) {
+  return arity == 0 ? accumulator_leaf(node_kind)
+                    : arity <= 3 && accumulator_op_of(node_kind, opcode, operand) != A_COUNT;
+}
+
 // Accumulator program of a row, by one warp; returns the instruction count
 // (the same on every lane), or -1 when the row needs the exact VM.
 // *temps_out: temporaries used.  The lanes classify the nodes, number the
@@ -1037,9 +1048,7 @@ __device__ inline int lower_accumulator_warp(const SearchDesc& s, const uint64_t
       m.arity[i] = uint8_t(arity);
       if (arity == 0) {
         m.aop[i] = kLeafOp;
-        // the accumulator VM reads constants and Int/Bool inputs; a bound
-        // read (a traversal binder) needs the exact VM
-        total &= nk == TK_CONSTANT || nk == TK_LOCAL;
+        total &= accumulator_leaf(nk);
       } else {
         const uint32_t op = accumulator_op_of(nk, __ldg(&info[o].opcode), __ldg(&info[o].operand));
         m.aop[i] = uint8_t(op);
