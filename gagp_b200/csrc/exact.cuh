@@ -452,7 +452,8 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
             break;
           }
           case N_FOR:
-            bad |= is_statement_tag(type_of(i + 1)) || !is_statement_tag(type_of(child(i, 1)));
+            // a bound that is no Int fails at run time too (the bytecode's is_int)
+            bad |= type_of(i + 1) != GAGP_TAG_INT || !is_statement_tag(type_of(child(i, 1)));
             break;
           default: break;
         }

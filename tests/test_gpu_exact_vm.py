@@ -125,3 +125,38 @@ def test_long_programs(engine, cases):
     want_f, want_w, _ = oracle.evaluate(blob, lt.cases, lt.settings, rows)
     assert np.array_equal(got_f, want_f)
     assert np.array_equal(got_w, want_w)
+
+
+def _statement(lt, name, kind, operand=None):
+    """The first expression of a printed name and tree kind (and target)."""
+    return next(i for i, e in enumerate(lt.tables.expressions)
+                if lt.tables.names[i] == name and e.node_kind == kind and operand in (None, e.operand))
+
+
+def test_loop_bounds_that_are_no_int(engine):
+    """A for_range over a Bool fails the case that reaches it, as the
+    bytecode's is_int test does; rows to be scored need not derive from the
+    grammar, so they can hold one."""
+    lt = T.from_files(W.list_statements(population=64, generations=2, seed=4, cases=70))
+    blob = abi.GrammarBlob(lt.tables)
+    at = lambda name, kind, operand=None: _statement(lt, name, kind, operand)  # noqa: E731
+    main, cons, nil = at("program", G.TK_PROGRAM), at("block_cons", G.TK_BLOCK), at("block_nil", G.TK_NIL)
+    acc_is, ret, var = at("assign", G.TK_ASSIGN, 0), at("return", G.TK_RETURN), at("var", G.TK_VAR, 0)
+    loop, when, gt = at("for_range", G.TK_FOR_RANGE), at("if_stmt", G.TK_IF), at("gt", G.TK_OPERATION)
+    t = next(i for i, e in enumerate(lt.tables.expressions) if e.kind == G.EK_INPUT and lt.tables.names[i] == "t")
+    one = next(i for i, e in enumerate(lt.tables.expressions) if e.kind == G.EK_CONSTANT)
+    add = at("add", G.TK_OPERATION)
+    positive = [gt, t, one]
+    body = [cons, acc_is, add, var, one, nil]
+    begin, end = [main, cons, acc_is, one], [cons, ret, var, nil]
+    rows = [(begin + [cons, loop] + positive + body + end, [5, 0, 1]),        # every case reaches the Bool bound
+            (begin + [cons, loop, t] + body + end, [5, 1]),                    # an Int bound, negative ones fail
+            (begin + [cons, when] + positive + [cons, loop] + positive + body + [nil, nil] + end, [5, 0, 0, 1])]
+    programs = [H.lower(blob, *r) for r in rows]
+    buffer = abi.RowsBuffer.from_rows(rows, lt.tables.max_nodes - lt.tables.fixed_nodes)
+    got_f, got_w = engine.evaluate_rows(lt, buffer)
+    want_f, want_w = _expected(lt, buffer, programs, lt.settings.fuel)
+    assert want_w[0] == 70 and want_f[0] < min(want_f[1:])
+    assert list(got_f) == want_f
+    assert list(got_w) == want_w
+    assert [v["runtime_errors"] for v in engine.judge_rows(lt, buffer, lt.cases)][0] == 70
