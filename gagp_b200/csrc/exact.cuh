@@ -172,7 +172,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   const int n_inputs = s.local_count;
   if (n_inputs > kExactSlots || s.return_fuel > 0xffu) return -1;
   bool bad = false;
-  int named = 0;
+  int named = 0, lets = 0;
   // ---- classes, charges, open slots
   {
     const bool unit = s.unit_fuel;
@@ -260,6 +260,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
           bad |= arity != want || int8_t(raw.x >> 16) != arity;
         }
         bad |= kind == N_BAD;
+        lets += kind == N_LET;
         m.kind[i] = kind;
         m.aux[i] = aux;
         m.flags[i] = flags;
@@ -278,6 +279,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
     bad |= open != 0 || seen > uint32_t(nc);
   }
   named = __reduce_max_sync(kFull, named);
+  lets = int(__reduce_add_sync(kFull, unsigned(lets)));
   if (__any_sync(kFull, bad)) return -1;
   __syncwarp();
   const int base_slot = n_inputs + named;
@@ -624,6 +626,25 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
     if (m.kind[i] == N_TRAVERSE) own = 5 + int(!alias(i + 1)) + int(!alias(m.end[i + 1]));
     else if (m.kind[i] == N_FOR) own = 2;
     top = max(top, held + own);
+  }
+  // The reference's compiler refuses a row with more open lets or live locals
+  // than its tables hold.  A let's value holds none of these slots while it
+  // runs, so of lets a row can nest more than that; the open traversals and
+  // loops are bounded by the slots (5 T + 2 F + inputs and locals <= 32), and
+  // what the compiler holds for them by 32 + 4 T <= 56 of its 64 locals, so
+  // up to 8 lets fit without counting.
+  static_assert(kExactSlots == 32 && kLowerLocals == 64 && kLowerLets >= 8, "rows of few lets are not counted");
+  if (lets > 8) {
+#pragma unroll 1
+    for (int i = lane; i < n; i += 32) {
+      int open = 0, locals = base_slot;
+      for (int x = m.par[i], child_of = i; child_of > 0; child_of = x, x = m.par[x]) {
+        const uint8_t kind = m.kind[x];
+        open += kind == N_LET;
+        locals += kind == N_LET ? 1 : kind == N_TRAVERSE ? 9 : kind == N_FOR ? 2 : 0;
+      }
+      bad |= open > kLowerLets || locals > kLowerLocals;
+    }
   }
   const int const_base = base_slot + __reduce_max_sync(kFull, top);
   const int length_base = const_base + const_count, slots = length_base + __popc(kept);

@@ -160,3 +160,65 @@ def test_loop_bounds_that_are_no_int(engine):
     assert list(got_f) == want_f
     assert list(got_w) == want_w
     assert [v["runtime_errors"] for v in engine.judge_rows(lt, buffer, lt.cases)][0] == 70
+
+
+@pytest.mark.parametrize("nested", ["value", "body"])
+@pytest.mark.parametrize("lets", [8, 9, 16, 17])
+def test_open_lets(engine, nested, lets):
+    """Rows of nested lets score up to the reference compiler's 16 open lets
+    and are refused past them, also where their slots would fit."""
+    with gzip.open(os.path.join(LOWER_DIR, "lower_scalar_let.json.gz"), "rt") as f:
+        fx = json.load(f)
+    lt = GU.load_task(fx)
+    blob = abi.GrammarBlob(lt.tables)
+    ex = lt.tables.expressions
+    let = next(i for i, e in enumerate(ex) if e.kind == G.EK_OPERATION and e.node_kind == G.TK_LET)
+    read = next(i for i, e in enumerate(ex) if e.kind == G.EK_BOUND)
+    add = next(i for i, e in enumerate(ex) if e.kind == G.EK_OPERATION and lt.tables.names[i] == "add")
+    x = next(i for i, e in enumerate(ex) if e.kind == G.EK_INPUT)
+    row = ([let] * lets + [x] + [read] * lets if nested == "value" else [let, x] * lets + [read], [])
+    program = H.lower(blob, *row)
+    assert (program is None) == (lets > 16)
+    buffer = abi.RowsBuffer.from_rows([row], lt.tables.max_nodes - lt.tables.fixed_nodes)
+    if program is None:
+        with pytest.raises(Exception, match="row evaluation failed"):
+            engine.evaluate_rows(lt, buffer)
+        return
+    got_f, got_w = engine.evaluate_rows(lt, buffer)
+    want_f, want_w = _expected(lt, buffer, [program], lt.settings.fuel)
+    assert list(got_f) == want_f
+    assert list(got_w) == want_w
+
+
+@pytest.mark.parametrize("lets", [9, 15, 16])
+def test_live_locals(engine, lets):
+    """Lets nested in one another's values inside five traversals over four
+    inputs: the row is refused past the compiler's 64 live locals (nine a
+    traversal, one a let), also where its slots would fit."""
+    with gzip.open(os.path.join(LOWER_DIR, "lower_list_let.json.gz"), "rt") as f:
+        fx = json.load(f)
+    fx["grammar"]["search_limits"]["max_nodes"] = 70
+    for name in ("u", "v"):
+        fx["grammar"]["inputs"].append({"name": name, "type": "Int"})
+        for case in fx["train"] + fx["test"]:
+            case["inputs"][name] = {"type": "int", "value": 1}
+    lt = GU.load_task(fx)
+    blob = abi.GrammarBlob(lt.tables)
+    ex, names = lt.tables.expressions, lt.tables.names
+    let, walk = (next(i for i, e in enumerate(ex) if e.kind == G.EK_OPERATION and e.node_kind == kind)
+                 for kind in (G.TK_LET, G.TK_TRAVERSE))
+    xs, t = (next(i for i, e in enumerate(ex) if e.kind == G.EK_INPUT and names[i] == name) for name in ("xs", "t"))
+    read = next(i for i, e in enumerate(ex) if e.kind == G.EK_BOUND and e.operand == ex[let].operand)
+    row = ([walk, xs, t, t] * 5 + [let] * lets + [t] + [read] * lets, [])
+    program = H.lower(blob, *row)
+    assert (program is None) == (4 + 45 + lets > 64)
+    buffer = abi.RowsBuffer.from_rows([row], lt.tables.max_nodes - lt.tables.fixed_nodes)
+    if program is None:
+        with pytest.raises(Exception, match="row evaluation failed"):
+            engine.evaluate_rows(lt, buffer)
+        return
+    lt.settings.fuel = 600  # some cases finish their nested loops
+    got_f, got_w = engine.evaluate_rows(lt, buffer)
+    want_f, want_w = _expected(lt, buffer, [program], lt.settings.fuel)
+    assert list(got_f) == want_f
+    assert list(got_w) == want_w
