@@ -129,7 +129,10 @@ struct gagp_engine {
   // stream-ordered pool of the searches' device blocks: admission and
   // retirement neither allocate from the driver nor synchronize the device
   cudaMemPool_t pool = nullptr;
-  // pinned staging of result downloads and row evaluations (grown on demand)
+  // pinned staging of result downloads and row evaluations (grown on demand);
+  // host threads may evaluate rows on one engine at the same time, so its
+  // user holds the mutex until its copies are done
+  std::mutex pinned_mutex;
   char* pinned = nullptr;
   size_t pinned_bytes = 0;
   // VM autotuner: per batch shape, the fast VM's cases per lane, chosen by
@@ -890,8 +893,9 @@ Plan plan_search(const gagp_grammar* g, const gagp_cases* c, const gagp_search_c
   return p;
 }
 
-// The engine's pinned staging, grown to `bytes`.  Nothing is in flight in it:
-// every user waits for its copies before it returns.
+// The engine's pinned staging, grown to `bytes`.  The caller holds its mutex.
+// Nothing is in flight in it: every user waits for its copies before it
+// returns.
 gagp_status pinned_at_least(gagp_engine* e, size_t bytes) {
   if (bytes <= e->pinned_bytes) return GAGP_OK;
   if (e->pinned) cudaFreeHost(e->pinned);
@@ -2455,7 +2459,8 @@ static gagp_status batch_advance_body(gagp_engine* e, const int32_t* ids, int32_
 // Row evaluation in a block of the engine's pool with its pinned staging.
 // Past the two limits the block is allocated and freed for the call alone,
 // and the staging is pageable: the engine keeps no more than these for row
-// evaluation, and at that size an allocation is small next to the work.
+// evaluation, and at that size an allocation is small next to the work.  The
+// staging is pageable too while another thread has the pinned one.
 constexpr size_t kEvalPoolBytes = size_t(256) << 20, kEvalPinnedBytes = size_t(64) << 20;
 
 static gagp_status eval_rows_on(gagp_engine* e, const gagp_grammar* grammar, const gagp_cases* cases,
@@ -2465,7 +2470,8 @@ static gagp_status eval_rows_on(gagp_engine* e, const gagp_grammar* grammar, con
   const EvalStaging sz = eval_staging(p, rows);
   std::unique_ptr<char[]> pageable;
   char* staging = nullptr;
-  if (sz.bytes <= kEvalPinnedBytes) {
+  std::unique_lock<std::mutex> mine(e->pinned_mutex, std::defer_lock);
+  if (sz.bytes <= kEvalPinnedBytes && mine.try_lock()) {
     if (const gagp_status st = pinned_at_least(e, sz.bytes); st != GAGP_OK) return st;
     staging = e->pinned;
   } else {
@@ -2681,6 +2687,7 @@ gagp_status gagp_b200_search_result(gagp_engine* e, int32_t id, gagp_search_resu
                o_hl = L.take(4 * size_t(H)), o_fit = L.take(8 * size_t(P)), o_wr = L.take(4 * size_t(P)),
                o_nodes = L.take(4 * size_t(P)), o_nc = L.take(4 * size_t(P)), o_cc = L.take(4 * size_t(P)),
                o_org = L.take(4 * size_t(P) * W), o_con = L.take(8 * size_t(P) * W), o_cnt = L.take(8 * 4);
+  const std::lock_guard<std::mutex> mine(e->pinned_mutex);
   if (const gagp_status st = pinned_at_least(e, L.total); st != GAGP_OK) return st;
   char* hb = e->pinned;
   auto fetch = [&](size_t off, const void* src, size_t bytes) -> cudaError_t {

@@ -79,3 +79,44 @@ def test_verdict_summaries_match_one_by_one():
     got = abi.verdict_summaries(out, 2)
     assert got == [out[0].summary(), out[1].summary()]
     assert [type(x) for x in got[0].values()] == [type(x) for x in out[0].summary().values()]
+
+
+@pytest.mark.gpu
+def test_rows_from_several_threads(tmp_path):
+    """Host threads that evaluate and judge rows on one engine at the same
+    time, calls of unequal sizes (the engine's staging grows meanwhile), while
+    another reads a search's result: every call gets its own rows' scores."""
+    from concurrent.futures import ThreadPoolExecutor
+    from gagp_b200.engine import Engine
+    lt = _task(tmp_path, population=512, seed=33, cases=40)
+    blob = abi.GrammarBlob(lt.tables)
+    rows = oracle.initial_population(blob, lt.settings)
+    want_f, want_w, _ = oracle.evaluate(blob, lt.cases, lt.settings, rows)
+    rng = np.random.default_rng(5)
+    picks = [rng.integers(0, 512, size=size) for size in (3, 4000, 17, 900, 12000, 64, 2500, 5)]
+
+    def evaluate(pick):
+        out = []
+        for _ in range(8):
+            f, w = engine.evaluate_rows(lt, _take(rows, pick))
+            out.append(np.array_equal(f, want_f[pick]) and np.array_equal(w, want_w[pick]))
+        return all(out)
+
+    def judge(pick):
+        taken = _take(rows, pick)
+        return all([v["wrong"] for v in engine.judge_rows(lt, taken, lt.cases)] == list(want_w[pick])
+                   for _ in range(8))
+
+    with Engine(0) as engine:
+        s = engine.admit(lt)
+        s.run()
+        want = s.result()
+
+        def read(_):
+            return all(s.result() == want for _ in range(8))
+
+        with ThreadPoolExecutor(len(picks) + 1) as pool:
+            jobs = [pool.submit(judge if i % 3 == 2 else evaluate, pick) for i, pick in enumerate(picks)]
+            jobs.append(pool.submit(read, None))
+            assert all(job.result() for job in jobs)
+        s.close()
