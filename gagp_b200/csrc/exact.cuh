@@ -145,13 +145,16 @@ __device__ __forceinline__ uint32_t warp_prefix(uint32_t v, uint32_t* total) {
 }
 
 // Register code of a row, by one warp; the instruction count (the same on
-// every lane), or -1 when the row takes the reference bytecode instead.
+// every lane), or negative when the row takes the reference bytecode instead.
 // words: [0] instructions | constants << 16, first constant slot, the list
 // inputs whose lengths follow the constants, slots; the instructions follow,
 // and one more word may be read past the last.  An IntList input's length
 // is read often (a loop bound, every index) and changes only when the program
 // assigns the input, so programs that do not keep it in a slot, loaded with
-// the inputs, and len of that input is an operand.
+// the inputs, and len of that input is an operand.  `keep` false: no length
+// is kept, for a row that fits the slots without them (kTooManySlots: this row
+// may be one); 2000 programs of a fold and 11 lengths over 12 list inputs and
+// 200 cases took 6.3 ms a call on the interpreter and take 2.0 this way.
 //
 // What bounds it: latency (a chain of shared-memory passes over the nodes, a
 // pass per question; about 40k cycles beside a full round's other warps).
@@ -163,9 +166,10 @@ __device__ __forceinline__ uint32_t warp_prefix(uint32_t v, uint32_t* total) {
 // is kept in shared memory, which took the walk from 143 to 47 us (selects
 // cost it 14 us more, taking what words share out of the per-class code gave
 // 10 back).
+constexpr int kTooManySlots = -2;
 __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t* node, int n, const int64_t* cval,
                                              int nc, uint4* words, int word_cap, int64_t* consts, ExactScratch& m,
-                                             int* slots_out) {
+                                             bool keep, int* slots_out) {
   const int lane = threadIdx.x & 31;
   if (n <= 0 || n > kMaxLowerNodes) return -1;
   const bool statements = is_statement_tag(s.slot_type);
@@ -483,7 +487,7 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
           m.kind[i + 1] == N_SLOT && m.aux[i + 1] < n_inputs)
         read |= 1u << m.aux[i + 1];
     }
-    kept = __reduce_or_sync(kFull, read) & ~__reduce_or_sync(kFull, assigned);
+    kept = keep ? __reduce_or_sync(kFull, read) & ~__reduce_or_sync(kFull, assigned) : 0u;
   }
   auto kept_length = [&](int i) -> bool { return m.kind[i] == N_SLOT && m.aux[i] < n_inputs && (kept >> m.aux[i] & 1u); };
   __syncwarp();
@@ -648,7 +652,8 @@ __device__ __noinline__ int lower_exact_warp(const SearchDesc& s, const uint64_t
   }
   const int const_base = base_slot + __reduce_max_sync(kFull, top);
   const int length_base = const_base + const_count, slots = length_base + __popc(kept);
-  if (slots > kExactSlots || __any_sync(kFull, bad)) return -1;
+  if (__any_sync(kFull, bad)) return -1;
+  if (slots > kExactSlots) return kept ? kTooManySlots : -1;
   __syncwarp();
   // ---- every node writes its words
   uint4* out = words + 1;

@@ -189,8 +189,11 @@ __global__ void __launch_bounds__(kLowerWarps<Exact> * 32, Exact ? 14 : 32)
       int32_t* bc = s.bc + size_t(slot) * 5 * s.bc_stride;
       int64_t* bc_consts = s.bc_consts + size_t(slot) * s.bc_stride;
       int slots = 0;
-      const int exact = lower_exact_warp(s, t.node, t.n, t.cval, t.nc, reinterpret_cast<uint4*>(bc),
-                                         s.bc_stride * 5 / 4, bc_consts, scratch[warp].exact, &slots);
+      int exact = kTooManySlots;
+#pragma unroll 1
+      for (int keep = 1; keep >= 0 && exact == kTooManySlots; --keep)
+        exact = lower_exact_warp(s, t.node, t.n, t.cval, t.nc, reinterpret_cast<uint4*>(bc), s.bc_stride * 5 / 4,
+                                 bc_consts, scratch[warp].exact, keep, &slots);
       if (lane == 0) {
         if (exact >= 0) {
           const int at = slots <= kExactNarrow ? atomicAdd(lists.exact_count, 1)

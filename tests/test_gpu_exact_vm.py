@@ -222,3 +222,38 @@ def test_live_locals(engine, lets):
     want_f, want_w = _expected(lt, buffer, [program], lt.settings.fuel)
     assert list(got_f) == want_f
     assert list(got_w) == want_w
+
+
+@pytest.mark.parametrize("lists", [7, 8, 9, 12, 15, 16, 30])
+def test_programs_of_many_list_inputs(engine, lists):
+    """A fold whose step adds the lengths of every other list input: with and
+    without slots for the lengths, and past the slots altogether."""
+    files = W.list_threshold(population=64, generations=2, seed=6, cases=40, max_nodes=100)
+    grammar = copy.deepcopy(files.grammar)
+    others = [f"y{j}" for j in range(lists - 1)]
+    grammar["inputs"] += [{"name": y, "type": "IntList"} for y in others]
+    step = next(nt for nt in grammar["nonterminals"] if nt["id"] == "Step")
+    step["alternatives"] += [{"id": "len_" + y, "weight": 1,
+                              "expression": {"signature": "len(IntList)->Int", "args": [{"input": y}]}} for y in others]
+    for k, case in enumerate(files.train):
+        for j, y in enumerate(others):
+            case["inputs"][y] = {"type": "int_list", "value": list(range((k * (j + 2)) % 7))}
+    files.grammar = grammar
+    lt = T.from_files(files)
+    blob = abi.GrammarBlob(lt.tables)
+    ex, names = lt.tables.expressions, lt.tables.names
+    at = lambda name, kind: next(i for i, e in enumerate(ex) if names[i] == name and e.kind == kind)  # noqa: E731
+    length, add = at("len", G.EK_OPERATION), at("add", G.EK_OPERATION)
+    body = [at("acc", G.EK_BOUND), at("element", G.EK_BOUND)]
+    for y in others:
+        body = [add] + body + [length, at(y, G.EK_INPUT)]
+    row = ([at("traverse", G.EK_OPERATION), at("xs", G.EK_INPUT), at("const", G.EK_CONSTANT), at("t", G.EK_INPUT),
+            add] + body, [0])
+    program = H.lower(blob, *row)
+    buffer = abi.RowsBuffer.from_rows([row], lt.tables.max_nodes - lt.tables.fixed_nodes)
+    for fuel in (200, lt.settings.fuel):
+        lt.settings.fuel = fuel
+        got_f, got_w = engine.evaluate_rows(lt, buffer)
+        want_f, want_w = _expected(lt, buffer, [program], fuel)
+        assert list(got_f) == want_f
+        assert list(got_w) == want_w
