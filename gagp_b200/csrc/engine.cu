@@ -2456,11 +2456,12 @@ static gagp_status batch_advance_body(gagp_engine* e, const int32_t* ids, int32_
   return st;
 }
 
-// Row evaluation in a block of the engine's pool with its pinned staging.
-// Past the two limits the block is allocated and freed for the call alone,
-// and the staging is pageable: the engine keeps no more than these for row
-// evaluation, and at that size an allocation is small next to the work.  The
-// staging is pageable too while another thread has the pinned one.
+// Row evaluation in a block of the engine's pool with its pinned staging, by
+// one thread at a time: a call that finds another thread's under way, or that
+// is past the two limits, allocates its block for itself and stages in
+// pageable memory (at that size an allocation is small next to the work).  So
+// does one whose block would not fit the arena limit next to the resident
+// searches: the pool keeps the block for later calls and admissions.
 constexpr size_t kEvalPoolBytes = size_t(256) << 20, kEvalPinnedBytes = size_t(64) << 20;
 
 static gagp_status eval_rows_on(gagp_engine* e, const gagp_grammar* grammar, const gagp_cases* cases,
@@ -2471,14 +2472,15 @@ static gagp_status eval_rows_on(gagp_engine* e, const gagp_grammar* grammar, con
   std::unique_ptr<char[]> pageable;
   char* staging = nullptr;
   std::unique_lock<std::mutex> mine(e->pinned_mutex, std::defer_lock);
-  if (sz.bytes <= kEvalPinnedBytes && mine.try_lock()) {
+  const bool first = mine.try_lock();
+  if (first && sz.bytes <= kEvalPinnedBytes) {
     if (const gagp_status st = pinned_at_least(e, sz.bytes); st != GAGP_OK) return st;
     staging = e->pinned;
   } else {
     pageable.reset(new (std::nothrow) char[sz.bytes]);
     if (!(staging = pageable.get())) return fail(GAGP_OUT_OF_MEMORY, "host staging of a row evaluation");
   }
-  const bool pooled = p.L.total <= kEvalPoolBytes;
+  const bool pooled = first && p.L.total <= kEvalPoolBytes && e->arena_used + p.L.total <= e->arena_limit;
   char* region = nullptr;
   if (pooled) CUDA_TRY(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&region), p.L.total, e->pool, e->stream));
   else CUDA_TRY(cudaMalloc(&region, p.L.total));

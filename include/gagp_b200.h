@@ -253,7 +253,9 @@ const char* gagp_b200_last_error(void);
 const char* gagp_b200_version(void);
 
 /* Creates the engine on `device`. `arena_bytes` bounds the device memory the
- * engine may hold for resident searches (0: 80% of free memory). */
+ * engine may hold for resident searches, and for row evaluations between calls
+ * (0: 80% of free memory); a row evaluation past it allocates its device
+ * memory for the call alone. */
 gagp_status gagp_b200_engine_create(int32_t device, uint64_t arena_bytes, gagp_engine** out);
 void gagp_b200_engine_destroy(gagp_engine* engine);
 

@@ -120,3 +120,22 @@ def test_rows_from_several_threads(tmp_path):
             jobs.append(pool.submit(read, None))
             assert all(job.result() for job in jobs)
         s.close()
+
+
+@pytest.mark.gpu
+def test_rows_past_the_arena_limit(tmp_path):
+    """An engine that may hold 8 MiB evaluates 20,000 rows (some 120 MiB on the
+    device) and keeps none of it afterwards."""
+    import torch
+    from gagp_b200.engine import Engine
+    lt = _task(tmp_path, population=512, seed=34, cases=20)
+    rows = oracle.initial_population(abi.GrammarBlob(lt.tables), lt.settings)
+    want_f, want_w, _ = oracle.evaluate(abi.GrammarBlob(lt.tables), lt.cases, lt.settings, rows)
+    index = np.arange(20000) % 512
+    with Engine(0, arena_bytes=8 << 20) as engine:
+        engine.evaluate_rows(lt, _take(rows, np.arange(9)))  # the kernels are loaded
+        before = torch.cuda.mem_get_info(0)[0]
+        f, w = engine.evaluate_rows(lt, _take(rows, index))
+        held = before - torch.cuda.mem_get_info(0)[0]
+    assert np.array_equal(f, want_f[index]) and np.array_equal(w, want_w[index])
+    assert held <= 16 << 20, held
