@@ -100,14 +100,6 @@ struct Rng {
     state = d.state;
     return d.value;
   }
-  __device__ __forceinline__ int64_t integer(int64_t lo, int64_t hi) {
-    const uint64_t sign = 1ULL << 63;
-    const uint64_t first = uint64_t(lo) ^ sign, last = uint64_t(hi) ^ sign;
-    const uint64_t width = last - first + 1;
-    const uint64_t bits = (first + (width ? bounded(width) : next())) ^ sign;
-    if (bits < sign) return int64_t(bits);
-    return INT64_MIN + int64_t(bits - sign);
-  }
   // bounded(upper) for a fixed upper with its rejection bound
   // ((2^64 - upper) mod upper) and magic floor((2^64 - 1) / upper) given:
   // the residue comes from a multiply-high quotient estimate, at most two
@@ -161,11 +153,6 @@ __host__ __device__ __forceinline__ uint64_t w_with_site(uint64_t w, uint64_t si
 __host__ __device__ __forceinline__ int len_nodes(int32_t l) { return l & 0xffff; }
 __host__ __device__ __forceinline__ int len_consts(int32_t l) { return (l >> 16) & 0xffff; }
 __host__ __device__ __forceinline__ int32_t make_len(int n, int c) { return n | (c << 16); }
-
-// Crossover class of sites opened by reference expression `entry`.
-__device__ __forceinline__ uint32_t class_of_entry(const SearchDesc& s, int entry) {
-  return entry < 0 ? kNoClass : uint32_t(s.info[entry].site_class);
-}
 
 // Definite assignment of grammar locals in a statement program
 // (phase_locals_defined, cpp/src/evolution/repro/gpu/device/phase_compile.cuh:170-200):

@@ -1027,13 +1027,10 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
   for (int m = tid; m < P; m += blockDim.x) keys[m] = s.key[m];
   for (int i = tid; i < 312; i += blockDim.x) mt[i] = s.mt[i];
   __syncthreads();
-  constexpr int kPerThread = Per;
-  constexpr bool kKeep = Per <= 4;  // the children's keys stay in registers
-  uint64_t kept[kKeep ? Per : 1];
-  if constexpr (kKeep) {
+  static_assert(Per == 1 || Per == 4, "draws and levels are read in pairs and fours");
+  uint64_t kept[Per];  // the children's keys
 #pragma unroll
-    for (int t = 0; t < Per; ++t) kept[t] = tid * Per + t < B ? s.c_key[tid * Per + t] : ~0ULL;
-  }
+  for (int t = 0; t < Per; ++t) kept[t] = tid * Per + t < B ? s.c_key[tid * Per + t] : ~0ULL;
   const long long rp = stream_ptrs(s)[0];
   long long wp = stream_ptrs(s)[1];
   const long long need = (long long)B * rs + 1;
@@ -1050,20 +1047,14 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
   int16_t* const on = reinterpret_cast<int16_t*>(stage);
   const int after = dyn_bytes - int(sizeof(uint64_t)) * (P + 1) - 64;
   const bool parallel_path = !replay && levels_apply(s, rp, wp) && s.level_plan[0] == s.round[0] + 1 &&
-                             blockDim.x == kPlaceThreads && B <= kPlaceThreads * kPerThread &&
+                             blockDim.x == kPlaceThreads && B <= kPlaceThreads * Per &&
                              after >= int(sizeof(int16_t)) * max(P, 2 * B);
   bool parallel_done = false;
   if (parallel_path) {
-    // thread tid owns children [16 tid, 16 tid + 16): cand[t] holds child
+    // thread tid owns children [Per tid, Per tid + Per): cand[t] holds child
     // begin + t's two draws, and once it is placed, its victim
     const int base = int(rp % cap);
-    const int begin = tid * kPerThread;
-    constexpr int kBatch = kPerThread < 4 ? kPerThread : 4;  // child keys loaded together
-    const uint64_t* __restrict__ ckey = s.c_key;
-    auto key_of = [&](int t) -> uint64_t {
-      if constexpr (kKeep) return kept[t];
-      else return ckey[begin + t];
-    };
+    const int begin = tid * Per;
     // the 2B draws (residues < P <= 65536), staged as 16-bit values with
     // coalesced loads, then read back per thread: child j's pair is the
     // 32-bit word j
@@ -1076,41 +1067,29 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
       }
     }
     // the children's levels, two a word (rows of child_level are padded)
-    uint32_t level_pair[(kPerThread + 1) / 2];
-    {
-      const uint32_t* pairs = reinterpret_cast<const uint32_t*>(s.child_level);
-      if constexpr (kPerThread == 1) {
-        level_pair[0] = begin < B ? uint32_t(uint16_t(s.child_level[begin])) : 0xffffu;
-      } else {
-#pragma unroll
-        for (int q = 0; q < kPerThread / 4; ++q) {
-          const uint2 v = begin + 4 * q < B ? *reinterpret_cast<const uint2*>(pairs + begin / 2 + 2 * q)
-                                            : make_uint2(~0u, ~0u);
-          level_pair[2 * q] = v.x;
-          level_pair[2 * q + 1] = v.y;
-        }
-      }
+    uint32_t level_pair[(Per + 1) / 2];
+    if constexpr (Per == 1) {
+      level_pair[0] = begin < B ? uint32_t(uint16_t(s.child_level[begin])) : 0xffffu;
+    } else {
+      const uint2 v = begin < B ? *reinterpret_cast<const uint2*>(s.child_level + begin) : make_uint2(~0u, ~0u);
+      level_pair[0] = v.x;
+      level_pair[1] = v.y;
     }
     __syncthreads();
-    uint32_t cand[kPerThread];
+    uint32_t cand[Per];
     {
       const uint32_t* words = reinterpret_cast<const uint32_t*>(stage);
-      if constexpr (kPerThread % 4 == 0) {
-        const uint4* pairs = reinterpret_cast<const uint4*>(words) + size_t(begin) / 4;
-#pragma unroll
-        for (int q = 0; q < kPerThread / 4; ++q) {
-          const uint4 v = begin < B ? pairs[q] : make_uint4(0, 0, 0, 0);
-          cand[4 * q] = v.x;
-          cand[4 * q + 1] = v.y;
-          cand[4 * q + 2] = v.z;
-          cand[4 * q + 3] = v.w;
-        }
+      if constexpr (Per == 1) {
+        cand[0] = begin < B ? words[begin] : 0;
       } else {
-#pragma unroll
-        for (int t = 0; t < kPerThread; ++t) cand[t] = begin + t < B ? words[begin + t] : 0;
+        const uint4 v = begin < B ? *reinterpret_cast<const uint4*>(words + begin) : make_uint4(0, 0, 0, 0);
+        cand[0] = v.x;
+        cand[1] = v.y;
+        cand[2] = v.z;
+        cand[3] = v.w;
       }
 #pragma unroll
-      for (int t = 0; t < kPerThread; ++t)
+      for (int t = 0; t < Per; ++t)
         if (begin + t >= B) {
           cand[t] = 0;
           level_pair[t / 2] |= 0xffffu << (16 * (t & 1));  // no level
@@ -1124,26 +1103,16 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
     const long long level_start = clock64();
     for (int level = 0; level < levels_run; ++level) {
 #pragma unroll
-      for (int h = 0; h < kPerThread; h += kBatch) {
-        uint32_t ready = 0;
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-          if ((level_pair[(h + u) / 2] >> (16 * ((h + u) & 1)) & 0xffffu) == uint32_t(level)) ready |= 1u << u;
-        uint64_t kv[kBatch];
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u) kv[u] = (ready >> u & 1) ? key_of(h + u) : 0;
-#pragma unroll
-        for (int u = 0; u < kBatch; ++u)
-          if (ready >> u & 1) {
-            const int d0 = int(cand[h + u] & 0xffff), d1 = int(cand[h + u] >> 16);
-            const uint64_t k0 = keys[d0], k1 = keys[d1];
-            // worst of the pair: the second replaces the first when the first is better
-            const int v = (k0 < k1 || (k0 == k1 && d0 < d1)) ? d1 : d0;
-            keys[v] = kv[u];
-            on[v] = int16_t(begin + h + u);
-            cand[h + u] = uint32_t(v);
-          }
-      }
+      for (int t = 0; t < Per; ++t)
+        if ((level_pair[t / 2] >> (16 * (t & 1)) & 0xffffu) == uint32_t(level)) {
+          const int d0 = int(cand[t] & 0xffff), d1 = int(cand[t] >> 16);
+          const uint64_t k0 = keys[d0], k1 = keys[d1];
+          // worst of the pair: the second replaces the first when the first is better
+          const int v = (k0 < k1 || (k0 == k1 && d0 < d1)) ? d1 : d0;
+          keys[v] = kept[t];
+          on[v] = int16_t(begin + t);
+          cand[t] = uint32_t(v);
+        }
       __syncthreads();
     }
     if (tid == 0)
@@ -1155,17 +1124,11 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
     uint64_t mk = ~0ULL;
     int mv = 0x7fffffff;
 #pragma unroll
-    for (int h = 0; h < kPerThread; h += kBatch) {
-      uint64_t kv[kBatch];
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) kv[u] = begin + h + u < B ? key_of(h + u) : ~0ULL;
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u)
-        if (begin + h + u < B && key_before(kv[u], int(cand[h + u]), mk, mv)) {
-          mk = kv[u];
-          mv = int(cand[h + u]);
-        }
-    }
+    for (int t = 0; t < Per; ++t)
+      if (begin + t < B && key_before(kept[t], int(cand[t]), mk, mv)) {
+        mk = kept[t];
+        mv = int(cand[t]);
+      }
     for (int o = 1; o < 32; o <<= 1) {
       const uint64_t uk = __shfl_up_sync(kFull, mk, o);
       const int uv = __shfl_up_sync(kFull, mv, o);
@@ -1202,23 +1165,17 @@ __device__ __noinline__ void place_round(const SearchDesc& s, PlaceShared& sh, u
     // a child whose victim is the best member before it would have redrawn
     bool hit = false;
 #pragma unroll
-    for (int h = 0; h < kPerThread; h += kBatch) {
-      uint64_t kv[kBatch];
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u) kv[u] = begin + h + u < B ? key_of(h + u) : 0;
-#pragma unroll
-      for (int u = 0; u < kBatch; ++u)
-        if (!hit && begin + h + u < B) {
-          const int v = int(cand[h + u]);
-          if (v == bv) {
-            atomicMin(&redraw_at, begin + h + u);
-            hit = true;
-          } else if (key_before(kv[u], v, bk, bv)) {
-            bk = kv[u];
-            bv = v;
-          }
+    for (int t = 0; t < Per; ++t)
+      if (!hit && begin + t < B) {
+        const int v = int(cand[t]);
+        if (v == bv) {
+          atomicMin(&redraw_at, begin + t);
+          hit = true;
+        } else if (key_before(kept[t], v, bk, bv)) {
+          bk = kept[t];
+          bv = v;
         }
-    }
+      }
     __syncthreads();
     parallel_done = redraw_at == 0x7fffffff;
     if (tid == 0)  // levels of the parallel path; a replay adds 2^20
