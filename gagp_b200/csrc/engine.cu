@@ -1960,13 +1960,20 @@ gagp_status capture_round(gagp_engine* e, const BatchView& v, RoundGraph* out) {
 }
 // `rounds` rounds of a batch.  Most runs launch them one after another: the
 // host is ahead of the device (10 to 40 stream operations a round), and
-// instantiating a graph of the round costs some 300 us a run for nothing in
-// return -- 24 rounds of P = 777 2.73 ms replayed, 2.40 launched; 50
-// generational rounds of 8 ranges 9.65 and 8.93; a served mix 98 and 85.  Long
-// runs of rounds split into ranges replay one: where the process created its
-// context with the default 8 hardware queues, ranges launched from 11 streams
-// wait for one another (128 rounds of P = 16384 33.9 ms replayed, 36.3
-// launched; with 32 queues 33.4 and 33.0).
+// capturing and instantiating a graph of the round costs a run 0.3 ms, 1 ms
+// with 8 ranges (24 rounds of P = 777 2.73 ms replayed, 2.40 launched; 50
+// generational rounds of 8 ranges 9.65 and 8.93; a served mix 98 and 85).
+// Long runs of rounds split into ranges replay one: a replayed round of theirs
+// is some 10 us shorter, and 20 to 45 where the process created its context
+// with the default 8 hardware queues, so that ranges launched from 11 streams
+// wait for one another.  In ms, launched with 32 and with 8 queues against
+// replayed (with either):
+//              32 rounds           64                  128
+//   P = 4096   4.9,  5.0 |  5.8    9.5,  9.8 |  9.9    18.6, 19.3 | 18.3
+//   P = 16384  9.3, 10.1 | 10.2   17.0, 18.9 | 17.6    31.2, 35.3 | 31.2
+// The line lies where both sides meet with 8 queues; with 32 they meet at 100
+// to 130 rounds, and runs between pay up to 5%.  Nothing tells how many queues
+// a context has.
 constexpr int kReplayRounds = 64;
 gagp_status launch_rounds(gagp_engine* e, const BatchView& v, int rounds) {
   if (rounds <= 0) return GAGP_OK;
@@ -2144,8 +2151,9 @@ EvalStaging eval_staging(const EvalPlan& p, const gagp_rows* rows) {
 // that exist, a sixth of the node words and constant slots they become -- and
 // one kernel unpacks them.  Host loops over node words, zeroed vectors, 16 MB
 // of pageable copies and an allocation per call took most of the 5.8 ms of
-// 16384 rows of 60 slots on 2000 cases (now 2.3 ms); 15 small copies and
-// memsets a third of the 153 us of 32 rows on 21 cases (now 105 us).
+// 16384 rows of 60 slots on 2000 cases (2.3 ms then, 1.5 with the present
+// VM); 15 small copies and memsets a third of the 153 us of 32 rows on 21
+// cases (now 107 us).
 gagp_status eval_rows_in(char* region, char* staging, const EvalStaging& sz, const EvalPlan& p, const gagp_grammar* g,
                          const gagp_cases* c, const gagp_search_config* cfg, const gagp_rows* rows, double* fitness,
                          uint32_t* wrong, uint32_t* errors, cudaStream_t stream, int sm_count, size_t max_smem) {
@@ -2983,10 +2991,9 @@ gagp_status gagp_b200_server_step(gagp_server* sv, int32_t* running, int32_t* qu
       for (Search* s : fresh) s->started = true;
     }
     if ((st = make_batch_view(e, list, &v)) != GAGP_OK) return st;
-    // up to rounds_per_step rounds (graph replays after the first), no more
-    // than the longest remaining search needs; a search that finishes within
-    // them idles (its kernels skip finished searches) until the states are
-    // read after the last
+    // up to rounds_per_step rounds, no more than the longest remaining search
+    // needs; a search that finishes within them idles (its kernels skip
+    // finished searches) until the states are read after the last
     int rounds = 1;
     for (int64_t t : sv->active) {
       const Request& r = *sv->requests.at(t);
