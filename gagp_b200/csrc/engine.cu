@@ -798,9 +798,9 @@ std::vector<char> gen_image(const gagp_grammar* g, const std::vector<gb::ExprInf
   return img;
 }
 
-// Instructions of a program's bytecode row, rounded so that a row also holds
+// Ints of a program's bytecode row of `stride` instructions: a row also holds
 // register code in 16-byte words.
-int bytecode_stride(const gagp_grammar* g, int maxv) { return int(align_up(size_t(gb::bytecode_bound(g, maxv)), 4)); }
+int bytecode_pitch(int stride) { return int(align_up(5 * size_t(stride), 4)); }
 
 // Device copy of the traversal table.
 std::vector<gb::RegionInfo> region_infos(const gagp_grammar* g) {
@@ -823,7 +823,7 @@ struct Plan {
       hist_sum, hist_fitness,
       hist_wrong,
       hist_nodes, hist_node, hist_cval, hist_len, counters;
-  int stride, code_stride, bc_stride, stream_capacity, slots;
+  int stride, code_stride, bc_stride, bc_pitch, stream_capacity, slots;
 };
 
 // Children per round: the steady-state batch, or the whole population under
@@ -839,7 +839,8 @@ Plan plan_search(const gagp_grammar* g, const gagp_cases* c, const gagp_search_c
   const int maxv = g->max_nodes - g->fixed_nodes;
   p.stride = int(align_up(size_t(maxv), 4));
   p.code_stride = 2 * maxv + 8;
-  p.bc_stride = bytecode_stride(g, maxv);
+  p.bc_stride = gb::bytecode_bound(g, maxv);
+  p.bc_pitch = bytecode_pitch(p.bc_stride);
   p.slots = std::max(P, B);
   const long long draws = (long long)B * cfg->replacement_size + 1;
   p.stream_capacity = int(((draws + 311) / 312 + 2) * 312);
@@ -878,7 +879,7 @@ Plan plan_search(const gagp_grammar* g, const gagp_cases* c, const gagp_search_c
   const size_t slots = size_t(p.slots);
   p.code = L.take(8 * slots * p.code_stride); p.code_len = L.take(4 * slots);
   p.kpool = L.take(8 * slots * S); p.code_temps = L.take(4 * slots); p.vm_acc = L.take(16 * slots);
-  p.bc = L.take(20 * slots * p.bc_stride); p.bc_len = L.take(4 * slots); p.bc_locals = L.take(4 * slots);
+  p.bc = L.take(4 * slots * p.bc_pitch); p.bc_len = L.take(4 * slots); p.bc_locals = L.take(4 * slots);
   p.bc_consts = L.take(8 * slots * p.bc_stride);
   p.mt = L.take(8 * 312); p.stream = L.take(8 * size_t(p.stream_capacity));
   p.stream_mod = L.take(4 * size_t(p.stream_capacity)); p.stream_head = L.take(16);
@@ -1399,6 +1400,7 @@ gagp_status gagp_b200_search_create(gagp_engine* e, const gagp_grammar* g, const
   d.bc = at<int32_t>(b, p.bc); d.bc_len = at<int32_t>(b, p.bc_len); d.bc_locals = at<int32_t>(b, p.bc_locals);
   d.bc_consts = at<int64_t>(b, p.bc_consts);
   d.bc_stride = p.bc_stride;
+  d.bc_pitch = p.bc_pitch;
   d.mt = at<uint64_t>(b, p.mt); d.stream = at<uint64_t>(b, p.stream); d.stream_mod = at<uint32_t>(b, p.stream_mod);
   d.stream_head = at<long long>(b, p.stream_head); d.stream_capacity = p.stream_capacity;
   d.mod_magic = ~0ULL / uint64_t(s->P);
@@ -2032,10 +2034,10 @@ namespace {
 // one caller-provided device region.
 struct EvalPlan {
   Layout L;
-  size_t desc, ex, info, minimum, local_types, regions, inputs, expected, lists, node, cval, len, code, code_len, kpool,
+  size_t desc, ex, info, minimum, local_types, regions, inputs, expected, lists, node, cval, len, code, code_len,
       code_temps, vm_acc, bc, bc_len, bc_locals, bc_consts, fitness, wrong, errors, counters, round, fast, exact,
       general, counts, off, region_list, region_ws, packed, results_end;
-  int stride, code_stride, bc_stride;
+  int stride, code_stride, bc_stride, bc_pitch;
   size_t region_words;  // bounded-region workspace per lane (0: the grammar has none)
 };
 // Counter words of a row evaluation: the lists' sizes, then (64 bits, from
@@ -2049,7 +2051,8 @@ EvalPlan plan_eval(const gagp_grammar* g, const gagp_cases* c, int rows) {
   const int maxv = g->max_nodes - g->fixed_nodes;
   p.stride = int(align_up(size_t(std::max(1, maxv)), 4));
   p.code_stride = 2 * maxv + 8;
-  p.bc_stride = bytecode_stride(g, maxv);
+  p.bc_stride = gb::bytecode_bound(g, maxv);
+  p.bc_pitch = bytecode_pitch(p.bc_stride);
   const int E = g->expression_count, C = c->case_count;
   const size_t R = size_t(std::max(1, rows)), S = size_t(p.stride);
   auto& L = p.L;
@@ -2070,14 +2073,14 @@ EvalPlan plan_eval(const gagp_grammar* g, const gagp_cases* c, int rows) {
   p.off = L.take(8);
   // the packed rows lie where the lowering writes the bytecode afterwards: a
   // row's 10 bytes per node and 12 more against 20 bytes per bytecode word,
-  // of which a row has at least as many as it has nodes and at least 4
-  p.bc = L.take(20 * R * p.bc_stride);
+  // of which a row has at least two more than it has nodes
+  p.bc = L.take(4 * R * p.bc_pitch);
   p.packed = p.bc;
   p.bc_len = L.take(4 * R); p.bc_locals = L.take(4 * R);
   p.bc_consts = L.take(8 * R * p.bc_stride);
   p.minimum = L.take(sizeof(uint32_t));
   p.node = L.take(8 * S * R); p.cval = L.take(8 * S * R); p.len = L.take(4 * R);
-  p.code = L.take(8 * R * p.code_stride); p.code_len = L.take(4 * R); p.kpool = L.take(8 * R * S);
+  p.code = L.take(8 * R * p.code_stride); p.code_len = L.take(4 * R);
   p.code_temps = L.take(4 * R); p.vm_acc = L.take(16 * R);
   p.fast = L.take(sizeof(gb::ProgramRef) * R); p.exact = L.take(sizeof(gb::ProgramRef) * R);
   p.general = L.take(sizeof(gb::ProgramRef) * R);
@@ -2243,7 +2246,7 @@ gagp_status eval_rows_in(char* region, char* staging, const EvalStaging& sz, con
   d.len = at<int32_t>(b, p.len);
   d.code = at<uint2>(b, p.code);
   d.code_len = at<int32_t>(b, p.code_len);
-  d.kpool = at<int64_t>(b, p.kpool);
+  d.kpool = d.cval;  // a row's constants are its program's
   d.code_stride = p.code_stride;
   d.code_temps = at<int32_t>(b, p.code_temps);
   d.vm_acc = at<unsigned long long>(b, p.vm_acc);
@@ -2252,6 +2255,7 @@ gagp_status eval_rows_in(char* region, char* staging, const EvalStaging& sz, con
   d.bc_locals = at<int32_t>(b, p.bc_locals);
   d.bc_consts = at<int64_t>(b, p.bc_consts);
   d.bc_stride = p.bc_stride;
+  d.bc_pitch = p.bc_pitch;
   d.fitness = at<double>(b, p.fitness);
   d.wrong = at<uint32_t>(b, p.wrong);
   d.errors = at<uint32_t>(b, p.errors);

@@ -186,13 +186,13 @@ __global__ void __launch_bounds__(kLowerWarps<Exact> * 32, Exact ? 14 : 32)
     if constexpr (!Exact) {
       if (lane == 0) raise_error(s, 30);  // the phase compiler rejects the row
     } else {
-      int32_t* bc = s.bc + size_t(slot) * 5 * s.bc_stride;
+      int32_t* bc = s.bc + size_t(slot) * s.bc_pitch;
       int64_t* bc_consts = s.bc_consts + size_t(slot) * s.bc_stride;
       int slots = 0;
       int exact = kTooManySlots;
 #pragma unroll 1
       for (int keep = 1; keep >= 0 && exact == kTooManySlots; --keep)
-        exact = lower_exact_warp(s, t.node, t.n, t.cval, t.nc, reinterpret_cast<uint4*>(bc), s.bc_stride * 5 / 4,
+        exact = lower_exact_warp(s, t.node, t.n, t.cval, t.nc, reinterpret_cast<uint4*>(bc), s.bc_pitch / 4,
                                  bc_consts, scratch[warp].exact, keep, &slots);
       if (lane == 0) {
         if (exact >= 0) {
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kExactWarps * 32, kExactBlocks) k_vm_exact(con
       if (c - lane >= s.C) continue;
       const bool live = c < s.C;
       const VmView view = vm_view(s);
-      const int32_t* code = s.bc + size_t(p.slot) * 5 * s.bc_stride;
+      const int32_t* code = s.bc + size_t(p.slot) * s.bc_pitch;
       const int64_t* consts = s.bc_consts + size_t(p.slot) * s.bc_stride;
       int64_t loss = 0;
       uint32_t wrong = 0, errors = 0;
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(kRegionThreads) k_vm_region(const SearchDesc* 
     if (c - lane >= s.C) continue;
     const int n = s.bc_len[p.slot], shape = s.bc_locals[p.slot];
     const int n_locals = shape & 0xff, n_main = (shape >> 16) & 0xffff;
-    const int32_t* code = s.bc + size_t(p.slot) * 5 * s.bc_stride;
+    const int32_t* code = s.bc + size_t(p.slot) * s.bc_pitch;
     const int64_t* consts = s.bc_consts + size_t(p.slot) * s.bc_stride;
     const int main_consts = s.code_temps[p.slot];
     const VmView view = vm_view(s);

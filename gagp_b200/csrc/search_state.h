@@ -262,7 +262,8 @@ struct SearchDesc {
   int32_t* bc_len;
   int32_t* bc_locals;                  // per lowered program: locals (inputs + temporaries) | stack bound << 8
   int64_t* bc_consts;
-  int32_t bc_stride;                   // instructions per program slot
+  int32_t bc_stride;                   // instructions (and constants) per program slot
+  int32_t bc_pitch;                    // ints per program slot: the instructions, a multiple of 16 bytes
   // ---- run generator (MT19937-64) and its output stream
   uint64_t* mt;                        // 312 words
   uint64_t* stream;                    // buffered outputs

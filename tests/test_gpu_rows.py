@@ -139,3 +139,25 @@ def test_rows_past_the_arena_limit(tmp_path):
         held = before - torch.cuda.mem_get_info(0)[0]
     assert np.array_equal(f, want_f[index]) and np.array_equal(w, want_w[index])
     assert held <= 16 << 20, held
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,cases,count", [("poly4", 256, 5631), ("polynomial", 21, 16316),
+                                              ("list_threshold", 200, 2836), ("list_statements", 200, 1380),
+                                              ("grid_paths", 40, 1936)])
+def test_static_rows_at_the_limit(name, cases, count):
+    """Row counts that just fit the static 32 MiB with rows, bytecode and lists
+    of their least size."""
+    from gagp_b200.engine import Engine, evaluate_rows_static
+    kw = {} if name == "polynomial" else {"cases": cases}
+    lt = T.from_files(W.make(name, population=128, generations=2, seed=8, **kw))
+    assert len(lt.cases.expected) == cases
+    with Engine(0) as engine:
+        s = engine.admit(lt)
+        s.run()
+        rows = s.result_buffer().final_rows
+        s.close()
+        want_f, want_w = engine.evaluate_rows(lt, rows)
+    index = np.arange(count) % rows.count
+    f, w = evaluate_rows_static(lt, _take(rows, index))
+    assert np.array_equal(f, want_f[index]) and np.array_equal(w, want_w[index])
